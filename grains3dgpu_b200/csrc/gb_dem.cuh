@@ -38,16 +38,15 @@ GB_D Contact<S> no_contact()
 // closestPointsSpheres (CollisionDetection.cpp:26-48); a sphere's radius is
 // its circumscribed radius, p[0] (the table's rcirc may include the crust)
 template <typename S>
-GB_D Contact<S> closest_spheres(const Body<S>& A, const Body<S>& B, const V3<S>& oA,
-                                const V3<S>& oB)
+GB_D Contact<S> closest_spheres(S rA, S rB, const V3<S>& oA, const V3<S>& oB)
 {
     V3<S>   vba     = oB - oA;
-    const S overlap = norm(vba) - A.p[0] - B.p[0];
+    const S overlap = norm(vba) - rA - rB;
     vba             = vba / norm(vba);
     if(overlap < S(0.0))
     {
         Contact<S> c;
-        c.pt      = oA + (A.p[0] + S(0.5) * overlap) * vba;
+        c.pt      = oA + (rA + S(0.5) * overlap) * vba;
         c.vec     = overlap * vba;
         c.overlap = overlap;
         return c;
@@ -61,7 +60,7 @@ GB_D Contact<S> closest_points(const Body<S>& A, const Body<S>& B, const M3<S>& 
                                const V3<S>& d, int* gjk_iters)
 {
     if(A.type == GB_SPHERE && B.type == GB_SPHERE)
-        return closest_spheres(A, B, oA, oB);
+        return closest_spheres(A.p[0], B.p[0], oA, oB);
     const S overlap = norm(d) - (A.rcirc + B.rcirc);
     if(!(overlap < S(0.0)))
         return no_contact<S>();

@@ -128,6 +128,8 @@ struct gb_ctx
     uint32_t obs_rect    = 0u;      // bit o: obstacle o (< 32) is a Rectangle
     bool     obs_gjk     = false;   // some obstacle is neither a Rectangle nor a drum
     bool     poly_bodies = false;   // some rigid body is a polyhedron
+    bool     all_spheres = false;   // every rigid body is a sphere
+    bool     some_spheres = false;  // some rigid body is a sphere
     std::vector<double> obs_vel;    // 6 per obstacle: velocity, angular velocity
     double*  d_obs_vel   = nullptr;
     double*  d_rcirc64 = nullptr;
@@ -137,6 +139,14 @@ struct gb_ctx
     void* d_shape64 = nullptr;
     void* d_verts64 = nullptr;
     void* d_obs_shape64 = nullptr;
+    // FP32 shape tables of the certified FP32 passes: d_shape and d_verts in
+    // the mixed mode, rounded copies in the FP64 modes
+    void* d_shape32 = nullptr;
+    void* d_verts32 = nullptr;
+    // per-particle records of the narrow phase (PoseRec, or SphereRec where
+    // every body is a sphere)
+    void* d_pose   = nullptr;
+    void* d_sphere = nullptr;
 
     // state
     double*   d_pos = nullptr; // 3n
@@ -161,8 +171,8 @@ struct gb_ctx
     double4*  d_spos = nullptr;
     float4*   d_spos32 = nullptr; // FP32 copy for the candidate pre-test
     uint32_t* d_slot   = nullptr; // kPairSlots candidates per particle (count pass)
-    uint32_t* d_gjkq   = nullptr; // the step's pairs that need GJK (pair capacity; the
-                                  // mixed mode: a second queue for its FP64 GJK after it)
+    uint32_t* d_gjkq   = nullptr; // the cull's queue of unordered pairs and, after it (pair
+                                  // capacity each), the records of the FP64 GJK
     uint32_t* d_obsq   = nullptr; // the step's obstacle records (pair capacity)
     uint32_t* d_gjkn   = nullptr; // their numbers (reset by the fill pass)
     uint32_t* d_ovf    = nullptr; // particles with more partners than pair slots
@@ -204,7 +214,7 @@ struct gb_ctx
     uint32_t* d_pb[2] = {nullptr, nullptr};
     uint32_t* d_pa = nullptr;
     void*     d_pf = nullptr; // 9 * cap storage values: f, t, m
-    uint8_t*  d_pc = nullptr;
+    uint8_t*  d_pc[2] = {nullptr, nullptr}; // contact flags, double-buffered with the list
     double*   d_info = nullptr;
     void*     d_xi[2] = {nullptr, nullptr}; // 3 * cap each
     int64_t   cap = 0;
@@ -335,6 +345,8 @@ Tables<S> tables_of(gb_ctx* c)
     t.shape64     = (const RBShape<double>*)c->d_shape64;
     t.verts64     = (const Vert<double>*)c->d_verts64;
     t.obs_shape64 = (const RBShape<double>*)c->d_obs_shape64;
+    t.shape32     = (const RBShape<float>*)c->d_shape32;
+    t.verts32     = (const Vert<float>*)c->d_verts32;
     return t;
 }
 
@@ -417,6 +429,34 @@ int upload_tables(gb_ctx* c)
     GB_CK(cudaMemcpy(c->d_verts, vv.data(), vv.size() * sizeof(vv[0]), cudaMemcpyHostToDevice));
     GB_CK(cudaMemcpy(c->d_rcirc64, rc.data(), rc.size() * sizeof(double), cudaMemcpyHostToDevice));
     return GB_OK;
+}
+
+// FP32 copies of the FP64 shape tables (each value rounded once, as the
+// mixed mode's upload rounds it)
+__global__ void __launch_bounds__(kBlock)
+    k_tables_to_float(int n_shapes, const RBShape<double>* __restrict__ s, RBShape<float>* __restrict__ so,
+                      int n_verts, const Vert<double>* __restrict__ v, Vert<float>* __restrict__ vo)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if(i < n_verts)
+        vo[i] = {(float)v[i].x, (float)v[i].y, (float)v[i].z, 0.0f};
+    if(i >= n_shapes)
+        return;
+    RBShape<float> r;
+    r.type       = s[i].type;
+    r.nverts     = s[i].nverts;
+    r.first_vert = s[i].first_vert;
+    for(int k = 0; k < 5; ++k)
+        r.p[k] = (float)s[i].p[k];
+    for(int k = 0; k < 8; ++k)
+        r.k[k] = (float)s[i].k[k];
+    r.crust = (float)s[i].crust;
+    r.rcirc = (float)s[i].rcirc;
+    for(int k = 0; k < 3; ++k)
+        r.bb[k] = (float)s[i].bb[k];
+    r.material = s[i].material;
+    r.pad      = 0;
+    so[i]      = r;
 }
 
 template <typename St>
@@ -564,9 +604,12 @@ int ensure_pairs(gb_ctx* c, int64_t need)
     // the previous step's history buffers must survive the growth
     uint32_t* npb[2] = {nullptr, nullptr};
     void*     nxi[2] = {nullptr, nullptr};
+    uint8_t*  npc[2] = {nullptr, nullptr};
     for(int b = 0; b < 2; ++b)
     {
         GB_TRY(dalloc(&npb[b], ncap));
+        if(hist || b == c->cur)
+            GB_TRY(dalloc(&npc[b], ncap));
         if(hist)
             GB_CK(cudaMalloc(&nxi[b], 3 * ncap * ss));
     }
@@ -577,6 +620,8 @@ int ensure_pairs(gb_ctx* c, int64_t need)
     {
         GB_CK(cudaMemcpy(npb[prev], c->d_pb[prev], c->cap * sizeof(uint32_t),
                          cudaMemcpyDeviceToDevice));
+        if(hist)
+            GB_CK(cudaMemcpy(npc[prev], c->d_pc[prev], c->cap, cudaMemcpyDeviceToDevice));
         if(hist)
             for(int k = 0; k < 3; ++k)
                 GB_CK(cudaMemcpy((char*)nxi[prev] + k * ncap * ss,
@@ -589,18 +634,18 @@ int ensure_pairs(gb_ctx* c, int64_t need)
         c->d_pb[b] = npb[b];
         dfree(c->d_xi[b]);
         c->d_xi[b] = nxi[b];
+        dfree(c->d_pc[b]);
+        c->d_pc[b] = npc[b];
     }
     dfree(c->d_pa);
     dfree(c->d_pf);
-    dfree(c->d_pc);
     dfree(c->d_info);
     dfree(c->d_gjkq);
-    GB_TRY(dalloc(&c->d_gjkq, (c->prec == GB_MIXED ? 2 : 1) * ncap));
+    GB_TRY(dalloc(&c->d_gjkq, 2 * ncap));
     dfree(c->d_obsq);
     GB_TRY(dalloc(&c->d_obsq, ncap));
     GB_TRY(dalloc(&c->d_pa, ncap));
     GB_CK(cudaMalloc(&c->d_pf, 9 * ncap * ss));
-    GB_TRY(dalloc(&c->d_pc, ncap));
     if(c->cfg.flags & GB_FLAG_RECORD_CONTACT_INFO)
         GB_TRY(dalloc(&c->d_info, 7 * ncap));
     c->cap = ncap;
@@ -1025,6 +1070,27 @@ int obstacle_cells(gb_ctx* c)
     return GB_OK;
 }
 
+// the arrays of the records that this run's narrow phase reads
+template <typename St>
+Records<St> records_of(gb_ctx* c)
+{
+    Records<St> rec;
+    rec.sphere = c->all_spheres ? (SphereRec<St>*)c->d_sphere : nullptr;
+    rec.pose   = c->all_spheres ? nullptr : (PoseRec<St>*)c->d_pose;
+    return rec;
+}
+
+// ... allocated with the bodies that decide which they are
+template <typename St>
+int alloc_records(gb_ctx* c)
+{
+    if(c->all_spheres && !c->d_sphere)
+        GB_TRY(dalloc((SphereRec<St>**)&c->d_sphere, c->n));
+    if(!c->all_spheres && !c->d_pose)
+        GB_TRY(dalloc((PoseRec<St>**)&c->d_pose, c->n));
+    return GB_OK;
+}
+
 // candidate pairs (particles, then obstacles): count -> scan -> fill, with no
 // host round trip: the total stays on the device (off[n]); a total beyond the
 // capacity aborts the step (kFlagCapacity) and the host replays it larger
@@ -1113,14 +1179,17 @@ int build_pairs(gb_ctx* c)
     GB_CK(launch(c->pdl, k_pair_fill<S>, nb, kBlock, s, n, c->d_skeys, c->d_sids, c->d_sorted_of,
                  c->d_spos, spos32, c->d_cstart, c->dims[0], c->dims[1], c->dims[2], c->d_count,
                  c->d_slot, oc, off, c->d_pa, c->d_pb[c->cur], c->cap,
-                 c->d_flags, c->d_gjkn, c->d_count + n + 1, c->d_ovf, c->ovf_phase, c->d_obsq));
+                 c->d_flags, c->d_gjkn, c->d_count + n + 1, c->d_ovf, c->ovf_phase, c->d_obsq,
+                 c->d_pc[c->cur], state_of<St>(c), tables_of<S>(c),
+                 records_of<St>(c)));
     c->count_zero = true; // the fill pass zeroes each count it reads
     GB_CK(launch(c->pdl, k_pair_fill_overflow<S>, 4 * c->sms, 128, s,
                  (const uint32_t*)c->d_gjkn + 2 + c->ovf_phase, (const uint32_t*)c->d_ovf,
                  (const uint32_t*)c->d_skeys, (const uint32_t*)c->d_sids,
                  (const uint32_t*)c->d_sorted_of, (const double4*)c->d_spos, spos32,
                  (const uint32_t*)c->d_cstart, c->dims[0], c->dims[1], c->dims[2],
-                 (const uint32_t*)off, c->d_pa, c->d_pb[c->cur], (const int*)c->d_flags));
+                 (const uint32_t*)off, c->d_pa, c->d_pb[c->cur], c->d_pc[c->cur],
+                 (const int*)c->d_flags));
     c->launches += 2;
     GB_CK(cudaGetLastError());
     mark(c, 5);
@@ -1140,12 +1209,13 @@ PairOut<store_t<S>> pair_out(gb_ctx* c)
         po.m[k] = (St*)c->d_pf + (6 + k) * cap;
         po.xi[k] = c->d_xi[c->cur] ? (St*)c->d_xi[c->cur] + k * cap : nullptr;
     }
-    po.contact  = c->d_pc;
+    po.contact  = c->d_pc[c->cur];
     po.pcount   = c->d_pcount;
     po.info     = c->d_info;
     const int prev = 1 - c->cur;
     po.prev_off = c->d_off[prev];
     po.prev_b   = c->d_pb[prev];
+    po.prev_contact = c->d_pc[prev];
     for(int k = 0; k < 3; ++k)
         po.prev_xi[k] = c->d_xi[prev] ? (const St*)c->d_xi[prev] + k * cap : nullptr;
     return po;
@@ -1190,14 +1260,14 @@ int run_detect(gb_ctx* c, int phases)
         // one wave of resident blocks walks the device-side total (off[n]):
         // a short list is spread over all of its warps (for_each_pair)
         const uint32_t* total = c->d_off[c->cur] + c->n;
-        auto one_wave = [&](const void* kernel) {
+        auto one_wave = [&](const void* kernel, int block) {
             int per_sm = 0;
-            if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0)
+            if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0)
                    != cudaSuccess
                || per_sm < 1)
                 per_sm = 1;
             return (int)std::max<int64_t>(
-                1, std::min<int64_t>(blocks(c->cap, 128), (int64_t)per_sm * c->sms));
+                1, std::min<int64_t>(blocks(c->cap, block), (int64_t)per_sm * c->sms));
         };
         const int kr  = c->has_kr ? 1 : 0;
         const int law = c->cfg.contact_law;
@@ -1207,36 +1277,34 @@ int run_detect(gb_ctx* c, int phases)
         // side, the obstacle one on the auxiliary stream.
         // the fill pass's count of this step's obstacle records
         const uint32_t* nobs_rec = c->d_gjkn + 4 + c->ovf_phase;
-        auto with_variant = [&](auto var) -> int {
-            constexpr int VAR = decltype(var)::value;
-            cudaStream_t  so  = s;
-            if(c->nob)
-            {
-                GB_CK(cudaEventRecord(c->ev_fork, s));
-                GB_CK(cudaStreamWaitEvent(c->aux_stream, c->ev_fork, 0));
-                so = c->aux_stream;
-            }
-            GB_CK(launch(c->pdl, k_narrow<S, VAR>, one_wave((const void*)k_narrow<S, VAR>), 128, s,
-                         total, c->d_flags, c->d_pa, c->d_pb[c->cur], st, tb, po, law, kr,
-                         S(c->cfg.dt), c->d_counters, c->d_gjkq, c->d_gjkn));
-            // the FP64 GJK's queue: the cull pass's, or in the mixed mode
-            // what the FP32 stage leaves of it (its certificate, a lower
-            // bound on the distance, holds for every GJK variant)
-            const uint32_t* q64 = c->d_gjkq;
-            const uint32_t* n64 = c->d_gjkn;
-            if constexpr(is_mixed<S>())
-            {
-                GB_CK(launch(c->pdl, k_narrow_gjk32, one_wave((const void*)k_narrow_gjk32), 128, s,
-                             (const uint32_t*)c->d_gjkn, (const int*)c->d_flags,
-                             (const uint32_t*)c->d_gjkq, (const uint32_t*)c->d_pa,
-                             (const uint32_t*)c->d_pb[c->cur], st, tb, po, law, kr,
-                             c->d_gjkq + c->cap, c->d_gjkn + 1));
-                c->launches += 1;
-                q64 = c->d_gjkq + c->cap;
-                n64 = c->d_gjkn + 1;
-            }
+        // particle pairs of shapes other than all spheres: the cull of the
+        // unordered pairs, the FP32 GJK on what it leaves, the FP64 GJK on
+        // both records of what that leaves
+        auto particle_pairs = [&](auto var) -> int {
+            constexpr int  VAR = decltype(var)::value;
+            constexpr bool JH  = VAR == GB_GJK_JH;
+            const auto*    pose = (const PoseRec<St>*)c->d_pose;
+            const uint32_t* off = c->d_off[c->cur];
+            auto            cull = [&](auto kernel) -> int {
+                GB_CK(launch(c->pdl, kernel, one_wave((const void*)kernel, 128), 128, s, total,
+                             (const int*)c->d_flags, (const uint32_t*)c->d_pa,
+                             (const uint32_t*)c->d_pb[c->cur], off, pose, st, tb, po, law, kr,
+                             S(c->cfg.dt), c->d_counters, c->d_gjkq, c->d_gjkn));
+                return GB_OK;
+            };
+            if(c->some_spheres)
+                GB_TRY(cull(k_narrow<S, JH, true>));
+            else
+                GB_TRY(cull(k_narrow<S, JH, false>));
+            GB_CK(launch(c->pdl, k_narrow_gjk32<St>, one_wave((const void*)k_narrow_gjk32<St>, 128),
+                         128, s, (const uint32_t*)c->d_gjkn, (const int*)c->d_flags,
+                         (const uint32_t*)c->d_gjkq, (const uint32_t*)c->d_pa,
+                         (const uint32_t*)c->d_pb[c->cur], off, pose, tb.shape32, tb.verts32,
+                         c->d_gjkq + c->cap, c->d_gjkn + 1));
+            const uint32_t* q64 = c->d_gjkq + c->cap;
+            const uint32_t* n64 = c->d_gjkn + 1;
             auto launch_gjk = [&](auto kernel, uint32_t lo, uint32_t hi) -> int {
-                GB_CK(launch(c->pdl, kernel, one_wave((const void*)kernel), 128, s, n64,
+                GB_CK(launch(c->pdl, kernel, one_wave((const void*)kernel, 128), 128, s, n64,
                              c->d_flags, q64, c->d_pa, c->d_pb[c->cur], st, tb, po, law, kr,
                              S(c->cfg.dt), c->d_counters, lo, hi));
                 return GB_OK;
@@ -1252,26 +1320,47 @@ int run_detect(gb_ctx* c, int phases)
             if constexpr(is_mixed<S>())
                 if(!c->poly_bodies)
                 {
-                    split = (uint32_t)(one_wave((const void*)k_narrow_gjk<S, VAR>) * 128 / 2);
+                    split = (uint32_t)(one_wave((const void*)k_narrow_gjk<S, VAR>, 128) * 128 / 2);
                     GB_TRY(launch_gjk(k_narrow_gjk<S, VAR, 3>, split, UINT32_MAX));
                     c->launches += 1;
                 }
             GB_TRY(launch_gjk(k_narrow_gjk<S, VAR>, 0u, split));
-            c->launches += 2;
+            c->launches += 3;
+            return GB_OK;
+        };
+        auto with_variant = [&](auto var) -> int {
+            constexpr int VAR = decltype(var)::value;
+            cudaStream_t  so  = s;
+            if(c->nob)
+            {
+                GB_CK(cudaEventRecord(c->ev_fork, s));
+                GB_CK(cudaStreamWaitEvent(c->aux_stream, c->ev_fork, 0));
+                so = c->aux_stream;
+            }
+            if(c->all_spheres)
+            {
+                GB_CK(launch(c->pdl, k_narrow_spheres<S>,
+                             one_wave((const void*)k_narrow_spheres<S>, kBlock), kBlock, s, total,
+                             (const int*)c->d_flags, (const uint32_t*)c->d_pa,
+                             (const uint32_t*)c->d_pb[c->cur], (const SphereRec<St>*)c->d_sphere,
+                             tb, po, law, kr, S(c->cfg.dt)));
+                c->launches += 1;
+            }
+            else
+                GB_TRY(particle_pairs(var));
             if(!c->nob)
                 return GB_OK;
             // Rectangles and drums are met by their own closed forms; any
             // other obstacle needs the general GJK compiled in
-            if(!c->obs_gjk)
-                k_narrow_obstacles<S, false, GB_GJK_JH>
-                    <<<one_wave((const void*)k_narrow_obstacles<S, false, GB_GJK_JH>), 128, 0, so>>>(
-                    nobs_rec, c->d_obsq, c->d_flags, c->d_pa, c->d_pb[c->cur], st, tb, po, law,
-                    kr, S(c->cfg.dt), c->d_counters);
+            auto obstacles = [&](auto kernel) {
+                kernel<<<one_wave((const void*)kernel, 128), 128, 0, so>>>(
+                    nobs_rec, c->d_obsq, c->d_flags, c->d_pa, c->d_pb[c->cur], st, tb, po, law, kr,
+                    S(c->cfg.dt), c->d_counters);
+            };
+            if(c->obs_gjk)
+                obstacles(k_narrow_obstacles<S, true, VAR>);
             else
-                k_narrow_obstacles<S, true, VAR>
-                    <<<one_wave((const void*)k_narrow_obstacles<S, true, VAR>), 128, 0, so>>>(
-                    nobs_rec, c->d_obsq, c->d_flags, c->d_pa, c->d_pb[c->cur], st, tb, po, law,
-                    kr, S(c->cfg.dt), c->d_counters);
+                obstacles(k_narrow_obstacles<S, false, GB_GJK_JH>);
             c->launches += 1;
             GB_CK(cudaEventRecord(c->ev_join, so));
             GB_CK(cudaStreamWaitEvent(s, c->ev_join, 0));
@@ -1640,7 +1729,7 @@ int gb_destroy(gb_ctx* c)
                     c->d_obs_mass, c->d_obs_plane, c->d_obs_vel, c->d_rcirc64, c->d_pos, c->d_rot, c->d_vel, c->d_omg, c->d_frc,
                     c->d_trq, c->d_rb_id, c->d_hash, c->d_iota, c->d_k[0], c->d_k[1], c->d_i[0],
                     c->d_i[1], c->d_hist, c->d_part, c->d_cstart, c->d_ccount, c->d_spos, c->d_spos32, c->d_slot, c->d_sorted_of, c->d_obsmask_id, c->d_count,
-                    c->d_off[0], c->d_off[1], c->d_pb[0], c->d_pb[1], c->d_pa, c->d_pf, c->d_pc,
+                    c->d_off[0], c->d_off[1], c->d_pb[0], c->d_pb[1], c->d_pa, c->d_pf, c->d_pc[0], c->d_pc[1], c->d_pose, c->d_sphere,
                     c->d_info, c->d_xi[0], c->d_xi[1], c->d_flags, c->d_counters, c->d_done,
                     c->d_contacts,
                     c->d_stage,     c->d_adj, c->d_tile_state, c->d_ticket, c->d_gjkq, c->d_gjkn,
@@ -1650,6 +1739,10 @@ int gb_destroy(gb_ctx* c)
     for(void* p : ptrs)
         if(p)
             cudaFree(p);
+    if(c->d_shape32 && c->d_shape32 != c->d_shape)
+        cudaFree(c->d_shape32);
+    if(c->d_verts32 && c->d_verts32 != c->d_verts)
+        cudaFree(c->d_verts32);
     if(c->d_shape64 && c->d_shape64 != c->d_shape)
         cudaFree(c->d_shape64);
     if(c->d_verts64 && c->d_verts64 != c->d_verts)
@@ -1715,11 +1808,15 @@ int gb_set_rigid_bodies(gb_ctx* c, const gb_rigid_body_desc* rbs, const double* 
     c->verts.assign(vertices, vertices + 3 * n_vertices);
     c->props.resize(c->nrb);
     double rmax = 0.0;
-    c->poly_bodies = false;
+    c->poly_bodies  = false;
+    c->all_spheres  = true;
+    c->some_spheres = false;
     for(int i = 0; i < c->nrb; ++i)
     {
         const gb_convex& cv = rbs[i].convex;
-        c->poly_bodies = c->poly_bodies || cv.type == GB_POLYHEDRON;
+        c->poly_bodies  = c->poly_bodies || cv.type == GB_POLYHEDRON;
+        c->all_spheres  = c->all_spheres && cv.type == GB_SPHERE;
+        c->some_spheres = c->some_spheres || cv.type == GB_SPHERE;
         if(cv.type == GB_POLYHEDRON
            && (cv.first_vertex < 0 || cv.first_vertex + cv.n_vertices > n_vertices))
             return GB_E_INVALID_ARG;
@@ -1763,6 +1860,12 @@ int gb_set_rigid_bodies(gb_ctx* c, const gb_rigid_body_desc* rbs, const double* 
         cudaFree(c->d_shape64);
         cudaFree(c->d_verts64);
     }
+    if(c->prec != GB_MIXED)
+    {
+        cudaFree(c->d_shape32);
+        cudaFree(c->d_verts32);
+    }
+    c->d_shape32 = c->d_verts32 = nullptr;
     c->d_shape64 = c->d_verts64 = nullptr;
     int st       = upload_tables<double>(c);
     c->d_shape64 = c->d_shape;
@@ -1771,7 +1874,23 @@ int gb_set_rigid_bodies(gb_ctx* c, const gb_rigid_body_desc* rbs, const double* 
     {
         c->d_shape = c->d_verts = nullptr; // keep the FP64 copies, add FP32 ones
         st                      = upload_tables<float>(c);
+        c->d_shape32            = c->d_shape;
+        c->d_verts32            = c->d_verts;
     }
+    else if(st == GB_OK && !c->all_spheres)
+    {
+        // the FP64 modes' FP32 copies, rounded on the device
+        const int nv = std::max((int)(c->verts.size() / 3), 1);
+        GB_TRY(dalloc((RBShape<float>**)&c->d_shape32, c->nrb));
+        GB_TRY(dalloc((Vert<float>**)&c->d_verts32, nv));
+        k_tables_to_float<<<blocks(std::max(c->nrb, nv), kBlock), kBlock>>>(
+            c->nrb, (const RBShape<double>*)c->d_shape, (RBShape<float>*)c->d_shape32, nv,
+            (const Vert<double>*)c->d_verts, (Vert<float>*)c->d_verts32);
+        GB_CK(cudaGetLastError());
+        GB_CK(cudaStreamSynchronize(0));
+    }
+    if(st == GB_OK)
+        st = c->prec == GB_MIXED ? alloc_records<float>(c) : alloc_records<double>(c);
     if(st)
         return st;
     c->rb_set     = true;
@@ -2110,7 +2229,7 @@ int gb_save_contacts(gb_ctx* c, void* buf, int64_t capacity, int64_t* size)
                           cudaMemcpyDeviceToDevice, s));
     GB_CK(cudaMemcpyAsync(b + 16 + 4 * (n + 1), c->d_pb[c->cur], 4 * (size_t)np,
                           cudaMemcpyDeviceToDevice, s));
-    GB_CK(cudaMemcpyAsync(b + 16 + 4 * (n + 1) + 4 * np, c->d_pc, (size_t)np,
+    GB_CK(cudaMemcpyAsync(b + 16 + 4 * (n + 1) + 4 * np, c->d_pc[c->cur], (size_t)np,
                           cudaMemcpyDeviceToDevice, s));
     GB_CK(cudaStreamSynchronize(s));
     return GB_OK;
@@ -2132,7 +2251,7 @@ int gb_load_contacts(gb_ctx* c, const void* buf)
                           cudaMemcpyDeviceToDevice, s));
     GB_CK(cudaMemcpyAsync(c->d_pb[c->cur], b + 16 + 4 * (n + 1), 4 * (size_t)np,
                           cudaMemcpyDeviceToDevice, s));
-    GB_CK(cudaMemcpyAsync(c->d_pc, b + 16 + 4 * (n + 1) + 4 * np, (size_t)np,
+    GB_CK(cudaMemcpyAsync(c->d_pc[c->cur], b + 16 + 4 * (n + 1) + 4 * np, (size_t)np,
                           cudaMemcpyDeviceToDevice, s));
     GB_CK(cudaStreamSynchronize(s));
     c->npairs          = np;
@@ -2203,7 +2322,7 @@ int gb_adjoint_step(gb_ctx* c, const double* adj_next, double* adj_prev, double*
     k_adj_integrate<<<nb, kBlock, 0, s>>>(n, c->cfg.dt, h, verlet ? 1 : 0, state, in, adj_next,
                                           adj_prev, lft);
     k_adj_contacts<<<nb, kBlock, 0, s>>>(n, state, (const RBShape<double>*)c->d_shape, in,
-                                         c->d_off[c->cur], c->d_pb[c->cur], c->d_pc, lft,
+                                         c->d_off[c->cur], c->d_pb[c->cur], c->d_pc[c->cur], lft,
                                          c->d_obs_tr, (const RBShape<double>*)c->d_obs_shape,
                                          laws, adj_prev, part);
     k_adj_reduce<<<1, 4 * kAdjMaxLaws, 0, s>>>(nb, 4 * nl, part, grad_laws);
@@ -2243,9 +2362,10 @@ int gb_get_stats(gb_ctx* c, gb_stats* o)
         // tests and GJK's first iteration), and those solved by the FP64 GJK
         uint32_t q[2] = {0, 0};
         GB_CK(cudaMemcpy(q, c->d_gjkn, sizeof(q), cudaMemcpyDeviceToHost));
-        const bool stage32 = c->prec == GB_MIXED;
-        o->gjk_calls       = c->detect_valid ? (int64_t)q[0] : 0;
-        o->gjk_fp64_calls  = c->detect_valid ? (int64_t)q[stage32 ? 1 : 0] : 0;
+        // (the first queue holds each unordered pair once)
+        const bool queued  = c->detect_valid && !c->all_spheres;
+        o->gjk_calls       = queued ? 2 * (int64_t)q[0] : 0;
+        o->gjk_fp64_calls  = queued ? (int64_t)q[1] : 0;
         o->fine_grid_cells = c->fine ? (int64_t)c->fine_nf : 0;
     }
     if(c->detect_valid && c->npairs > 0)
@@ -2253,7 +2373,7 @@ int gb_get_stats(gb_ctx* c, gb_stats* o)
         // particle pairs only: obstacle candidates share the list
         std::vector<uint8_t>  pc(c->npairs);
         std::vector<uint32_t> pb(c->npairs);
-        GB_CK(cudaMemcpy(pc.data(), c->d_pc, c->npairs, cudaMemcpyDeviceToHost));
+        GB_CK(cudaMemcpy(pc.data(), c->d_pc[c->cur], c->npairs, cudaMemcpyDeviceToHost));
         GB_CK(cudaMemcpy(pb.data(), c->d_pb[c->cur], c->npairs * sizeof(uint32_t),
                          cudaMemcpyDeviceToHost));
         int64_t k = 0, obs = 0, ko = 0;
@@ -2353,7 +2473,7 @@ int gb_debug_dump(gb_ctx* c, int32_t kind, void* out, int64_t capacity, int64_t*
             {
                 GB_CK(cudaMemcpy(a.data(), c->d_pa, P * 4, cudaMemcpyDeviceToHost));
                 GB_CK(cudaMemcpy(b.data(), c->d_pb[c->cur], P * 4, cudaMemcpyDeviceToHost));
-                GB_CK(cudaMemcpy(pc.data(), c->d_pc, P, cudaMemcpyDeviceToHost));
+                GB_CK(cudaMemcpy(pc.data(), c->d_pc[c->cur], P, cudaMemcpyDeviceToHost));
             }
             std::vector<double> info;
             if(kind == GB_DUMP_CONTACT_INFO && P)
@@ -2587,11 +2707,11 @@ int gb_rawdata_write(gb_rawdata_writer* w, double time)
         uint32_t*       cn  = (w->flags & GB_RAW_COORDINATION_NUMBER) ? w->d_cn : nullptr;
         if(c->prec == GB_MIXED)
             k_raw_snapshot<float><<<blocks(n, kBlock), kBlock, 0, c->stream>>>(
-                n, c->d_pos, (const float*)c->d_vel, (const float*)c->d_omg, off, c->d_pc,
+                n, c->d_pos, (const float*)c->d_vel, (const float*)c->d_omg, off, c->d_pc[c->cur],
                 w->d_snap, cn);
         else
             k_raw_snapshot<double><<<blocks(n, kBlock), kBlock, 0, c->stream>>>(
-                n, c->d_pos, (const double*)c->d_vel, (const double*)c->d_omg, off, c->d_pc,
+                n, c->d_pos, (const double*)c->d_vel, (const double*)c->d_omg, off, c->d_pc[c->cur],
                 w->d_snap, cn);
         c->launches += 1;
         GB_CK(cudaGetLastError());

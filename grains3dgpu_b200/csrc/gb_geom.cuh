@@ -2,6 +2,8 @@
 // GJK with Johnson's sub-algorithm.
 #pragma once
 
+#include <cstring>
+
 #include "gb_math.cuh"
 #include "../../include/grains_b200.h"
 
@@ -13,7 +15,7 @@ namespace gb
 // on every call (Superquadric.cpp:169-205); each is the same IEEE value the
 // reference computes inline.
 template <typename St>
-struct RBShape
+struct alignas(16) RBShape
 {
     int32_t type;
     int32_t nverts;
@@ -61,20 +63,29 @@ template <typename S>
 GB_D Body<S> load_body(const RBShape<store_t<S>>* __restrict__ tab, uint32_t rb,
                        const Vert<store_t<S>>* __restrict__ verts)
 {
-    const RBShape<store_t<S>>* r = tab + rb;
-    Body<S>                    b;
-    b.type   = __ldg(&r->type);
-    b.nverts = __ldg(&r->nverts);
-    b.verts  = verts + __ldg(&r->first_vert);
+    // the record in 16-byte loads (six in FP32, eleven in FP64)
+    using Rec            = RBShape<store_t<S>>;
+    constexpr int kWords = sizeof(Rec) / sizeof(int4);
+    const int4*   src    = reinterpret_cast<const int4*>(tab + rb);
+    int4          w[kWords];
+#pragma unroll
+    for(int i = 0; i < kWords; ++i)
+        w[i] = __ldg(src + i);
+    Rec r;
+    memcpy(&r, w, sizeof(r));
+    Body<S> b;
+    b.type   = r.type;
+    b.nverts = r.nverts;
+    b.verts  = verts + r.first_vert;
 #pragma unroll
     for(int i = 0; i < 5; ++i)
-        b.p[i] = S(__ldg(&r->p[i]));
+        b.p[i] = S(r.p[i]);
 #pragma unroll
     for(int i = 0; i < 8; ++i)
-        b.k[i] = S(__ldg(&r->k[i]));
-    b.crust = S(__ldg(&r->crust));
-    b.rcirc = S(__ldg(&r->rcirc));
-    b.bb    = mk<S>(S(__ldg(&r->bb[0])), S(__ldg(&r->bb[1])), S(__ldg(&r->bb[2])));
+        b.k[i] = S(r.k[i]);
+    b.crust = S(r.crust);
+    b.rcirc = S(r.rcirc);
+    b.bb    = mk<S>(S(r.bb[0]), S(r.bb[1]), S(r.bb[2]));
     return b;
 }
 
@@ -327,6 +338,49 @@ GB_D bool obb_overlap(const V3<S>& a, const V3<S>& b, const M3<S>& RA, const M3<
 #undef O_
 #undef OA_
     return true;
+}
+
+// Whether obb_overlap of the same two boxes, evaluated in FP32 or FP64 and
+// with either body first, finds them apart: one of its 15 axes separates them
+// by more than `delta`.  The test is the same for both orders (the face axes
+// swap, a cross axis maps to its mirror), so only rounding tells them apart:
+// with c and the half extents within s = rA + rB, the FP32 rotations, their
+// product and the sums move either side of a test by less than 2e-6 s, a basis
+// off orthonormal by 2e-5 (the most a pose record admits) by some 4e-5 s, and
+// the caller's delta = 1e-4 s covers both.
+GB_D bool obb_apart(const V3<float>& a, const V3<float>& b, const M3<float>& RA,
+                    const M3<float>& RB, const V3<float>& d, float delta)
+{
+    const M3<float> oriT = transpose(RA);
+    const V3<float> cen  = mul(oriT, d);
+    const M3<float> ori  = mul(oriT, RB);
+    float           oa[9];
+#pragma unroll
+    for(int i = 0; i < 9; ++i)
+        oa[i] = fabsf(ori.m[i]) + k_loweps<float>();
+    const float A[3] = {a.x, a.y, a.z}, B[3] = {b.x, b.y, b.z}, c[3] = {cen.x, cen.y, cen.z};
+    float       gap = -INFINITY; // the largest separation over the axes
+#pragma unroll
+    for(int i = 0; i < 3; ++i)
+        gap = fmaxf(gap, fabsf(c[i])
+                             - (A[i] + B[0] * oa[3 * i] + B[1] * oa[3 * i + 1] + B[2] * oa[3 * i + 2]));
+#pragma unroll
+    for(int i = 0; i < 3; ++i)
+        gap = fmaxf(gap, fabsf(c[0] * ori.m[i] + c[1] * ori.m[3 + i] + c[2] * ori.m[6 + i])
+                             - (B[i] + A[0] * oa[i] + A[1] * oa[3 + i] + A[2] * oa[6 + i]));
+    if(gap > delta)
+        return true;
+#pragma unroll
+    for(int j = 0; j < 3; ++j)
+#pragma unroll
+        for(int i = 0; i < 3; ++i)
+        {
+            const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+            gap = fmaxf(gap, fabsf(c[i2] * ori.m[3 * i1 + j] - c[i1] * ori.m[3 * i2 + j])
+                                 - (A[i1] * oa[3 * i2 + j] + A[i2] * oa[3 * i1 + j]
+                                    + B[j1] * oa[3 * i + j2] + B[j2] * oa[3 * i + j1]));
+        }
+    return gap > delta;
 }
 
 // ---------------------------------------------------------------------------

@@ -47,6 +47,82 @@ struct Tables
     const RBShape<double>* shape64;
     const Vert<double>*    verts64;
     const RBShape<double>* obs_shape64;
+    // FP32 ones, read by the certified FP32 passes of every mode (the mixed
+    // mode's own tables; rounded copies in the FP64 modes)
+    const RBShape<float>* shape32;
+    const Vert<float>*    verts32;
+};
+
+// ---- records of the particles that have candidates ------------------------------
+// The narrow phase gathers its particles at random ids.  From the
+// structure-of-arrays state a particle's pose is seven to twelve 4- and 8-byte
+// loads in as many sectors, beside a dozen of its body record; the fill pass,
+// which runs over the particles that have candidates anyway, packs what the
+// culls read into one aligned record.  Pose: the centre, the body, and what
+// the oriented-box test reads in FP32 (the mixed mode's quaternion, the FP64
+// modes' basis).  `r` is the bounding radius: negative for a sphere, infinite
+// for a pose that the FP32 certificates do not cover (a basis off orthonormal
+// by more than 2e-5: its pairs all go to the FP64 solve).
+template <typename St>
+struct alignas(32) PoseRec // FP64 modes: 96 bytes, three sectors
+{
+    double   x, y, z;
+    uint32_t rb;
+    float    r;
+    float    R[9];
+    float    bb[3];
+    float    pad[4];
+};
+template <>
+struct alignas(32) PoseRec<float> // mixed: 64 bytes, two sectors
+{
+    double   x, y, z;
+    uint32_t rb;
+    float    r;
+    float    q[4];
+    float    bb[3];
+    float    pad;
+};
+
+// Spheres, where every body is one: all that a contact reads of a particle.
+template <typename St>
+struct alignas(32) SphereRec // 64 bytes mixed, 96 FP64
+{
+    double   x, y, z, r;
+    St       v[3], w[3], mass;
+    uint32_t material;
+};
+
+template <typename T>
+GB_D T load_rec(const T* p)
+{
+    constexpr int kWords = sizeof(T) / sizeof(int4);
+    int4          w[kWords];
+#pragma unroll
+    for(int k = 0; k < kWords; ++k)
+        w[k] = __ldg(reinterpret_cast<const int4*>(p) + k);
+    T t;
+    memcpy(&t, w, sizeof(t));
+    return t;
+}
+
+template <typename T>
+GB_D void store_rec(T* p, const T& t)
+{
+    constexpr int kWords = sizeof(T) / sizeof(int4);
+    int4          w[kWords];
+    memcpy(w, &t, sizeof(t));
+#pragma unroll
+    for(int k = 0; k < kWords; ++k)
+        reinterpret_cast<int4*>(p)[k] = w[k];
+}
+
+// the records' arrays, by particle id; null where the step does not read them
+template <typename St>
+struct Records
+{
+    PoseRec<St>*   pose;
+    SphereRec<St>* sphere;
 };
 
 // ---- mixed precision narrow phase --------------------------------------------
@@ -86,11 +162,10 @@ GB_D Contact<float> to_f(const Contact<double>& c)
 
 // closestPointsSpheres (CollisionDetection.cpp:26-48) for the mixed mode:
 // the closed form directly in FP64, the point relative to A's centre.
-GB_D Contact<float> closest_spheres_mixed(const Tables<float>& tb, uint32_t ra, uint32_t rb,
-                                          const double xa[3], const double xb[3])
+GB_D Contact<float> closest_spheres_mixed(double rA, double rB, const double xa[3],
+                                          const double xb[3])
 {
     const V3<double> d64 = mk<double>(xb[0] - xa[0], xb[1] - xa[1], xb[2] - xa[2]);
-    const double     rA = tb.shape64[ra].p[0], rB = tb.shape64[rb].p[0]; // the radii
     const double     nd = norm(d64), overlap = nd - rA - rB;
     if(!(overlap < 0.0))
         return no_contact<float>();
@@ -112,7 +187,7 @@ GB_D Contact<float> closest_mixed(const Tables<float>& tb, const State<float>& s
 {
     const V3<double> d64 = mk<double>(xb[0] - xa[0], xb[1] - xa[1], xb[2] - xa[2]);
     if(A.type == GB_SPHERE && B.type == GB_SPHERE)
-        return closest_spheres_mixed(tb, ra, rb, xa, xb);
+        return closest_spheres_mixed(tb.shape64[ra].p[0], tb.shape64[rb].p[0], xa, xb);
     const V3<float> d = cvt3<float>(d64);
     if(!(norm(d) - (A.rcirc + B.rcirc) < 0.0f))
         return no_contact<float>();
@@ -871,11 +946,79 @@ GB_D void bitonic_sort(uint32_t (&t)[M])
             }
 }
 
+// Particle a's pose or sphere record (Records).
+template <typename S>
+GB_D void write_records(uint32_t a, const State<store_t<S>>& st, const Tables<S>& tb,
+                        const Records<store_t<S>>& rec)
+{
+    using St          = store_t<S>;
+    const uint32_t rb = st.rb_id[a];
+    if(rec.sphere)
+    {
+        SphereRec<St> o;
+        o.x = st.pos[0][a];
+        o.y = st.pos[1][a];
+        o.z = st.pos[2][a];
+        o.r = tb.shape64[rb].p[0];
+#pragma unroll
+        for(int k = 0; k < 3; ++k)
+        {
+            o.v[k] = st.vel[k][a];
+            o.w[k] = st.omg[k][a];
+        }
+        o.mass     = tb.inertia[rb].mass;
+        o.material = (uint32_t)tb.shape[rb].material;
+        store_rec(rec.sphere + a, o);
+    }
+    if(rec.pose)
+    {
+        const RBShape<float>& sh = tb.shape32[rb];
+        PoseRec<St>           o;
+        o.x  = st.pos[0][a];
+        o.y  = st.pos[1][a];
+        o.z  = st.pos[2][a];
+        o.rb = rb;
+        o.r  = sh.type == GB_SPHERE ? -sh.rcirc : sh.rcirc;
+        if constexpr(is_mixed<S>())
+        {
+#pragma unroll
+            for(int k = 0; k < 4; ++k)
+                o.q[k] = st.rot[k][a];
+        }
+        else
+        {
+#pragma unroll
+            for(int k = 0; k < 9; ++k)
+                o.R[k] = (float)st.rot[k][a];
+            // the certificates hold for both orders of a pair, whose frames
+            // agree only as far as the bases are rotations
+            bool ok = true;
+#pragma unroll
+            for(int i = 0; i < 3; ++i)
+#pragma unroll
+                for(int j = i; j < 3; ++j)
+                {
+                    const float g = o.R[3 * i] * o.R[3 * j] + o.R[3 * i + 1] * o.R[3 * j + 1]
+                                    + o.R[3 * i + 2] * o.R[3 * j + 2];
+                    ok = ok && fabsf(g - (i == j ? 1.0f : 0.0f)) < 2e-5f;
+                }
+            if(!ok && sh.type != GB_SPHERE)
+                o.r = INFINITY;
+        }
+#pragma unroll
+        for(int k = 0; k < 3; ++k)
+            o.bb[k] = sh.bb[k];
+        store_rec(rec.pose + a, o);
+    }
+}
+
 // Fill pass, one thread per particle id a (most have no candidate and read
 // only count[a]): the pair records of a at offset[a] -- its particle
 // candidates from the slots of its sorted position s = sorted_of[a], sorted
 // ascending (the enumeration order), or enumerated again in order when there
-// were more than kPairSlots -- then its obstacle candidates.
+// were more than kPairSlots -- then its obstacle candidates.  Every record's
+// contact flag starts at 0, so that the narrow phase writes the records of
+// contacts only (outputs are read where the flag is set).
 template <typename S>
 __global__ void __launch_bounds__(kBlock)
     k_pair_fill(int n, const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ sids,
@@ -886,14 +1029,16 @@ __global__ void __launch_bounds__(kBlock)
                 const uint32_t* __restrict__ offset, uint32_t* __restrict__ pair_a,
                 uint32_t* __restrict__ pair_b, int64_t cap, int* __restrict__ flags,
                 uint32_t* __restrict__ gjk_count, uint32_t* __restrict__ pslot,
-                uint32_t* __restrict__ ovf_list, int ovf_phase, uint32_t* __restrict__ obs_queue)
+                uint32_t* __restrict__ ovf_list, int ovf_phase, uint32_t* __restrict__ obs_queue,
+                uint8_t* __restrict__ contact, State<store_t<S>> st, Tables<S> tb,
+                Records<store_t<S>> rec)
 {
     grid_dep_sync();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if(a == 0)
     {
         // the narrow phase's GJK queues of this step start empty: [0] the
-        // cull pass's, [1] the mixed mode's FP32 stage's; [2 + phase] counts
+        // cull pass's, [1] the FP32 stage's; [2 + phase] counts
         // this step's overflowing particles and [4 + phase] its obstacle
         // records, [3 - phase] and [5 - phase] (last step's, read by its
         // overflow and obstacle passes) start the next step at zero
@@ -951,8 +1096,9 @@ __global__ void __launch_bounds__(kBlock)
         for(int k = 0; k < kPairSlots; ++k)
             if((uint32_t)k < cp)
             {
-                pair_a[out + k] = a;
-                pair_b[out + k] = sids[t[k]];
+                pair_a[out + k]  = a;
+                pair_b[out + k]  = sids[t[k]];
+                contact[out + k] = 0;
             }
         out += cp;
     }
@@ -973,10 +1119,13 @@ __global__ void __launch_bounds__(kBlock)
             obs_queue[q + j] = (uint32_t)out + j;
     }
     for_each_obstacle_candidate(oc, a, (uint32_t)s, [&](uint32_t o) {
-        pair_a[out] = a;
-        pair_b[out] = kObstacleBit | o;
+        pair_a[out]  = a;
+        pair_b[out]  = kObstacleBit | o;
+        contact[out] = 0;
         ++out;
     });
+    if(cp)
+        write_records<S>((uint32_t)a, st, tb, rec);
 }
 
 // The particle pairs of the particles whose partners overflowed their slots,
@@ -992,7 +1141,8 @@ __global__ void __launch_bounds__(128)
                          const double4* __restrict__ spos, const float4* __restrict__ spos32,
                          const uint32_t* __restrict__ cstart, uint32_t nx, uint32_t ny, uint32_t nz,
                          const uint32_t* __restrict__ offset, uint32_t* __restrict__ pair_a,
-                         uint32_t* __restrict__ pair_b, const int* __restrict__ flags)
+                         uint32_t* __restrict__ pair_b, uint8_t* __restrict__ contact,
+                         const int* __restrict__ flags)
 {
     grid_dep_sync();
     constexpr bool STRICT = is_strict<S>(), PRE32 = is_mixed<S>();
@@ -1027,6 +1177,7 @@ __global__ void __launch_bounds__(128)
                 const uint32_t k = out + __popc(bits & ((1u << lane) - 1u));
                 pair_a[k]        = a;
                 pair_b[k]        = sids[t];
+                contact[k]       = 0;
             }
             out += __popc(bits);
         });
@@ -1040,24 +1191,42 @@ struct PairOut
     St*      f[3];
     St*      t[3];
     St*      m[3];     // rolling moment (only when some kr != 0)
-    uint8_t* contact;  // kContactParticle / kContactObstacle when overlap < 0, else 0
-    uint32_t* pcount;  // contacts per particle id (zero before the narrow phase; the
-                       // per-particle kernel reads and clears them)
+    uint8_t* contact;  // kContactParticle / kContactObstacle when overlap < 0, else 0 (set
+                       // to 0 by the fill pass; the other outputs are written, and
+                       // read, for contacts only)
+    uint32_t* pcount;  // 1 where particle id has a contact (zero before the narrow phase;
+                       // the per-particle kernel reads and clears it)
     double*  info;     // optional: 7 per pair (point, vector, overlap) in world frame
     // tangential history (history law): current step out, previous step in
     St*             xi[3];
     const uint32_t* prev_off;
     const uint32_t* prev_b;
+    const uint8_t*  prev_contact;
     const St*       prev_xi[3];
 };
 
-// the outputs of pair p: force, torque, rolling moment, spring, contact flag,
-// and (when recorded) the contact point in world frame, vector and overlap
+// the tangential spring of the pair (a, b) at the end of the last step (zero
+// where it was no contact)
 template <typename S>
-GB_D void store_pair(const PairOut<store_t<S>>& po, int64_t p, const Force<S>& F,
+GB_D V3<S> previous_spring(const PairOut<store_t<S>>& po, uint32_t a, uint32_t b)
+{
+    for(uint32_t k = po.prev_off[a]; k < po.prev_off[a + 1]; ++k)
+        if(po.prev_b[k] == b)
+            return po.prev_contact[k]
+                       ? mk<S>(S(po.prev_xi[0][k]), S(po.prev_xi[1][k]), S(po.prev_xi[2][k]))
+                       : zero3<S>();
+    return zero3<S>();
+}
+
+// the outputs of contact p of particle a: force, torque, rolling moment,
+// spring, contact flag, and (when recorded) the contact point in world frame,
+// vector and overlap
+template <typename S>
+GB_D void store_pair(const PairOut<store_t<S>>& po, int64_t p, uint32_t a, const Force<S>& F,
                      const V3<S>& xi_new, uint8_t flag, int law_kind, int has_kr,
                      const Contact<S>& ci, const double xa[3])
 {
+    po.pcount[a] = 1u;
 #pragma unroll
     for(int k = 0; k < 3; ++k)
     {
@@ -1172,11 +1341,9 @@ GB_D void narrow_obstacle(int64_t p, uint32_t a, int o, const State<store_t<S>>&
         ci = closest_drum(A, RA, oA, oO, mk<S>(RO.m[2], RO.m[5], RO.m[8]), O.p[0]);
     else if constexpr(GEN)
         ci = closest_points<VAR>(A, O, RA, RO, oA, oO, oO - oA, &iters);
-    const bool hit = ci.overlap < S(0.0);
-    Force<S>   F;
-    F.f = F.t = F.m = zero3<S>();
-    if(hit)
+    if(ci.overlap < S(0.0))
     {
+        Force<S>     F;
         const Law<S> L  = load_law<S>(tb.law, tb.shape[ra].material, tb.obs_shape[o].material);
         const S      m1 = S(tb.inertia[ra].mass);
         const S      m2 = S(tb.obs_mass[o]);
@@ -1211,41 +1378,10 @@ GB_D void narrow_obstacle(int64_t p, uint32_t a, int o, const State<store_t<S>>&
                               arm);
         }
         atomicAdd(&counters[0], 1ull);
+        store_pair<S>(po, p, a, F, zero3<S>(), kContactObstacle, law_kind, has_kr, ci, xa);
     }
-    store_pair<S>(po, p, F, zero3<S>(), hit ? kContactObstacle : uint8_t(0), law_kind, has_kr, ci,
-                  xa);
-    if(hit)
-        atomicAdd(po.pcount + a, 1u);
     if(iters)
         atomicAdd(&counters[1], (unsigned long long)iters);
-}
-
-// particle pair record p (obstacle records are k_narrow_obstacles'); VAR: the GJK
-// Whether a particle pair reaches GJK: the bounding tests of
-// closestPointsRigidBodies (CollisionDetection.cpp:195-228) as closest_mixed
-// and closest_points evaluate them -- not two spheres (closed form), bounding
-// spheres overlapping, OBBs overlapping -- so that the GJK pass repeats
-// exactly these decisions.
-template <typename S>
-GB_D bool needs_gjk(const Body<S>& A, const Body<S>& B, const M3<S>& RA, const M3<S>& RB,
-                    const double xa[3], const double xb[3], const V3<S>& d)
-{
-    if(A.type == GB_SPHERE && B.type == GB_SPHERE)
-        return false;
-    if constexpr(is_mixed<S>())
-    {
-        const V3<double> d64 = mk<double>(xb[0] - xa[0], xb[1] - xa[1], xb[2] - xa[2]);
-        const V3<float>  df  = cvt3<float>(d64);
-        if(!(norm(df) - (A.rcirc + B.rcirc) < 0.0f))
-            return false;
-        return obb_overlap(A.bb, B.bb, RA, RB, df);
-    }
-    else
-    {
-        if(!(norm(d) - (A.rcirc + B.rcirc) < S(0.0)))
-            return false;
-        return obb_overlap(A.bb, B.bb, RA, RB, d);
-    }
 }
 
 // The first iteration of GJK-JH (gjk_jh, GJK_JH.cpp:332-371), where it
@@ -1258,42 +1394,43 @@ GB_D bool needs_gjk(const Body<S>& A, const Body<S>& B, const M3<S>& RA, const M
 //     contact;
 //   g < -margin: mu stays 0 < the absolute tolerance, GJK stops at this
 //     iteration and returns |v|; if that exceeds the crusts: no contact.
-// Every other pair (in particular every contact) takes the full GJK.  The
-// FP64 modes evaluate exactly GJK's first iteration, with a margin far
-// above FP64 rounding; the mixed mode evaluates it in FP32 (supports,
-// frames and dot products), with a margin of 1e-4 of the bounding radii,
-// some 20 times a bound on the FP32 error of g (support values are
-// Lipschitz in the direction with constant |x| <= R_circ, so the FP32
-// direction error of ~3e-7 moves them by < 1e-9 m; the FP32 supports and
-// frames add a few 1e-9 m): a pair decided here is one that the FP64 GJK
-// also finds out of contact, so the mixed mode's contact set and contact
-// geometry stay those of its FP64 GJK.
+// Every other pair (in particular every contact) takes the full GJK.  It is
+// evaluated in FP32 in every mode (supports, frames and dot products), with a
+// margin of 1e-4 of the bounding radii, some 20 times a bound on the FP32
+// error of g (support values are Lipschitz in the direction with constant
+// |x| <= R_circ, so the FP32 direction error of ~3e-7 moves them by < 1e-9 m;
+// the FP32 supports and frames add a few 1e-9 m): a pair decided here is one
+// that the FP64 GJK also finds out of contact, so the contact set and the
+// contact geometry stay those of the FP64 GJK.  Both rules are the same for
+// (A, B) and (B, A): the pair of the other order has v and w mirrored, so
+// each unordered pair is decided once, for both its records.
 // The first rule holds for every GJK variant (each returns the norm of a
 // point of the Minkowski difference, at least the true distance, which g
 // bounds from below); the second is GJK-JH's own stopping rule (JH_RULE).
-template <typename S, bool JH_RULE = true>
-GB_D bool gjk_first_iteration_separates(const Body<S>& A, const Body<S>& B, const M3<S>& RA,
-                                        const M3<S>& RB, const V3<S>& d)
+// `s` is the sum of the bounding radii (infinite: nothing is decided).
+template <bool JH_RULE>
+GB_D bool gjk_first_iteration_separates(const Body<float>& A, const Body<float>& B,
+                                        const M3<float>& RA, const M3<float>& RB,
+                                        const V3<float>& d, float s)
 {
-    Tr<S>       b2a;
-    const M3<S> RAt = transpose(RA);
-    b2a.R           = mul(RAt, RB);
-    b2a.o           = mul(RAt, d);
-    const V3<S> s0A = support(A, zero3<S>()), s0B = support(B, zero3<S>());
-    const V3<S> v   = s0A - apply(b2a, s0B);
-    const S     dist = norm(v);
-    const V3<S> pa = support_first(A, -v), qb = support_first(B, mul_t(b2a.R, v));
-    const V3<S> w  = pa - apply(b2a, qb);
-    const S     g  = dot(v, w) / dist;
-    const S     ct = A.crust + B.crust;
-    const S     margin = is_mixed<S>() ? S(1e-4) * (A.rcirc + B.rcirc) + S(1e-9)
-                                       : S(1e-9) * (A.rcirc + B.rcirc) + S(1e-15);
+    Tr<float>       b2a;
+    const M3<float> RAt = transpose(RA);
+    b2a.R               = mul(RAt, RB);
+    b2a.o               = mul(RAt, d);
+    const V3<float> s0A = support(A, zero3<float>()), s0B = support(B, zero3<float>());
+    const V3<float> v    = s0A - apply(b2a, s0B);
+    const float     dist = norm(v);
+    const V3<float> pa = support_first(A, -v), qb = support_first(B, mul_t(b2a.R, v));
+    const V3<float> w  = pa - apply(b2a, qb);
+    const float     g  = dot(v, w) / dist;
+    const float     ct = A.crust + B.crust;
+    const float     margin = 1e-4f * s + 1e-9f;
     if(g > ct + margin)
         return true;
     return JH_RULE && g < -margin && dist - ct > margin;
 }
 
-// ---- the mixed mode's FP32 GJK stage ------------------------------------------
+// ---- the FP32 GJK stage ------------------------------------------
 // Closest point to the origin of the segment (a, b) or the triangle (a, b, c)
 // (Ericson, Real-Time Collision Detection, 5.1.2 and 5.1.5, by Voronoi
 // regions), with the vertices of the feature it lies on put in y0..y(n-1).
@@ -1394,14 +1531,14 @@ constexpr int kGjk32MaxIter = 24;
 // converged below the crusts (a contact or a near miss), reached the
 // origin, left the finite range, or ran out of iterations.
 GB_D bool gjk_fp32_separates(const Body<float>& A, const Body<float>& B, const M3<float>& RA,
-                             const M3<float>& RB, const V3<float>& d)
+                             const M3<float>& RB, const V3<float>& d, float s)
 {
     Tr<float>       b2a;
     const M3<float> RAt = transpose(RA);
     b2a.R               = mul(RAt, RB);
     b2a.o               = mul(RAt, d);
     const float ct      = A.crust + B.crust;
-    const float margin  = 1e-4f * (A.rcirc + B.rcirc) + 1e-9f;
+    const float margin  = 1e-4f * s + 1e-9f;
     V3<float>   y0 = support(A, zero3<float>()) - apply(b2a, support(B, zero3<float>()));
     V3<float>   y1 = y0, y2 = y0;
     int         n  = 1;
@@ -1466,27 +1603,51 @@ GB_D bool gjk_fp32_separates(const Body<float>& A, const Body<float>& B, const M
     return false;
 }
 
-// Pair record p: contact detection, contact law, outputs.  QUEUE (the cull
-// pass, k_narrow): the pair is finished here when it is two spheres (closed
-// form) or out of contact by the bounding tests or GJK-JH's first iteration,
-// and queued for the GJK pass otherwise -- no GJK is compiled into this
-// pass, which keeps its registers low.  Without QUEUE (k_narrow_gjk): the
-// full closestPointsRigidBodies.
-template <typename S, int VAR, bool QUEUE = false>
-GB_D void narrow_pair(int64_t p, const uint32_t* __restrict__ pair_a,
-                      const uint32_t* __restrict__ pair_b, const State<store_t<S>>& st,
-                      const Tables<S>& tb, const PairOut<store_t<S>>& po, int law_kind, int has_kr,
-                      S dt, unsigned long long* __restrict__ counters,
-                      uint32_t* __restrict__ gjk_queue = nullptr,
-                      uint32_t* __restrict__ gjk_count = nullptr)
+// The contact law for contact `ci` of the particle pair record p = (a, b) and
+// its outputs.  B's centre is at oB in the working coordinates.
+template <typename S>
+GB_D void pair_contact(int64_t p, uint32_t a, uint32_t b, const Law<S>& L, S m1, S m2,
+                       const V3<S>& vA, const V3<S>& vB, const V3<S>& wA, const V3<S>& wB,
+                       const V3<S>& oA, const V3<S>& oB, const Contact<S>& ci, const double xa[3],
+                       const PairOut<store_t<S>>& po, int law_kind, int has_kr, S dt)
 {
-    const uint32_t a = pair_a[p], b = pair_b[p];
-    if(b & kObstacleBit) // k_narrow_obstacles
-        return;
+    Force<S> F;
+    V3<S>    xi_new = zero3<S>();
+    // arm = contact point - A's centre
+    V3<S> arm, ptw;
+    if constexpr(is_mixed<S>())
+    {
+        arm = ci.pt;
+        ptw = mk<S>(S(xa[0] + to_d(ci.pt.x)), S(xa[1] + to_d(ci.pt.y)), S(xa[2] + to_d(ci.pt.z)));
+    }
+    else
+    {
+        arm = ci.pt - oA;
+        ptw = ci.pt;
+    }
+    if(law_kind == GB_LAW_HOOKE)
+    {
+        // Kinematics::kinematicsAtPoint with the absolute contact point
+        const V3<S> rel = (vA + cross(wA, ptw)) - (vB + cross(wB, ptw));
+        F               = hooke(L, ci, rel, wA - wB, m1, m2, arm);
+    }
+    else
+    {
+        const V3<S> armB = ci.pt - oB;
+        const V3<S> rel  = (vA + cross(wA, arm)) - (vB + cross(wB, armB));
+        F = hooke_history(L, ci, rel, m1, m2, dt, previous_spring<S>(po, a, b), xi_new, arm);
+    }
+    store_pair<S>(po, p, a, F, xi_new, kContactParticle, law_kind, has_kr, ci, xa);
+}
+
+// Pair record p: closestPointsRigidBodies, contact law, outputs.  SPHERES: a
+// pair of spheres, whose closed form needs no rotation and no body record.
+template <typename S, int VAR, bool SPHERES = false>
+GB_D void narrow_pair(int64_t p, uint32_t a, uint32_t b, const State<store_t<S>>& st,
+                      const Tables<S>& tb, const PairOut<store_t<S>>& po, int law_kind, int has_kr,
+                      S dt, unsigned long long* __restrict__ counters)
+{
     const uint32_t ra = st.rb_id[a], rb = st.rb_id[b];
-    const Body<S>  A = load_body<S>(tb.shape, ra, tb.verts);
-    const Body<S>  B = load_body<S>(tb.shape, rb, tb.verts);
-    const M3<S>    RA = load_rot<S>(st, a), RB = load_rot<S>(st, b);
     const double   xa[3] = {st.pos[0][a], st.pos[1][a], st.pos[2][a]};
     const double   xb[3] = {st.pos[0][b], st.pos[1][b], st.pos[2][b]};
     V3<S>          oA, oB, d;
@@ -1504,81 +1665,32 @@ GB_D void narrow_pair(int64_t p, const uint32_t* __restrict__ pair_a,
     }
     int        iters = 0;
     Contact<S> ci;
-    if constexpr(QUEUE)
+    if constexpr(SPHERES)
     {
-        constexpr bool JH = (VAR & ~kGjkPaired) == GB_GJK_JH;
-        if(A.type == GB_SPHERE && B.type == GB_SPHERE)
-        {
-            if constexpr(is_mixed<S>())
-                ci = closest_spheres_mixed(tb, ra, rb, xa, xb);
-            else
-                ci = closest_spheres(A, B, oA, oB);
-        }
-        else if(!needs_gjk<S>(A, B, RA, RB, xa, xb, d)
-                || (JH && gjk_first_iteration_separates<S, true>(A, B, RA, RB, d))
-                || (!JH && is_mixed<S>()
-                    && gjk_first_iteration_separates<S, false>(A, B, RA, RB, d)))
-            ci = no_contact<S>();
-        else
-        {
-            // the GJK pass (k_narrow_gjk) takes this pair and stores its outputs
-            gjk_queue[atomicAdd(gjk_count, 1u)] = (uint32_t)p;
-            return;
-        }
-    }
-    else if constexpr(is_mixed<S>())
-        ci = closest_mixed<VAR>(tb, st, a, b, ra, rb, A, B, RA, RB, xa, xb, &iters);
-    else
-        ci = closest_points<VAR>(A, B, RA, RB, oA, oB, d, &iters);
-    const bool hit = ci.overlap < S(0.0);
-    Force<S>         F;
-    F.f = F.t = F.m = zero3<S>();
-    V3<S> xi_new    = zero3<S>();
-    if(hit)
-    {
-        const Law<S> L  = load_law<S>(tb.law, tb.shape[ra].material, tb.shape[rb].material);
-        const S      m1 = S(tb.inertia[ra].mass), m2 = S(tb.inertia[rb].mass);
-        const V3<S>  vA = load3<S>(st.vel, a), vB = load3<S>(st.vel, b);
-        const V3<S>  wA = load3<S>(st.omg, a), wB = load3<S>(st.omg, b);
-        // arm = contact point - A's centre
-        V3<S> arm, ptw;
+        const double rA = tb.shape64[ra].p[0], rB = tb.shape64[rb].p[0];
         if constexpr(is_mixed<S>())
-        {
-            arm = ci.pt;
-            ptw = mk<S>(S(xa[0] + to_d(ci.pt.x)), S(xa[1] + to_d(ci.pt.y)),
-                        S(xa[2] + to_d(ci.pt.z)));
-        }
+            ci = closest_spheres_mixed(rA, rB, xa, xb);
         else
-        {
-            arm = ci.pt - oA;
-            ptw = ci.pt;
-        }
-        if(law_kind == GB_LAW_HOOKE)
-        {
-            // Kinematics::kinematicsAtPoint with the absolute contact point
-            const V3<S> rel = (vA + cross(wA, ptw)) - (vB + cross(wB, ptw));
-            F               = hooke(L, ci, rel, wA - wB, m1, m2, arm);
-        }
+            ci = closest_spheres(S(rA), S(rB), oA, oB);
+    }
+    else
+    {
+        const Body<S> A  = load_body<S>(tb.shape, ra, tb.verts);
+        const Body<S> B  = load_body<S>(tb.shape, rb, tb.verts);
+        const M3<S>   RA = load_rot<S>(st, a), RB = load_rot<S>(st, b);
+        if constexpr(is_mixed<S>())
+            ci = closest_mixed<VAR>(tb, st, a, b, ra, rb, A, B, RA, RB, xa, xb, &iters);
         else
-        {
-            const V3<S> armB = is_mixed<S>() ? ci.pt - d : ci.pt - oB;
-            const V3<S> rel  = (vA + cross(wA, arm)) - (vB + cross(wB, armB));
-            V3<S>       xi_prev = zero3<S>();
-            for(uint32_t k = po.prev_off[a]; k < po.prev_off[a + 1]; ++k)
-                if(po.prev_b[k] == b)
-                {
-                    xi_prev = mk<S>(S(po.prev_xi[0][k]), S(po.prev_xi[1][k]), S(po.prev_xi[2][k]));
-                    break;
-                }
-            F = hooke_history(L, ci, rel, m1, m2, dt, xi_prev, xi_new, arm);
-        }
+            ci = closest_points<VAR>(A, B, RA, RB, oA, oB, d, &iters);
     }
     // a lane pair (kGjkPaired) holds the same results: its even lane stores them
     if((VAR & kGjkPaired) && (threadIdx.x & 1u))
         return;
-    store_pair<S>(po, p, F, xi_new, hit ? kContactParticle : uint8_t(0), law_kind, has_kr, ci, xa);
-    if(hit)
-        atomicAdd(po.pcount + a, 1u);
+    if(ci.overlap < S(0.0))
+        pair_contact<S>(p, a, b, load_law<S>(tb.law, tb.shape[ra].material, tb.shape[rb].material),
+                        S(tb.inertia[ra].mass), S(tb.inertia[rb].mass), load3<S>(st.vel, a),
+                        load3<S>(st.vel, b), load3<S>(st.omg, a), load3<S>(st.omg, b), oA, oB, ci,
+                        xa, po, law_kind, has_kr, dt);
     if(iters)
         atomicAdd(&counters[1], (unsigned long long)iters);
 }
@@ -1609,39 +1721,259 @@ GB_D void for_each_pair(int64_t npairs, F&& f)
             f(p);
 }
 
-// The particle-particle narrow phase in two passes.  k_narrow walks the pair
-// list (its length is read on the device, *total, the scan's grand total, so
-// the host launches a resident-sized grid without waiting for it): every
-// pair that its bounding tests cull, and every sphere pair, is finished
-// there; a pair that needs GJK goes to a queue instead.  k_narrow_gjk then
-// spreads the queue -- a few hundred to a few thousand pairs -- over all
-// resident warps, so that a warp holds one or two GJK chains rather than
-// every GJK pair among 32 consecutive records of the list.
-template <typename S, int VAR>
-__global__ void __launch_bounds__(128, sizeof(store_t<S>) == 4 ? 5 : 1)
+// The narrow phase of a run whose bodies are all spheres: every record's
+// closed form and law in one pass, one thread per record, from the sphere
+// records of the fill pass (two to three sectors a particle, where the
+// structure-of-arrays state costs a sector per component).
+template <typename S>
+__global__ void __launch_bounds__(kBlock)
+    k_narrow_spheres(const uint32_t* __restrict__ total, const int* __restrict__ flags,
+                     const uint32_t* __restrict__ pair_a, const uint32_t* __restrict__ pair_b,
+                     const SphereRec<store_t<S>>* __restrict__ rec, Tables<S> tb,
+                     PairOut<store_t<S>> po, int law_kind, int has_kr, S dt)
+{
+    grid_dep_sync();
+    if(step_aborted(flags))
+        return;
+    const int64_t np = *total, stride = (int64_t)gridDim.x * blockDim.x;
+    for(int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += stride)
+    {
+        const uint32_t a = pair_a[p], b = pair_b[p];
+        if(b & kObstacleBit) // k_narrow_obstacles
+            continue;
+        const SphereRec<store_t<S>> A = load_rec(rec + a), B = load_rec(rec + b);
+        const double                xa[3] = {A.x, A.y, A.z}, xb[3] = {B.x, B.y, B.z};
+        V3<S>                       oA, oB;
+        Contact<S>                  ci;
+        if constexpr(is_mixed<S>())
+        {
+            oA = zero3<S>();
+            oB = mk<S>(S(xb[0] - xa[0]), S(xb[1] - xa[1]), S(xb[2] - xa[2]));
+            ci = closest_spheres_mixed(A.r, B.r, xa, xb);
+        }
+        else
+        {
+            oA = mk<S>(S(A.x), S(A.y), S(A.z));
+            oB = mk<S>(S(B.x), S(B.y), S(B.z));
+            ci = closest_spheres(S(A.r), S(B.r), oA, oB);
+        }
+        if(!(ci.overlap < S(0.0)))
+            continue;
+        pair_contact<S>(p, a, b, load_law<S>(tb.law, (int)A.material, (int)B.material), S(A.mass),
+                        S(B.mass), mk<S>(S(A.v[0]), S(A.v[1]), S(A.v[2])),
+                        mk<S>(S(B.v[0]), S(B.v[1]), S(B.v[2])),
+                        mk<S>(S(A.w[0]), S(A.w[1]), S(A.w[2])),
+                        mk<S>(S(B.w[0]), S(B.w[1]), S(B.w[2])), oA, oB, ci, xa, po, law_kind,
+                        has_kr, dt);
+    }
+}
+
+// the pose record of a particle for the FP32 passes
+struct Pose32
+{
+    double    x, y, z;
+    uint32_t  rb;
+    float     r;
+    M3<float> R;
+    V3<float> bb;
+};
+
+template <typename St>
+GB_D Pose32 load_pose(const PoseRec<St>* __restrict__ rec, uint32_t i)
+{
+    const PoseRec<St> o = load_rec(rec + i);
+    Pose32            p;
+    p.x  = o.x;
+    p.y  = o.y;
+    p.z  = o.z;
+    p.rb = o.rb;
+    p.r  = o.r;
+    p.bb = mk<float>(o.bb[0], o.bb[1], o.bb[2]);
+    if constexpr(sizeof(St) == 4)
+        p.R = quat_to_matrix<float>(o.q[0], o.q[1], o.q[2], o.q[3]);
+    else
+    {
+#pragma unroll
+        for(int k = 0; k < 9; ++k)
+            p.R.m[k] = o.R[k];
+    }
+    return p;
+}
+
+GB_D V3<float> centre_difference(const Pose32& A, const Pose32& B)
+{
+    return mk<float>(float(B.x - A.x), float(B.y - A.y), float(B.z - A.z));
+}
+
+// the record (b, a) of record (a, b): b's records hold the mirror of each of
+// a's (the candidate test is symmetric); kNoRecord, never expected, if not
+constexpr uint32_t kNoRecord = 0xffffffffu;
+
+GB_D uint32_t mirror_record(const uint32_t* __restrict__ off, const uint32_t* __restrict__ pair_b,
+                            uint32_t a, uint32_t b)
+{
+    for(uint32_t k = off[b], e = off[b + 1]; k < e; ++k)
+        if(pair_b[k] == a)
+            return k;
+    return kNoRecord;
+}
+
+// A warp's queue of pairs in shared memory: lanes push what they keep, packed
+// by a ballot, and the warp pops 32 at a time, so that each stage of the cull
+// runs with all lanes busy whatever the stage before it left.
+struct WarpQueue
+{
+    uint32_t p[64], a[64], b[64];
+};
+
+GB_D void warp_push(WarpQueue& q, unsigned& n, bool take, uint32_t p, uint32_t a, uint32_t b)
+{
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if(take)
+    {
+        const unsigned k = n + __popc(m & ((1u << (threadIdx.x & 31u)) - 1u));
+        q.p[k]           = p;
+        q.a[k]           = a;
+        q.b[k]           = b;
+    }
+    n += __popc(m);
+    __syncwarp();
+}
+
+// The last min(n, 32) entries of the queue, one per lane; false on the lanes
+// past them.
+GB_D bool warp_pop(const WarpQueue& q, unsigned& n, uint32_t& p, uint32_t& a, uint32_t& b)
+{
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned k    = n < 32u ? n : 32u;
+    const bool     mine = lane < k;
+    n -= k;
+    if(mine)
+    {
+        p = q.p[n + lane];
+        a = q.a[n + lane];
+        b = q.b[n + lane];
+    }
+    __syncwarp();
+    return mine;
+}
+
+// The cull, k_narrow: every unordered candidate pair once, in FP32, in stages
+// that a warp runs on packed lanes (WarpQueue): its record (a, b) with a < b
+// is taken from the list; two spheres are solved for both records (closed
+// form); a sphere against another shape is no contact (the reference's GJK
+// starts from Sphere::support(0), whose 0/0 makes every distance NaN:
+// Sphere.cpp:111); the oriented boxes, then GJK's first iteration, drop the
+// pairs that both records' FP64 tests drop; what is left goes to gjk_queue as
+// record p (k_narrow_gjk32).  Decisions are certified (obb_apart,
+// gjk_first_iteration_separates), so every mode, the bit-exact one included,
+// keeps the contacts of its own FP64 tests, which the last pass repeats for
+// each record it solves.
+template <typename S, bool JH_RULE, bool SPHERES>
+__global__ void __launch_bounds__(128, 5)
     k_narrow(const uint32_t* __restrict__ total, const int* __restrict__ flags,
              const uint32_t* __restrict__ pair_a, const uint32_t* __restrict__ pair_b,
+             const uint32_t* __restrict__ off, const PoseRec<store_t<S>>* __restrict__ pose,
              State<store_t<S>> st, Tables<S> tb, PairOut<store_t<S>> po, int law_kind, int has_kr,
              S dt, unsigned long long* __restrict__ counters, uint32_t* __restrict__ gjk_queue,
              uint32_t* __restrict__ gjk_count)
 {
     grid_dep_sync();
+    __shared__ WarpQueue s_boxes[4], s_first[4], s_sphere[SPHERES ? 4 : 1];
     if(step_aborted(flags))
         return;
-    for_each_pair(*total, [&](int64_t p) {
-        narrow_pair<S, VAR, true>(p, pair_a, pair_b, st, tb, po, law_kind, has_kr, dt, counters,
-                            gjk_queue, gjk_count);
-    });
+    const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    WarpQueue &    boxes = s_boxes[w], &first = s_first[w], &sphere = s_sphere[SPHERES ? w : 0];
+    unsigned       nboxes = 0, nfirst = 0, nsphere = 0; // warp-uniform
+    const int64_t  np     = *total;
+    const int64_t  stride = (int64_t)gridDim.x * blockDim.x;
+    int64_t        base   = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~int64_t(31);
+    while(true)
+    {
+        const bool more = base < np;
+        if(more)
+        {
+            const int64_t p    = base + lane;
+            uint32_t      a    = 0, b = 0;
+            bool          take = false;
+            if(p < np)
+            {
+                a    = pair_a[p];
+                b    = pair_b[p];
+                take = a < b && !(b & kObstacleBit);
+            }
+            warp_push(boxes, nboxes, take, (uint32_t)p, a, b);
+            base += stride;
+        }
+        if(nboxes >= 32 || (!more && nboxes))
+        {
+            uint32_t   p = 0, a = 0, b = 0;
+            const bool mine = warp_pop(boxes, nboxes, p, a, b);
+            bool       keep = false, both = false;
+            if(mine)
+            {
+                const Pose32 A = load_pose(pose, a), B = load_pose(pose, b);
+                const bool   sa = SPHERES && A.r < 0.0f, sb = SPHERES && B.r < 0.0f;
+                both            = sa && sb;
+                if(!sa && !sb)
+                    keep = !obb_apart(A.bb, B.bb, A.R, B.R, centre_difference(A, B),
+                                      1e-4f * (A.r + B.r));
+            }
+            warp_push(first, nfirst, keep, p, a, b);
+            if constexpr(SPHERES)
+                warp_push(sphere, nsphere, both, p, a, b);
+        }
+        const bool flush = !more && !nboxes;
+        if(nfirst >= 32 || (flush && nfirst))
+        {
+            uint32_t   p = 0, a = 0, b = 0;
+            const bool mine = warp_pop(first, nfirst, p, a, b);
+            bool       keep = false;
+            if(mine)
+            {
+                const Pose32      A  = load_pose(pose, a), B = load_pose(pose, b);
+                const Body<float> bA = load_body<float>(tb.shape32, A.rb, tb.verts32);
+                const Body<float> bB = load_body<float>(tb.shape32, B.rb, tb.verts32);
+                keep = !gjk_first_iteration_separates<JH_RULE>(bA, bB, A.R, B.R,
+                                                               centre_difference(A, B), A.r + B.r);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, keep);
+            uint32_t       k = 0;
+            if(lane == 0 && m)
+                k = atomicAdd(gjk_count, (uint32_t)__popc(m));
+            k = __shfl_sync(0xffffffffu, k, 0);
+            if(keep)
+                gjk_queue[k + __popc(m & ((1u << lane) - 1u))] = p;
+        }
+        if constexpr(SPHERES)
+            if(nsphere >= 32 || (flush && nsphere))
+            {
+                uint32_t p = 0, a = 0, b = 0;
+                if(warp_pop(sphere, nsphere, p, a, b))
+                {
+                    const uint32_t pm = mirror_record(off, pair_b, a, b);
+                    for(int k = 0; k < (pm == kNoRecord ? 1 : 2); ++k)
+                        narrow_pair<S, GB_GJK_JH, true>(k ? pm : p, k ? b : a, k ? a : b, st, tb,
+                                                        po, law_kind, has_kr, dt, counters);
+                }
+                __syncwarp();
+            }
+        if(flush && !nfirst && !nsphere)
+            break;
+    }
 }
 
-// The mixed mode's FP32 stage over the cull pass's queue: a pair that
-// gjk_fp32_separates decides is finished here (no contact, the outputs the
-// FP64 GJK would store), the others go to the FP64 GJK's queue.
+// The FP32 GJK stage over the cull's queue: a pair that gjk_fp32_separates
+// decides has no contact (its certificate, a lower bound on the distance,
+// holds for every GJK variant and for both records); of every other pair both
+// records go to the FP64 GJK's queue.
+template <typename St>
 __global__ void __launch_bounds__(128)
     k_narrow_gjk32(const uint32_t* __restrict__ gjk_count, const int* __restrict__ flags,
                    const uint32_t* __restrict__ gjk_queue, const uint32_t* __restrict__ pair_a,
-                   const uint32_t* __restrict__ pair_b, State<float> st, Tables<float> tb,
-                   PairOut<float> po, int law_kind, int has_kr, uint32_t* __restrict__ queue64,
+                   const uint32_t* __restrict__ pair_b, const uint32_t* __restrict__ off,
+                   const PoseRec<St>* __restrict__ pose, const RBShape<float>* __restrict__ shape,
+                   const Vert<float>* __restrict__ verts, uint32_t* __restrict__ queue64,
                    uint32_t* __restrict__ count64)
 {
     grid_dep_sync();
@@ -1650,23 +1982,17 @@ __global__ void __launch_bounds__(128)
     for_each_pair(*gjk_count, [&](int64_t q) {
         const uint32_t    p = gjk_queue[q];
         const uint32_t    a = pair_a[p], b = pair_b[p];
-        const uint32_t    ra = st.rb_id[a], rb = st.rb_id[b];
-        const Body<float> A  = load_body<float>(tb.shape, ra, tb.verts);
-        const Body<float> B  = load_body<float>(tb.shape, rb, tb.verts);
-        const M3<float>   RA = load_rot<float>(st, a), RB = load_rot<float>(st, b);
-        const V3<float>   d  = mk<float>(float(st.pos[0][b] - st.pos[0][a]),
-                                         float(st.pos[1][b] - st.pos[1][a]),
-                                         float(st.pos[2][b] - st.pos[2][a]));
-        if(gjk_fp32_separates(A, B, RA, RB, d))
+        const Pose32      A = load_pose(pose, a), B = load_pose(pose, b);
+        const Body<float> bA = load_body<float>(shape, A.rb, verts);
+        const Body<float> bB = load_body<float>(shape, B.rb, verts);
+        if(!gjk_fp32_separates(bA, bB, A.R, B.R, centre_difference(A, B), A.r + B.r))
         {
-            const double xa[3] = {st.pos[0][a], st.pos[1][a], st.pos[2][a]};
-            Force<float> F;
-            F.f = F.t = F.m = zero3<float>();
-            store_pair<float>(po, p, F, zero3<float>(), uint8_t(0), law_kind, has_kr,
-                              no_contact<float>(), xa);
+            const uint32_t pm = mirror_record(off, pair_b, a, b);
+            const uint32_t k  = atomicAdd(count64, pm == kNoRecord ? 1u : 2u);
+            queue64[k]        = p;
+            if(pm != kNoRecord)
+                queue64[k + 1] = pm;
         }
-        else
-            queue64[atomicAdd(count64, 1u)] = p;
     });
 }
 
@@ -1699,8 +2025,9 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS)
     const int64_t nslots = ((int64_t)gridDim.x * blockDim.x) >> 1;
     const int64_t slot   = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 1;
     auto          one    = [&](int64_t q) {
-        narrow_pair<S, VAR | kGjkPaired>(gjk_queue[q], pair_a, pair_b, st, tb, po, law_kind,
-                                         has_kr, dt, counters);
+        const uint32_t p = gjk_queue[q];
+        narrow_pair<S, VAR | kGjkPaired>(p, pair_a[p], pair_b[p], st, tb, po, law_kind, has_kr,
+                                         dt, counters);
     };
     if(nq < nslots)
     {
@@ -1860,8 +2187,8 @@ __global__ void __launch_bounds__(kBlock, sizeof(store_t<S>) == 4 ? 4 : 2)
             T = zero3<S>();
         }
         // the particle's pairs, then its obstacle pairs, in list order; most
-        // particles have no contact (the narrow phase counts them) and skip
-        // their list
+        // particles have no contact (the narrow phase marks those that have)
+        // and skip their list
         const uint32_t ncon = po.pcount[i];
         if(ncon)
             po.pcount[i] = 0u;
