@@ -57,24 +57,26 @@ GB_D Contact<S> closest_spheres(S rA, S rB, const V3<S>& oA, const V3<S>& oB)
 template <int VAR = GB_GJK_JH, typename S>
 GB_D Contact<S> closest_points(const Body<S>& A, const Body<S>& B, const M3<S>& RA,
                                const M3<S>& RB, const V3<S>& oA, const V3<S>& oB,
-                               const V3<S>& d, int* gjk_iters)
+                               const V3<S>& d, int* gjk_iters, bool active = true)
 {
-    if(A.type == GB_SPHERE && B.type == GB_SPHERE)
-        return closest_spheres(A.p[0], B.p[0], oA, oB);
+    // in a lane pair (kGjkPaired) every lane goes on to the GJK
+    constexpr bool PAIRED = (VAR & kGjkPaired) != 0;
+    if constexpr(!PAIRED)
+        if(A.type == GB_SPHERE && B.type == GB_SPHERE)
+            return closest_spheres(A.p[0], B.p[0], oA, oB);
     const S overlap = norm(d) - (A.rcirc + B.rcirc);
-    if(!(overlap < S(0.0)))
-        return no_contact<S>();
-    if(!obb_overlap(A.bb, B.bb, RA, RB, d))
+    active = active && overlap < S(0.0) && obb_overlap(A.bb, B.bb, RA, RB, d);
+    if(!PAIRED && !active)
         return no_contact<S>();
     // b2a = Transform3(a2w, b2w) (Transform3.cpp:34-39, :313-318)
     Tr<S> b2a;
     const M3<S> RAt = transpose(RA);
     b2a.R           = mul(RAt, RB);
     b2a.o           = mul(RAt, d);
-    GjkResult<S> g  = gjk<VAR>(A, B, b2a);
+    GjkResult<S> g  = gjk<VAR>(A, B, b2a, active);
     *gjk_iters += g.iters;
     S distance = g.dist - (A.crust + B.crust);
-    if(distance > S(0.0))
+    if(!active || distance > S(0.0))
         return no_contact<S>();
     const V3<S> ptA = mul(RA, g.pa) + oA;
     const V3<S> ptB = mul(RB, g.pb) + oB;

@@ -239,6 +239,21 @@ GB_D V3<S> support_first(const Body<S>& b, const V3<S>& v)
 // dependent chain of an iteration: ~2,000 cycles for an FP64 superquadric.)
 constexpr int kGjkPaired = 8;
 
+// A GJK's loop condition.  PAIRED: the whole warp (all 32 lanes call the
+// GJK, lanes without a pair with run = false) goes round until its last pair
+// is done, which brings the lanes back together before each iteration's
+// supports.  Without that they drift apart in the simplex branches and the
+// warp runs the supports several times over, a few lanes each (measured: 7
+// of 32 lanes active in the signed-volume GJK, 2-5 in the FP32 one).
+template <bool PAIRED>
+GB_D bool gjk_goes_on(bool run)
+{
+    if constexpr(PAIRED)
+        return __any_sync(0xffffffffu, run);
+    else
+        return run;
+}
+
 GB_D float lane_shfl(unsigned mask, float v, unsigned src)
 {
     return __shfl_sync(mask, v, src);
@@ -528,10 +543,11 @@ struct GjkResult
 };
 
 // computeClosestPoints_GJK_JH (GJK_JH.cpp:310-391), in A's frame with b2a.
-// `max_iter` caps the iterations (the reference's cap is 1000).
+// `max_iter` caps the iterations (the reference's cap is 1000).  `active`:
+// see gjk_goes_on (false: the result is not used).
 template <typename S, bool PAIRED = false>
 GB_D GjkResult<S> gjk_jh(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
-                         int max_iter = 1000)
+                         bool active = true, int max_iter = 1000)
 {
     unsigned bits = 0, last = 0, last_bit = 0, all_bits = 0;
     V3<S>    p[4], q[4];
@@ -559,30 +575,39 @@ GB_D GjkResult<S> gjk_jh(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
     V3<S> v    = s0A - apply(b2a, s0B);
     V3<S> w    = v;
     S     dist = norm(v);
-    while(bits < 15 && dist > k_higheps<S>() && num_iterations < max_iter)
+    bool  run  = active && dist > k_higheps<S>();
+    while(gjk_goes_on<PAIRED>(run))
     {
-        last     = 0;
-        last_bit = 1;
-        while(bits & last_bit)
+        if(run)
         {
-            ++last;
-            last_bit <<= 1;
+            last     = 0;
+            last_bit = 1;
+            while(bits & last_bit)
+            {
+                ++last;
+                last_bit <<= 1;
+            }
+            support2<PAIRED>(A, -v, B, mul_t(b2a.R, v), p[last], q[last]);
+            w         = p[last] - apply(b2a, q[last]);
+            const S g = dot(v, w) / dist;
+            if(mu < g)
+                mu = g;
+            if(dist - mu <= dist * rel_error || mu < abs_error || jh.degenerate(all_bits, w))
+                run = false;
+            else
+            {
+                jh.y[last] = w;
+                all_bits   = bits | last_bit;
+                ++num_iterations;
+                if(!jh.closest(bits, last, last_bit, all_bits, v))
+                    run = false;
+                else
+                {
+                    dist = norm(v);
+                    run  = bits < 15 && dist > k_higheps<S>() && num_iterations < max_iter;
+                }
+            }
         }
-        support2<PAIRED>(A, -v, B, mul_t(b2a.R, v), p[last], q[last]);
-        w       = p[last] - apply(b2a, q[last]);
-        const S g = dot(v, w) / dist;
-        if(mu < g)
-            mu = g;
-        if(dist - mu <= dist * rel_error || mu < abs_error)
-            break;
-        if(jh.degenerate(all_bits, w))
-            break;
-        jh.y[last] = w;
-        all_bits   = bits | last_bit;
-        ++num_iterations;
-        if(!jh.closest(bits, last, last_bit, all_bits, v))
-            break;
-        dist = norm(v);
     }
     // computePoints (GJK_JH.cpp:108-130)
     GjkResult<S> r;
@@ -840,7 +865,8 @@ GB_D bool sv_degenerate(unsigned bits, const V3<S> y[4], const V3<S>& w)
 //   d_k = delta_k d_{k-1}/|d_{k-1}| + (1 - delta_k) y_k/|y_k|.
 // Without NESTEROV it is computeClosestPoints_GJK_AY (GJK_AY.cpp:392-469).
 template <typename S, bool NESTEROV, bool PAIRED = false>
-GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a)
+GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
+                         bool active = true)
 {
     unsigned bits = 0, last = 0;
     V3<S>    p[4], q[4], y[4];
@@ -857,8 +883,11 @@ GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a)
     V3<S>   v = s0A - apply(b2a, s0B);
     V3<S>   w = v, d = v, s_prev = v;
     S       dist = norm(v);
-    while(bits < 15 && dist > k_higheps<S>() && num_iterations < 1000)
+    bool    run  = active && dist > k_higheps<S>();
+    while(gjk_goes_on<PAIRED>(run))
     {
+        if(!run)
+            continue;
         for(unsigned k = 0; k < 4; ++k)
             if(!(bits & (1u << k)))
             {
@@ -895,9 +924,10 @@ GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a)
         const S mu = dist - dot(v, w) / dist;
         if(mu < dist * rel_error || mu < abs_error || sv_degenerate(bits, y, w))
         {
-            if(!momentum)
-                break;
-            momentum = false; // not a certified gap: redo this iteration along x_k
+            // with momentum not a certified gap: this iteration is redone
+            // along x_k
+            run      = momentum;
+            momentum = false;
             continue;
         }
         y[last] = w;
@@ -906,6 +936,7 @@ GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a)
         v    = sv_subalgorithm(y, bits, lambdas);
         dist = norm(v);
         s_prev = w;
+        run    = bits < 15 && dist > k_higheps<S>() && num_iterations < 1000;
     }
     // computePoints (GJK_AY.cpp:319-337)
     GjkResult<S> r;
@@ -926,16 +957,16 @@ GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a)
 // the GJK of a variant (GB_GJK_JH | GB_GJK_SV | GB_GJK_NESTEROV), optionally
 // with kGjkPaired
 template <int VAR, typename S>
-GB_D GjkResult<S> gjk(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a)
+GB_D GjkResult<S> gjk(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a, bool active)
 {
     constexpr bool PAIRED = (VAR & kGjkPaired) != 0;
     constexpr int  KIND   = VAR & ~kGjkPaired;
     if constexpr(KIND == GB_GJK_SV)
-        return gjk_sv<S, false, PAIRED>(A, B, b2a);
+        return gjk_sv<S, false, PAIRED>(A, B, b2a, active);
     else if constexpr(KIND == GB_GJK_NESTEROV)
-        return gjk_sv<S, true, PAIRED>(A, B, b2a);
+        return gjk_sv<S, true, PAIRED>(A, B, b2a, active);
     else
-        return gjk_jh<S, PAIRED>(A, B, b2a);
+        return gjk_jh<S, PAIRED>(A, B, b2a, active);
 }
 
 } // namespace gb

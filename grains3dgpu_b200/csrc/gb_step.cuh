@@ -93,14 +93,17 @@ struct alignas(32) SphereRec // 64 bytes mixed, 96 FP64
     uint32_t material;
 };
 
+// a record in 32-byte loads and stores, a sector each (sm_100's widest)
 template <typename T>
 GB_D T load_rec(const T* p)
 {
-    constexpr int kWords = sizeof(T) / sizeof(int4);
-    int4          w[kWords];
+    constexpr int kWords = sizeof(T) / 32;
+    uint64_t      w[4 * kWords];
 #pragma unroll
     for(int k = 0; k < kWords; ++k)
-        w[k] = __ldg(reinterpret_cast<const int4*>(p) + k);
+        asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+            : "=l"(w[4 * k]), "=l"(w[4 * k + 1]), "=l"(w[4 * k + 2]), "=l"(w[4 * k + 3])
+            : "l"(reinterpret_cast<const char*>(p) + 32 * k));
     T t;
     memcpy(&t, w, sizeof(t));
     return t;
@@ -109,12 +112,15 @@ GB_D T load_rec(const T* p)
 template <typename T>
 GB_D void store_rec(T* p, const T& t)
 {
-    constexpr int kWords = sizeof(T) / sizeof(int4);
-    int4          w[kWords];
+    constexpr int kWords = sizeof(T) / 32;
+    uint64_t      w[4 * kWords];
     memcpy(w, &t, sizeof(t));
 #pragma unroll
     for(int k = 0; k < kWords; ++k)
-        reinterpret_cast<int4*>(p)[k] = w[k];
+        asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(
+                         reinterpret_cast<char*>(p) + 32 * k),
+                     "l"(w[4 * k]), "l"(w[4 * k + 1]), "l"(w[4 * k + 2]), "l"(w[4 * k + 3])
+                     : "memory");
 }
 
 // the records' arrays, by particle id; null where the step does not read them
@@ -177,22 +183,18 @@ GB_D Contact<float> closest_spheres_mixed(double rA, double rB, const double xa[
     return to_f(c);
 }
 
-// closestPointsRigidBodies for the mixed mode; points relative to A's centre.
-// VAR: the GJK variant of the FP64 solve.
+// closestPointsRigidBodies for the mixed mode on a lane pair (kGjkPaired; not
+// two spheres); points relative to A's centre.  VAR: the GJK variant of the
+// FP64 solve; active: the lane has a pair.
 template <int VAR>
 GB_D Contact<float> closest_mixed(const Tables<float>& tb, const State<float>& st, uint32_t a,
                                   uint32_t b, uint32_t ra, uint32_t rb, const Body<float>& A,
                                   const Body<float>& B, const M3<float>& RA, const M3<float>& RB,
-                                  const double xa[3], const double xb[3], int* iters)
+                                  const double xa[3], const double xb[3], int* iters, bool active)
 {
     const V3<double> d64 = mk<double>(xb[0] - xa[0], xb[1] - xa[1], xb[2] - xa[2]);
-    if(A.type == GB_SPHERE && B.type == GB_SPHERE)
-        return closest_spheres_mixed(tb.shape64[ra].p[0], tb.shape64[rb].p[0], xa, xb);
-    const V3<float> d = cvt3<float>(d64);
-    if(!(norm(d) - (A.rcirc + B.rcirc) < 0.0f))
-        return no_contact<float>();
-    if(!obb_overlap(A.bb, B.bb, RA, RB, d))
-        return no_contact<float>();
+    const V3<float>  d   = cvt3<float>(d64);
+    active = active && norm(d) - (A.rcirc + B.rcirc) < 0.0f && obb_overlap(A.bb, B.bb, RA, RB, d);
     // every pair that passes the bounding tests is solved on the FP64 path of
     // the FP64 mode
     const Body<double> A64 = load_body<double>(tb.shape64, ra, tb.verts64);
@@ -202,10 +204,10 @@ GB_D Contact<float> closest_mixed(const Tables<float>& tb, const State<float>& s
     const M3<double>   RAt64 = transpose(RA64);
     b2a64.R                  = mul(RAt64, RB64);
     b2a64.o                  = mul(RAt64, d64);
-    const GjkResult<double> g = gjk<VAR>(A64, B64, b2a64);
+    const GjkResult<double> g = gjk<VAR>(A64, B64, b2a64, active);
     *iters += g.iters;
     const double distance = g.dist - (A64.crust + B64.crust);
-    if(distance > 0.0)
+    if(!active || distance > 0.0)
         return no_contact<float>();
     const V3<double> ptA = mul(RA64, g.pa);
     const V3<double> ptB = mul(RB64, g.pb) + d64;
@@ -1527,11 +1529,12 @@ constexpr int kGjk32MaxIter = 24;
 // lower bound v.w/|v| on the distance of the cores, whatever the simplex
 // arithmetic did, with the FP32 error bound of gjk_first_iteration_separates.
 // True: the largest bound exceeds the crusts by that margin, so the FP64 GJK
-// finds no contact either.  False (the FP64 GJK decides): the iterates
-// converged below the crusts (a contact or a near miss), reached the
-// origin, left the finite range, or ran out of iterations.
+// finds no contact either.  False (the FP64 GJK decides): an iterate came
+// within the crusts and the margin (a contact or a near miss), reached the
+// origin, left the finite range, or they ran out of iterations.
+// Called by whole warps (gjk_goes_on), lanes without a pair with run = false.
 GB_D bool gjk_fp32_separates(const Body<float>& A, const Body<float>& B, const M3<float>& RA,
-                             const M3<float>& RB, const V3<float>& d, float s)
+                             const M3<float>& RB, const V3<float>& d, float s, bool run)
 {
     Tr<float>       b2a;
     const M3<float> RAt = transpose(RA);
@@ -1544,23 +1547,27 @@ GB_D bool gjk_fp32_separates(const Body<float>& A, const Body<float>& B, const M
     int         n  = 1;
     V3<float>   v  = y0;
     float       mu = -INFINITY;
-    for(int k = 0; k < kGjk32MaxIter; ++k)
+    bool        separates = false;
+    for(int k = 0; k < kGjk32MaxIter && gjk_goes_on<true>(run); ++k)
     {
         const float vv = dot(v, v);
-        if(!(vv > 1e-30f))
-            return false;
+        run            = run && vv > 1e-30f;
+        if(!run)
+            continue;
         const V3<float> w = support_first(A, -v)
                             - apply(b2a, support_first(B, mul_t(b2a.R, v)));
         const float vw = dot(v, w);
         const float nv = sqrtf(vv);
         const float g  = vw / nv;
-        if(!(g == g))
-            return false;
-        mu = fmaxf(mu, g);
-        if(mu > ct + margin)
-            return true;
-        if(nv - mu <= margin || vv - vw <= 1e-6f * vv)
-            return false;
+        mu             = fmaxf(mu, g); // (a NaN g ends it below)
+        separates      = mu > ct + margin;
+        // nv bounds the distance from above: within the crusts and the margin
+        // no lower bound can pass them
+        if(separates || !(g == g) || nv <= ct + margin || vv - vw <= 1e-6f * vv)
+        {
+            run = false;
+            continue;
+        }
         if(n == 1)
             v = closest_on_segment(y0, w, y0, y1, n);
         else if(n == 2)
@@ -1600,7 +1607,7 @@ GB_D bool gjk_fp32_separates(const Body<float>& A, const Body<float>& B, const M
             }
         }
     }
-    return false;
+    return separates;
 }
 
 // The contact law for contact `ci` of the particle pair record p = (a, b) and
@@ -1645,7 +1652,7 @@ GB_D void pair_contact(int64_t p, uint32_t a, uint32_t b, const Law<S>& L, S m1,
 template <typename S, int VAR, bool SPHERES = false>
 GB_D void narrow_pair(int64_t p, uint32_t a, uint32_t b, const State<store_t<S>>& st,
                       const Tables<S>& tb, const PairOut<store_t<S>>& po, int law_kind, int has_kr,
-                      S dt, unsigned long long* __restrict__ counters)
+                      S dt, unsigned long long* __restrict__ counters, bool active = true)
 {
     const uint32_t ra = st.rb_id[a], rb = st.rb_id[b];
     const double   xa[3] = {st.pos[0][a], st.pos[1][a], st.pos[2][a]};
@@ -1679,12 +1686,12 @@ GB_D void narrow_pair(int64_t p, uint32_t a, uint32_t b, const State<store_t<S>>
         const Body<S> B  = load_body<S>(tb.shape, rb, tb.verts);
         const M3<S>   RA = load_rot<S>(st, a), RB = load_rot<S>(st, b);
         if constexpr(is_mixed<S>())
-            ci = closest_mixed<VAR>(tb, st, a, b, ra, rb, A, B, RA, RB, xa, xb, &iters);
+            ci = closest_mixed<VAR>(tb, st, a, b, ra, rb, A, B, RA, RB, xa, xb, &iters, active);
         else
-            ci = closest_points<VAR>(A, B, RA, RB, oA, oB, d, &iters);
+            ci = closest_points<VAR>(A, B, RA, RB, oA, oB, d, &iters, active);
     }
     // a lane pair (kGjkPaired) holds the same results: its even lane stores them
-    if((VAR & kGjkPaired) && (threadIdx.x & 1u))
+    if((VAR & kGjkPaired) && (!active || (threadIdx.x & 1u)))
         return;
     if(ci.overlap < S(0.0))
         pair_contact<S>(p, a, b, load_law<S>(tb.law, tb.shape[ra].material, tb.shape[rb].material),
@@ -1719,6 +1726,28 @@ GB_D void for_each_pair(int64_t npairs, F&& f)
     else
         for(int64_t p = tid; p < npairs; p += nthreads)
             f(p);
+}
+
+// The same for passes that whole warps run together: f(p, valid) on every lane
+// of the warp, `step` (1 or 2) lanes per pair, lanes without a pair with
+// valid = false and a p that may be read (npairs > 0).
+template <int STEP, typename F>
+GB_D void for_each_pair_converged(int64_t npairs, F&& f)
+{
+    constexpr int kPairs = 32 / STEP; // pairs a warp holds at a time
+    const int64_t nwarps = (int64_t)gridDim.x * blockDim.x / 32;
+    const int64_t warp   = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int     slot   = (int)(threadIdx.x & 31u) / STEP;
+    if(npairs < nwarps * kPairs)
+    {
+        const int64_t k = (npairs + nwarps - 1) / nwarps; // <= kPairs
+        const int64_t p = warp * k + slot;
+        if(warp * k < npairs)
+            f(slot < k && p < npairs ? p : npairs - 1, slot < k && p < npairs);
+    }
+    else
+        for(int64_t base = warp * kPairs; base < npairs; base += nwarps * kPairs)
+            f(base + slot < npairs ? base + slot : npairs - 1, base + slot < npairs);
 }
 
 // The narrow phase of a run whose bodies are all spheres: every record's
@@ -1979,13 +2008,15 @@ __global__ void __launch_bounds__(128)
     grid_dep_sync();
     if(step_aborted(flags))
         return;
-    for_each_pair(*gjk_count, [&](int64_t q) {
+    for_each_pair_converged<1>(*gjk_count, [&](int64_t q, bool valid) {
         const uint32_t    p = gjk_queue[q];
         const uint32_t    a = pair_a[p], b = pair_b[p];
         const Pose32      A = load_pose(pose, a), B = load_pose(pose, b);
         const Body<float> bA = load_body<float>(shape, A.rb, verts);
         const Body<float> bB = load_body<float>(shape, B.rb, verts);
-        if(!gjk_fp32_separates(bA, bB, A.R, B.R, centre_difference(A, B), A.r + B.r))
+        const bool        open = !gjk_fp32_separates(bA, bB, A.R, B.R, centre_difference(A, B),
+                                                     A.r + B.r, valid);
+        if(valid && open)
         {
             const uint32_t pm = mirror_record(off, pair_b, a, b);
             const uint32_t k  = atomicAdd(count64, pm == kNoRecord ? 1u : 2u);
@@ -1997,9 +2028,10 @@ __global__ void __launch_bounds__(128)
 }
 
 // One queued pair per lane pair (kGjkPaired: the two supports of a GJK
-// iteration in parallel); a short queue is spread over all warps as in
-// for_each_pair, a long one walked with a stride.  Both lanes of a pair take
-// the same path throughout, so their shuffles always meet.  MIN_BLOCKS > 1
+// iteration in parallel), the warp's pairs going through the iterations
+// together; a short queue is spread over all warps, a long one walked with a
+// stride.  Both lanes of a pair take the same path throughout, so their
+// shuffles always meet.  MIN_BLOCKS > 1
 // caps its registers for more resident warps (Johnson's tables and some
 // values spill to local memory): faster where the supports are closed forms
 // (superquadrics) and the queue outnumbers the default's lane pairs, slower
@@ -2022,25 +2054,11 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS)
     const int64_t nq     = *gjk_count;
     if(nq < (int64_t)min_queue || nq >= (int64_t)max_queue)
         return;
-    const int64_t nslots = ((int64_t)gridDim.x * blockDim.x) >> 1;
-    const int64_t slot   = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 1;
-    auto          one    = [&](int64_t q) {
+    for_each_pair_converged<2>(nq, [&](int64_t q, bool valid) {
         const uint32_t p = gjk_queue[q];
         narrow_pair<S, VAR | kGjkPaired>(p, pair_a[p], pair_b[p], st, tb, po, law_kind, has_kr,
-                                         dt, counters);
-    };
-    if(nq < nslots)
-    {
-        const int64_t nwarps = nslots >> 4;                 // 16 lane pairs per warp
-        const int64_t k      = (nq + nwarps - 1) / nwarps;  // <= 16
-        const int64_t pl     = (threadIdx.x & 31) >> 1;     // the lane pair within the warp
-        const int64_t q      = (slot >> 4) * k + pl;
-        if(pl < k && q < nq)
-            one(q);
-    }
-    else
-        for(int64_t q = slot; q < nq; q += nslots)
-            one(q);
+                                         dt, counters, valid);
+    });
 }
 
 // ---- per-particle kernel -------------------------------------------------------
