@@ -643,36 +643,30 @@ GB_D unsigned sv_same_sign(S a, S b)
     return (unsigned)(!((a > S(0.0)) ^ (b > S(0.0)))); // compareSigns (GJK_AY.cpp:8-12)
 }
 
-// sum of lambda_i y_i over the used points (computeVector, GJK_AY.cpp:304-316)
+// The sub-algorithm below keeps the simplex in registers: slots, faces and
+// edges are picked by selects on their index, since an indexed local array
+// costs a round trip to memory per access.
+
+// vertex i (0..3) of y
 template <typename S>
-GB_D V3<S> sv_point(const V3<S> y[4], unsigned used, const S lambdas[4])
+GB_D V3<S> sv_pick(const V3<S> y[4], unsigned i)
 {
-    V3<S> o = zero3<S>();
-#pragma unroll
-    for(unsigned i = 0; i < 4; ++i)
-        if(used & (1u << i))
-            o = o + lambdas[i] * y[i];
-    return o;
+    const V3<S> lo = i & 1u ? y[1] : y[0], hi = i & 1u ? y[3] : y[2];
+    return i & 2u ? hi : lo;
 }
 
-// s1d (GJK_AY.cpp:15-84)
-template <typename S>
-GB_D void sv_s1d(const V3<S> y[4], unsigned& bits, S lambdas[4])
+// the k-th (0..2) vertex other than j, in ascending order
+GB_D unsigned sv_other(unsigned j, unsigned k)
 {
-    bool     s1_set = false;
-    unsigned i1 = 0, i2 = 0;
-    for(unsigned i = 0; i < 4; ++i)
-        if(bits & (1u << i))
-        {
-            if(s1_set)
-            {
-                i2 = i;
-                break;
-            }
-            i1     = i;
-            s1_set = true;
-        }
-    const V3<S> t      = y[i2] - y[i1];
+    return k + (k >= j ? 1u : 0u);
+}
+
+// s1d (GJK_AY.cpp:15-84) on the segment (A, B), in slot order: the used
+// vertices (bit 0: A, bit 1: B) and their weights
+template <typename S>
+GB_D unsigned sv_edge(const V3<S>& A, const V3<S>& B, S& la, S& lb)
+{
+    const V3<S> t      = B - A;
     unsigned    I      = 0;
     S           neg_tI = -t.x;
     if(s_fabs(t.y) > s_fabs(neg_tI))
@@ -685,56 +679,45 @@ GB_D void sv_s1d(const V3<S> y[4], unsigned& bits, S lambdas[4])
         I      = 2;
         neg_tI = -t.z;
     }
-    const S pI  = dot(y[i2], t) / norm2(t) * neg_tI + comp(y[i2], I);
-    const S C0  = -comp(y[i2], I) + pI, C1 = comp(y[i1], I) - pI;
+    const S pI  = dot(B, t) / norm2(t) * neg_tI + comp(B, I);
+    const S C0  = -comp(B, I) + pI, C1 = comp(A, I) - pI;
     const unsigned sc0 = sv_same_sign(neg_tI, C0), sc1 = sv_same_sign(neg_tI, C1);
     if(sc0 + sc1 == 2)
     {
-        lambdas[i1] = C0 / neg_tI;
-        lambdas[i2] = C1 / neg_tI;
+        la = C0 / neg_tI;
+        lb = C1 / neg_tI;
+        return 3u;
     }
-    else if(sc0)
+    if(sc0)
     {
-        bits &= ~(1u << i2);
-        lambdas[i1] = S(1.0);
+        la = S(1.0);
+        lb = S(0.0);
+        return 1u;
     }
-    else
-    {
-        bits &= ~(1u << i1);
-        lambdas[i2] = S(1.0);
-    }
+    la = S(0.0);
+    lb = S(1.0);
+    return 2u;
 }
 
-// s2d (GJK_AY.cpp:87-212)
+// s2d (GJK_AY.cpp:87-212) on the triangle Y, in slot order: the used vertices
+// (bit i: Y[i]) and their weights
 template <typename S>
-GB_D void sv_s2d(const V3<S> y[4], unsigned& bits, S lambdas[4])
+GB_D unsigned sv_face(const V3<S> Y[3], S l[3])
 {
-    unsigned counter = 0, i0 = 0, i1 = 0, i2 = 0;
-    for(unsigned i = 0; i < 4; ++i)
-        if(bits & (1u << i))
-        {
-            if(counter == 0)
-                i0 = i;
-            else if(counter == 1)
-                i1 = i;
-            else
-                i2 = i;
-            counter += 1;
-        }
-    const V3<S> n  = cross(y[i1] - y[i0], y[i2] - y[i0]);
-    const V3<S> p0 = (dot(y[i0], n) / norm2(n)) * n;
-    const V3<S>& Y0 = y[i0];
-    const V3<S>& Y1 = y[i1];
-    const V3<S>& Y2 = y[i2];
-    unsigned     ix = 1, iy = 2;
-    S mu_max = (Y1.y * Y2.z + Y0.y * Y1.z + Y2.y * Y0.z - Y1.y * Y0.z - Y2.y * Y1.z - Y0.y * Y2.z);
-    S mu     = (Y1.z * Y0.x + Y2.z * Y1.x + Y0.z * Y2.x - Y1.z * Y2.x - Y0.z * Y1.x - Y2.z * Y0.x);
+    const V3<S> n  = cross(Y[1] - Y[0], Y[2] - Y[0]);
+    const V3<S> p0 = (dot(Y[0], n) / norm2(n)) * n;
+    unsigned    ix = 1, iy = 2;
+    S mu_max = (Y[1].y * Y[2].z + Y[0].y * Y[1].z + Y[2].y * Y[0].z - Y[1].y * Y[0].z
+                - Y[2].y * Y[1].z - Y[0].y * Y[2].z);
+    S mu     = (Y[1].z * Y[0].x + Y[2].z * Y[1].x + Y[0].z * Y[2].x - Y[1].z * Y[2].x
+            - Y[0].z * Y[1].x - Y[2].z * Y[0].x);
     if(s_fabs(mu) > s_fabs(mu_max))
     {
         mu_max = mu;
         ix     = 0;
     }
-    mu = (Y1.x * Y2.y + Y0.x * Y1.y + Y2.x * Y0.y - Y1.x * Y0.y - Y2.x * Y1.y - Y0.x * Y2.y);
+    mu = (Y[1].x * Y[2].y + Y[0].x * Y[1].y + Y[2].x * Y[0].y - Y[1].x * Y[0].y - Y[2].x * Y[1].y
+          - Y[0].x * Y[2].y);
     if(s_fabs(mu) > s_fabs(mu_max))
     {
         mu_max = mu;
@@ -742,46 +725,54 @@ GB_D void sv_s2d(const V3<S> y[4], unsigned& bits, S lambdas[4])
         iy     = 1;
     }
     const S px = comp(p0, ix), py = comp(p0, iy);
-    const S y0x = comp(Y0, ix), y0y = comp(Y0, iy), y1x = comp(Y1, ix), y1y = comp(Y1, iy);
-    const S y2x = comp(Y2, ix), y2y = comp(Y2, iy);
+    const S y0x = comp(Y[0], ix), y0y = comp(Y[0], iy), y1x = comp(Y[1], ix), y1y = comp(Y[1], iy);
+    const S y2x = comp(Y[2], ix), y2y = comp(Y[2], iy);
     S       C[3];
     C[0] = (px * y1y + py * y2x + y1x * y2y - px * y2y - py * y1x - y2x * y1y);
     C[1] = (px * y2y + py * y0x + y2x * y0y - px * y0y - py * y2x - y0x * y2y);
     C[2] = (px * y0y + py * y1x + y0x * y1y - px * y1y - py * y0x - y1x * y0y);
-    const unsigned sc[3] = {sv_same_sign(mu_max, C[0]), sv_same_sign(mu_max, C[1]),
-                            sv_same_sign(mu_max, C[2])};
-    if(sc[0] + sc[1] + sc[2] == 3)
-    {
-        lambdas[i0] = C[0] / mu_max;
-        lambdas[i1] = C[1] / mu_max;
-        lambdas[i2] = C[2] / mu_max;
-        return;
-    }
-    S              d        = S(100000.0);
-    unsigned       new_bits = 0;
-    const unsigned idx[3]   = {i0, i1, i2};
+    unsigned open = 0; // the edges (by the vertex they leave out) to look at
+#pragma unroll
     for(unsigned j = 0; j < 3; ++j)
-        if(!sc[j])
+        open |= (1u - sv_same_sign(mu_max, C[j])) << j;
+    if(!open)
+    {
+#pragma unroll
+        for(int j = 0; j < 3; ++j)
+            l[j] = C[j] / mu_max;
+        return 7u;
+    }
+    S        d    = S(100000.0);
+    unsigned used = 0;
+    l[0] = l[1] = l[2] = S(0.0);
+    for(; open; open &= open - 1u)
+    {
+        const unsigned j = (unsigned)__ffs(open) - 1u;
+        const V3<S>    A = j == 0 ? Y[1] : Y[0], B = j == 2 ? Y[1] : Y[2];
+        S              la, lb;
+        const unsigned e = sv_edge(A, B, la, lb);
+        V3<S>          np = zero3<S>();
+        if(e & 1u)
+            np = np + la * A;
+        if(e & 2u)
+            np = np + lb * B;
+        const S d_star = dot(np, np);
+        if(d_star < d)
         {
-            unsigned new_used       = bits & ~(1u << idx[j]);
-            S        new_lambdas[4] = {S(0.0), S(0.0), S(0.0), S(0.0)};
-            sv_s1d(y, new_used, new_lambdas);
-            const V3<S> np     = sv_point(y, new_used, new_lambdas);
-            const S     d_star = dot(np, np);
-            if(d_star < d)
-            {
-                new_bits = new_used;
-                d        = d_star;
-                for(unsigned i = 0; i < 4; ++i)
-                    lambdas[i] = new_lambdas[i];
-            }
+            d    = d_star;
+            l[0] = j == 0 ? S(0.0) : la;
+            l[1] = j == 0 ? la : (j == 2 ? lb : S(0.0));
+            l[2] = j == 2 ? S(0.0) : lb;
+            used = (e & 1u) << (j == 0 ? 1 : 0) | (e >> 1) << (j == 2 ? 1 : 2);
         }
-    bits = new_bits;
+    }
+    return used;
 }
 
-// s3d (GJK_AY.cpp:215-301)
+// s3d (GJK_AY.cpp:215-301), its inside test: the faces (by the vertex they
+// leave out) to look at, or none and the weights
 template <typename S>
-GB_D void sv_s3d(const V3<S> y[4], unsigned& bits, S lambdas[4])
+GB_D unsigned sv_tetrahedron(const V3<S> y[4], S lambdas[4])
 {
     S C[4];
     C[0] = y[3].x * y[2].y * y[1].z + y[2].x * y[1].y * y[3].z + y[1].x * y[3].y * y[2].z
@@ -792,66 +783,130 @@ GB_D void sv_s3d(const V3<S> y[4], unsigned& bits, S lambdas[4])
            - y[0].x * y[1].y * y[3].z - y[1].x * y[3].y * y[0].z - y[3].x * y[0].y * y[1].z;
     C[3] = y[0].x * y[1].y * y[2].z + y[1].x * y[2].y * y[0].z + y[2].x * y[0].y * y[1].z
            - y[2].x * y[1].y * y[0].z - y[1].x * y[0].y * y[2].z - y[0].x * y[2].y * y[1].z;
-    const S  dM = C[0] + C[1] + C[2] + C[3];
-    unsigned sc[4];
+    const S  dM   = C[0] + C[1] + C[2] + C[3];
+    unsigned open = 0;
 #pragma unroll
-    for(int i = 0; i < 4; ++i)
-        sc[i] = sv_same_sign(dM, C[i]);
-    if(sc[0] + sc[1] + sc[2] + sc[3] == 4)
+    for(unsigned i = 0; i < 4; ++i)
+        open |= (1u - sv_same_sign(dM, C[i])) << i;
+    if(!open)
     {
 #pragma unroll
         for(int i = 0; i < 4; ++i)
             lambdas[i] = C[i] / dM;
-        return;
     }
-    S        d        = S(100000.0);
-    unsigned new_bits = 0;
-    for(unsigned j = 0; j < 4; ++j)
-        if(!sc[j])
-        {
-            unsigned new_used       = bits & ~(1u << j);
-            S        new_lambdas[4] = {S(0.0), S(0.0), S(0.0), S(0.0)};
-            sv_s2d(y, new_used, new_lambdas);
-            const V3<S> np     = sv_point(y, new_used, new_lambdas);
-            const S     d_star = dot(np, np);
-            if(d_star < d)
-            {
-                new_bits = new_used;
-                d        = d_star;
-                for(unsigned i = 0; i < 4; ++i)
-                    lambdas[i] = new_lambdas[i];
-            }
-        }
-    bits = new_bits;
+    return open;
 }
 
-// sv_subalgorithm (GJK_AY.cpp:340-368): new simplex, weights and closest point
-template <typename S>
+// sv_subalgorithm (GJK_AY.cpp:340-368): new simplex, weights and closest
+// point.  PAIRED (kGjkPaired): the two lanes of a pair share a tetrahedron's
+// open faces, the even lane the first and third, the odd one the second and
+// fourth, and agree on the nearest (the first one on ties, as one lane going
+// through all of them finds it); a triangle is one face, which both evaluate.
+template <bool PAIRED, typename S>
 GB_D V3<S> sv_subalgorithm(const V3<S> y[4], unsigned& bits, S lambdas[4])
 {
-    unsigned num_used = 0;
-#pragma unroll
-    for(unsigned i = 0; i < 4; ++i)
-        num_used += (bits >> i) & 1u;
+    const unsigned num_used = __popc(bits);
     if(num_used == 1)
     {
+#pragma unroll
         for(unsigned i = 0; i < 4; ++i)
             if(bits & (1u << i))
                 lambdas[i] = S(1.0);
     }
     else if(num_used == 2)
-        sv_s1d(y, bits, lambdas);
-    else if(num_used == 3)
-        sv_s2d(y, bits, lambdas);
+    {
+        const unsigned i = (unsigned)__ffs(bits) - 1u, j = 31u - (unsigned)__clz(bits);
+        S              la, lb;
+        const unsigned e = sv_edge(sv_pick(y, i), sv_pick(y, j), la, lb);
+#pragma unroll
+        for(unsigned k = 0; k < 4; ++k)
+            lambdas[k] = k == i ? la : (k == j ? lb : lambdas[k]);
+        bits = (e & 1u) << i | (e >> 1) << j;
+    }
     else
-        sv_s3d(y, bits, lambdas);
-    return sv_point(y, bits, lambdas);
+    {
+        const bool triangle = num_used == 3;
+        unsigned   open     = triangle ? 15u ^ bits : sv_tetrahedron(y, lambdas);
+        if(open)
+        {
+            const bool share = PAIRED && !triangle;
+            if(share) // this lane's faces
+            {
+                const unsigned first = open & (0u - open), rest = open ^ first;
+                const unsigned second = rest & (0u - rest), rest2 = rest ^ second;
+                const unsigned third  = rest2 & (0u - rest2);
+                open = threadIdx.x & 1u ? second | (rest2 ^ third) : first | third;
+            }
+            S        d    = S(100000.0);
+            unsigned used = 0, best = 4;
+            S        l[3] = {S(0.0), S(0.0), S(0.0)};
+            for(; open; open &= open - 1u)
+            {
+                const unsigned j    = (unsigned)__ffs(open) - 1u;
+                const V3<S>    Y[3] = {j == 0 ? y[1] : y[0], j <= 1 ? y[2] : y[1],
+                                       j <= 2 ? y[3] : y[2]};
+                S              ln[3];
+                const unsigned un = sv_face(Y, ln);
+                V3<S>          np = zero3<S>();
+#pragma unroll
+                for(unsigned k = 0; k < 3; ++k)
+                    if(un & (1u << k))
+                        np = np + ln[k] * Y[k];
+                const S d_star = dot(np, np);
+                if(triangle || d_star < d)
+                {
+                    d    = d_star;
+                    best = j;
+                    used = un;
+                    l[0] = ln[0];
+                    l[1] = ln[1];
+                    l[2] = ln[2];
+                }
+            }
+            if(share)
+            {
+                const unsigned lane = threadIdx.x & 31u, peer = lane ^ 1u;
+                const unsigned mask = 3u << (lane & ~1u);
+                const S        dp   = lane_shfl(mask, d, peer);
+                const unsigned bp   = __shfl_sync(mask, best, peer);
+                const unsigned up   = __shfl_sync(mask, used, peer);
+                const bool     theirs = dp < d || (dp == d && bp < best);
+#pragma unroll
+                for(int k = 0; k < 3; ++k)
+                {
+                    const S lp = lane_shfl(mask, l[k], peer);
+                    l[k]       = theirs ? lp : l[k];
+                }
+                best = theirs ? bp : best;
+                used = theirs ? up : used;
+            }
+            bits = 0;
+            if(best < 4)
+#pragma unroll
+                for(unsigned k = 0; k < 3; ++k)
+                {
+                    const unsigned i = sv_other(best, k);
+                    bits |= (used >> k & 1u) << i;
+#pragma unroll
+                    for(unsigned m = 0; m < 4; ++m)
+                        lambdas[m] = m == i ? l[k] : lambdas[m];
+                }
+        }
+    }
+    // computeVector (GJK_AY.cpp:304-316)
+    V3<S> o = zero3<S>();
+#pragma unroll
+    for(unsigned i = 0; i < 4; ++i)
+        if(bits & (1u << i))
+            o = o + lambdas[i] * y[i];
+    return o;
 }
 
 // w equal to a vertex of the simplex `bits` (degenerate, GJK_AY.cpp:373-386)
 template <typename S>
 GB_D bool sv_degenerate(unsigned bits, const V3<S> y[4], const V3<S>& w)
 {
+#pragma unroll
     for(unsigned i = 0; i < 4; ++i)
         if((bits & (1u << i)) && y[i].x == w.x && y[i].y == w.y && y[i].z == w.z)
             return true;
@@ -888,12 +943,7 @@ GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
     {
         if(!run)
             continue;
-        for(unsigned k = 0; k < 4; ++k)
-            if(!(bits & (1u << k)))
-            {
-                last = k;
-                break;
-            }
+        last = (unsigned)__ffs(~bits) - 1u; // the first free slot
         if constexpr(NESTEROV)
         {
             if(momentum)
@@ -919,8 +969,9 @@ GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
         }
         else
             d = v;
-        support2<PAIRED>(A, -d, B, mul_t(b2a.R, d), p[last], q[last]);
-        w         = p[last] - apply(b2a, q[last]);
+        V3<S> pn, qn;
+        support2<PAIRED>(A, -d, B, mul_t(b2a.R, d), pn, qn);
+        w          = pn - apply(b2a, qn);
         const S mu = dist - dot(v, w) / dist;
         if(mu < dist * rel_error || mu < abs_error || sv_degenerate(bits, y, w))
         {
@@ -930,10 +981,15 @@ GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
             momentum = false;
             continue;
         }
-        y[last] = w;
+#pragma unroll
+        for(unsigned i = 0; i < 4; ++i)
+            if(i == last)
+                y[i] = w;
+        p[last] = pn;
+        q[last] = qn;
         bits |= 1u << last;
         ++num_iterations;
-        v    = sv_subalgorithm(y, bits, lambdas);
+        v    = sv_subalgorithm<PAIRED>(y, bits, lambdas);
         dist = norm(v);
         s_prev = w;
         run    = bits < 15 && dist > k_higheps<S>() && num_iterations < 1000;

@@ -1714,17 +1714,11 @@ GB_D void for_each_pair(int64_t npairs, F&& f)
 {
     const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
     const int64_t tid      = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if(npairs < nthreads)
-    {
-        const int64_t nwarps = nthreads >> 5;
-        const int64_t k      = (npairs + nwarps - 1) / nwarps; // <= 32
-        const int64_t lane   = threadIdx.x & 31;
-        const int64_t p      = (tid >> 5) * k + lane;
-        if(lane < k && p < npairs)
-            f(p);
-    }
-    else
-        for(int64_t p = tid; p < npairs; p += nthreads)
+    const int64_t nwarps   = nthreads >> 5, lane = threadIdx.x & 31;
+    // records per warp and round: a short list's share, or one per lane
+    const int64_t k = npairs < nthreads ? (npairs + nwarps - 1) / nwarps : 32;
+    if(lane < k)
+        for(int64_t p = (tid >> 5) * k + lane; p < npairs; p += nwarps * k)
             f(p);
 }
 
@@ -1738,16 +1732,13 @@ GB_D void for_each_pair_converged(int64_t npairs, F&& f)
     const int64_t nwarps = (int64_t)gridDim.x * blockDim.x / 32;
     const int64_t warp   = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const int     slot   = (int)(threadIdx.x & 31u) / STEP;
-    if(npairs < nwarps * kPairs)
+    // pairs per warp and round: a short list's share, or all a warp holds
+    const int64_t k = npairs < nwarps * kPairs ? (npairs + nwarps - 1) / nwarps : kPairs;
+    for(int64_t base = warp * k; base < npairs; base += nwarps * k)
     {
-        const int64_t k = (npairs + nwarps - 1) / nwarps; // <= kPairs
-        const int64_t p = warp * k + slot;
-        if(warp * k < npairs)
-            f(slot < k && p < npairs ? p : npairs - 1, slot < k && p < npairs);
+        const bool valid = slot < k && base + slot < npairs;
+        f(valid ? base + slot : npairs - 1, valid);
     }
-    else
-        for(int64_t base = warp * kPairs; base < npairs; base += nwarps * kPairs)
-            f(base + slot < npairs ? base + slot : npairs - 1, base + slot < npairs);
 }
 
 // The narrow phase of a run whose bodies are all spheres: every record's
