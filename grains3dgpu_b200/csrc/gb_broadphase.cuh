@@ -430,13 +430,14 @@ __global__ void __launch_bounds__(kBlock) k_scan_apply(const uint32_t* __restric
 // tile is already running and the look-back ends; a bound on the wait still
 // stops it and flags kFlagScanStall.  Words of earlier scans carry another
 // epoch and read as unpublished, so the state needs no clearing between scans.
-// In place (in == out) is allowed.  abort_flags as for k_scan_apply.
+// In place (in == out) is allowed.  in2 (optional): the entries scanned are
+// in[i] + in2[i].  abort_flags as for k_scan_apply.
 constexpr unsigned long long kScanAggregate = 1ull, kScanPrefix = 2ull;
 constexpr uint32_t           kScanEpochMask = (1u << 30) - 1u;
 constexpr uint32_t           kScanSpinLimit = 1u << 20; // the default bound of the wait
 
 __global__ void __launch_bounds__(kBlock)
-    k_scan_onepass(const uint32_t* in, uint32_t* out, int64_t n,
+    k_scan_onepass(const uint32_t* in, const uint32_t* in2, uint32_t* out, int64_t n,
                    unsigned long long* __restrict__ tile_state,
                    unsigned long long* __restrict__ ticket, unsigned long long ticket_base,
                    uint32_t epoch, uint32_t* __restrict__ grand_total,
@@ -463,20 +464,28 @@ __global__ void __launch_bounds__(kBlock)
     // a thread's kItems (8) consecutive entries in two 16-byte loads where
     // they lie wholly in range and the arrays are 16-byte aligned
     const bool vec = kItems == 8 && base + kItems <= n
-                     && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u)
-                            == 0;
+                     && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(in2)
+                          | reinterpret_cast<uintptr_t>(out))
+                         & 15u) == 0;
     if(vec)
     {
         const uint4 a = *reinterpret_cast<const uint4*>(in + base);
         const uint4 b = *reinterpret_cast<const uint4*>(in + base + 4);
         v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
         v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        if(in2)
+        {
+            const uint4 c = *reinterpret_cast<const uint4*>(in2 + base);
+            const uint4 d = *reinterpret_cast<const uint4*>(in2 + base + 4);
+            v[0] += c.x, v[1] += c.y, v[2] += c.z, v[3] += c.w;
+            v[4] += d.x, v[5] += d.y, v[6] += d.z, v[7] += d.w;
+        }
     }
     else
     {
 #pragma unroll
         for(int j = 0; j < kItems; ++j)
-            v[j] = base + j < n ? in[base + j] : 0u;
+            v[j] = base + j < n ? in[base + j] + (in2 ? in2[base + j] : 0u) : 0u;
     }
 #pragma unroll
     for(int j = 0; j < kItems; ++j)

@@ -541,6 +541,13 @@ int ensure_stage(gb_ctx* c)
     return GB_OK;
 }
 
+// the two candidate counts of each id are 16-byte aligned arrays (vector loads
+// of the scan)
+size_t count_stride(const gb_ctx* c)
+{
+    return ((size_t)c->n + 4) & ~size_t(3);
+}
+
 int alloc_state(gb_ctx* c)
 {
     const size_t n = c->n, ss = store_size(c->prec);
@@ -567,7 +574,7 @@ int alloc_state(gb_ctx* c)
     GB_TRY(dalloc(&c->d_slot, (size_t)n * kPairSlots));
     GB_TRY(dalloc(&c->d_sorted_of, n));
     GB_TRY(dalloc(&c->d_obsmask_id, n));
-    GB_TRY(dalloc(&c->d_count, 2 * ((size_t)n + 1))); // count by id, then slot index by sorted position
+    GB_TRY(dalloc(&c->d_count, 2 * count_stride(c))); // obstacle, then particle candidates by id
     GB_TRY(dalloc(&c->d_contacts, n));
     GB_TRY(dalloc(&c->d_flags, 1));
     GB_TRY(dalloc(&c->d_counters, 4));
@@ -658,7 +665,7 @@ int ensure_pairs(gb_ctx* c, int64_t need)
 // exclusive scan of n counts in one launch (k_scan_onepass); every block
 // takes a ticket, so the host knows the counter's value before each launch
 int scan_u32(gb_ctx* c, const uint32_t* in, uint32_t* out, int64_t n, uint32_t* d_total,
-             const int* abort_flags = nullptr)
+             const int* abort_flags = nullptr, const uint32_t* in2 = nullptr)
 {
     const int nb = std::max(1, blocks(n, kTile));
     if((size_t)nb > c->tile_cap)
@@ -678,7 +685,7 @@ int scan_u32(gb_ctx* c, const uint32_t* in, uint32_t* out, int64_t n, uint32_t* 
                               c->stream));
         c->scan_epoch = 1;
     }
-    GB_CK(launch(c->pdl, k_scan_onepass, nb, kBlock, c->stream, in, out, n, c->d_tile_state,
+    GB_CK(launch(c->pdl, k_scan_onepass, nb, kBlock, c->stream, in, in2, out, n, c->d_tile_state,
                  c->d_ticket, c->tickets, c->scan_epoch, d_total, abort_flags, c->d_flags,
                  c->scan_spin_limit));
     c->tickets += (unsigned long long)nb;
@@ -1114,8 +1121,10 @@ int build_pairs(gb_ctx* c)
         GB_CK(cudaGetLastError());
         c->mask_valid = true;
     }
+    uint32_t* const obs_count = c->d_count;
+    uint32_t* const pcount    = c->d_count + count_stride(c);
     if(!c->count_zero)
-        GB_CK(cudaMemsetAsync(c->d_count, 0, 2 * ((size_t)n + 1) * sizeof(uint32_t), s));
+        GB_CK(cudaMemsetAsync(c->d_count, 0, 2 * count_stride(c) * sizeof(uint32_t), s));
     CellGeometry geo;
     for(int k = 0; k < 3; ++k)
         geo.mn[k] = c->cfg.origin[k];
@@ -1153,33 +1162,33 @@ int build_pairs(gb_ctx* c)
                      (const uint32_t*)c->d_sorted_of, c->d_fskey, c->d_fids, c->d_fref, c->d_fpos,
                      f32, (const int*)c->d_flags));
         c->fcount_zero = true; // each particle took back the count it added
-        GB_CK(launch(c->pdl, k_pair_count_fine<S>, nb, kBlock, s, n,
+        GB_CK(launch(c->pdl, k_pair_count_fine<S>, kHalfRows * nb, kBlock, s, n,
                      (const uint32_t*)c->d_fstart, g, (const uint32_t*)c->d_fskey,
                      (const uint32_t*)c->d_fids, (const uint32_t*)c->d_fref,
-                     (const double4*)c->d_fpos, (const float4*)f32, c->d_count,
-                     c->d_count + n + 1, c->d_slot, oc, (const int*)c->d_flags));
+                     (const double4*)c->d_fpos, (const float4*)f32, obs_count, pcount, c->d_slot,
+                     oc, (const int*)c->d_flags));
         const int nbl = std::max(1, blocks((int64_t)c->fine_nlarge * 32, kBlock));
         GB_CK(launch(c->pdl, k_pair_count_large<S>, nbl, kBlock, s, n,
                      (const uint32_t*)c->d_fstart, g, (const uint32_t*)c->d_fids,
                      (const uint32_t*)c->d_fref, (const double4*)c->d_fpos, (const float4*)f32,
-                     c->d_count, c->d_count + n + 1, c->d_slot, oc, (const int*)c->d_flags));
+                     obs_count, pcount, c->d_slot, oc, (const int*)c->d_flags));
         c->launches += 4;
     }
     else
     {
-        GB_CK(launch(c->pdl, k_pair_count<S>, nb, kBlock, s, n, c->d_skeys, c->d_sids,
+        GB_CK(launch(c->pdl, k_pair_count<S>, kHalfRows * nb, kBlock, s, n, c->d_skeys, c->d_sids,
                      c->d_spos, spos32, c->d_cstart, c->dims[0], c->dims[1], c->dims[2], geo,
-                     c->d_count, c->d_count + n + 1, c->d_slot, oc, (const int*)c->d_flags));
+                     obs_count, pcount, c->d_slot, oc, (const int*)c->d_flags));
         c->launches += 1;
     }
     GB_CK(cudaGetLastError());
-    GB_TRY(scan_u32(c, c->d_count, off, n, off + n, c->d_flags));
+    GB_TRY(scan_u32(c, pcount, off, n, off + n, c->d_flags, c->nob ? obs_count : nullptr));
     mark(c, 4);
     c->ovf_phase ^= 1;
     GB_CK(launch(c->pdl, k_pair_fill<S>, nb, kBlock, s, n, c->d_skeys, c->d_sids, c->d_sorted_of,
-                 c->d_spos, spos32, c->d_cstart, c->dims[0], c->dims[1], c->dims[2], c->d_count,
-                 c->d_slot, oc, off, c->d_pa, c->d_pb[c->cur], c->cap,
-                 c->d_flags, c->d_gjkn, c->d_count + n + 1, c->d_ovf, c->ovf_phase, c->d_obsq,
+                 c->d_spos, spos32, c->d_cstart, c->dims[0], c->dims[1], c->dims[2], obs_count,
+                 pcount, c->d_slot, oc, off, c->d_pa, c->d_pb[c->cur], c->cap,
+                 c->d_flags, c->d_gjkn, c->d_ovf, c->ovf_phase, c->d_obsq,
                  c->d_pc[c->cur], state_of<St>(c), tables_of<S>(c),
                  records_of<St>(c)));
     c->count_zero = true; // the fill pass zeroes each count it reads

@@ -558,19 +558,24 @@ GB_D void for_each_candidate(int s, const uint32_t* __restrict__ skeys,
     }
 }
 
-// Count pass over half of the stencil, one thread per sorted particle s.
-// The candidate test is symmetric bit for bit (b - a is -(a - b) exactly, and
-// the radius sum commutes), so each unordered pair is tested once: by s for
-// the partners t after it in the stencil's enumeration order -- the rest of
-// its own row (the cells x, x + 1 of row (dz, dy) = (0, 0) from s + 1 on,
-// one contiguous range) and the 4 rows (0, +1), (+1, -1), (+1, 0), (+1, +1).
-// A hit counts for both particles: count[id] (zeroed; the scan's input) and
-// pslot[sorted position] (zeroed; the slot index) by atomics, and the first
-// kPairSlots partners of each sorted position go to its slots in arrival
-// order.  The enumeration order of a particle's candidates is ascending
-// sorted position (rows ascend in (z, y), cells in x, ids within a cell), so
-// the fill pass restores it by sorting the slots.  Obstacle candidates are
-// added to count[id] by the particle itself.
+// Count pass over half of the stencil, five threads per sorted particle s,
+// one per row.  The candidate test is symmetric bit for bit (b - a is
+// -(a - b) exactly, and the radius sum commutes), so each unordered pair is
+// tested once: by s for the partners t after it in the stencil's enumeration
+// order -- the rest of its own row (the cells x, x + 1 of row (dz, dy) =
+// (0, 0) from s + 1 on, one contiguous range) and the 4 rows (0, +1),
+// (+1, -1), (+1, 0), (+1, +1).  A hit is recorded for both particles
+// (record_candidate): pcount[id] (zeroed) counts by one atomic, whose result
+// is the partner's slot, and the first kPairSlots partners go to the id's
+// slots in arrival order.  The enumeration order of a particle's candidates
+// is ascending sorted position (rows ascend in (z, y), cells in x, ids within
+// a cell), so the fill pass restores it by sorting the slots.  Obstacle
+// candidates are counted in obs_count[id] by the particle's own-row thread;
+// the scan adds the two.
+//
+// The rows are walked by threads of their own because the walk is a chain of
+// dependent loads (row bounds, then candidates): one thread per particle
+// waited through five chains in turn, and a small packing left the chip idle.
 //
 // Reach: a particle b hashed to a neighbour cell lies beyond the cell faces
 // that separate that cell from a's (a centre clamped into the grid lies
@@ -593,82 +598,80 @@ struct CellGeometry
     double rmax;  // largest bounding radius of any particle
 };
 
+// Candidate v (a sorted position) of particle id u: its slot and the count.
+GB_D void record_candidate(uint32_t id_u, uint32_t v, uint32_t* __restrict__ pcount,
+                           uint32_t* __restrict__ slot)
+{
+    const uint32_t k = atomicAdd(pcount + id_u, 1u);
+    if(k < kPairSlots)
+        slot[(size_t)id_u * kPairSlots + k] = v;
+}
+
+constexpr int kHalfRows = 5; // the rows of the half stencil, one thread each
+
 template <typename S>
 __global__ void __launch_bounds__(kBlock, sizeof(store_t<S>) == 4 ? 8 : 6)
     k_pair_count(int n, const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ sids,
                  const double4* __restrict__ spos, const float4* __restrict__ spos32,
                  const uint32_t* __restrict__ cstart, uint32_t nx, uint32_t ny, uint32_t nz,
-                 CellGeometry geo, uint32_t* __restrict__ count, uint32_t* __restrict__ pslot,
-                 uint32_t* __restrict__ slot, ObsCand oc, const int* abort_flags)
+                 CellGeometry geo, uint32_t* __restrict__ obs_count,
+                 uint32_t* __restrict__ pcount, uint32_t* __restrict__ slot, ObsCand oc,
+                 const int* abort_flags)
 {
     grid_dep_sync();
     constexpr bool STRICT = is_strict<S>(), PRE32 = is_mixed<S>();
-    const int      s      = blockIdx.x * blockDim.x + threadIdx.x;
+    const int      r      = 4 + (int)(blockIdx.x % kHalfRows); // row r of the 3 x 3 (dz, dy)
+    const int      s      = (int)(blockIdx.x / kHalfRows * blockDim.x + threadIdx.x);
     if(s >= n || step_aborted(abort_flags))
         return;
-    if(oc.n)
+    if(oc.n && r == 4)
     {
         const uint32_t a   = sids[s];
         const int      obs = obstacle_candidates(oc, a, (uint32_t)s);
         if(obs)
-            atomicAdd(count + a, (uint32_t)obs);
+            obs_count[a] = (uint32_t)obs;
     }
     const uint32_t key = skeys[s];
-    const double4  pa  = spos[s];
+    const int      cx = key % nx, cy = (key / nx) % ny, cz = key / (nx * ny);
+    const int      dz = r / 3 - 1, dy = r % 3 - 1;
+    const int      z = cz + dz, y = cy + dy;
+    if(z >= (int)nz || y < 0 || y >= (int)ny)
+        return;
+    const double4 pa = spos[s];
+    bool          left = cx > 0, right = cx + 1 < (int)nx;
+    if constexpr(!PRE32)
+    {
+        // distances from a to the faces of its cell (0 if a lies outside it)
+        const double reach = (pa.w + geo.rmax) * (1.0 + 1e-6) + 1e-6 * geo.cell;
+        const double r2    = reach * reach;
+        const double gxm   = fmax(pa.x - (geo.mn[0] + cx * geo.cell), 0.0);
+        const double gxp   = fmax(geo.mn[0] + (cx + 1) * geo.cell - pa.x, 0.0);
+        const double gy    = dy < 0   ? fmax(pa.y - (geo.mn[1] + cy * geo.cell), 0.0)
+                             : dy > 0 ? fmax(geo.mn[1] + (cy + 1) * geo.cell - pa.y, 0.0)
+                                      : 0.0;
+        const double gz    = dz > 0 ? fmax(geo.mn[2] + (cz + 1) * geo.cell - pa.z, 0.0) : 0.0;
+        const double d2    = gy * gy + gz * gz;
+        if(d2 > r2)
+            return;
+        left  = left && !(d2 + gxm * gxm > r2);
+        right = right && !(d2 + gxp * gxp > r2);
+    }
+    const uint32_t row = ((uint32_t)z * ny + (uint32_t)y) * nx;
+    const uint32_t t0 = r == 4 ? (uint32_t)s + 1 : cstart[row + (uint32_t)(left ? cx - 1 : cx)];
+    const uint32_t t1 = cstart[row + (uint32_t)(right ? cx + 2 : cx + 1)];
     float4         pa32;
     if constexpr(PRE32)
         pa32 = spos32[s];
-    const int cx = key % nx, cy = (key / nx) % ny, cz = key / (nx * ny);
-    auto record = [&](uint32_t u, uint32_t v) {
-        const uint32_t k = atomicAdd(pslot + u, 1u);
-        if(k < kPairSlots)
-            slot[(size_t)u * kPairSlots + k] = v;
-        atomicAdd(count + sids[u], 1u);
-    };
-    // distances from a to the faces of its cell (0 if a lies outside it)
-    constexpr bool PRUNE = !PRE32;
-    double         r2 = 0.0, gxm = 0.0, gxp = 0.0, gym = 0.0, gyp = 0.0, gzp = 0.0;
-    if constexpr(PRUNE)
-    {
-        const double reach = (pa.w + geo.rmax) * (1.0 + 1e-6) + 1e-6 * geo.cell;
-        r2                 = reach * reach;
-        gxm = fmax(pa.x - (geo.mn[0] + cx * geo.cell), 0.0);
-        gxp = fmax(geo.mn[0] + (cx + 1) * geo.cell - pa.x, 0.0);
-        gym = fmax(pa.y - (geo.mn[1] + cy * geo.cell), 0.0);
-        gyp = fmax(geo.mn[1] + (cy + 1) * geo.cell - pa.y, 0.0);
-        gzp = fmax(geo.mn[2] + (cz + 1) * geo.cell - pa.z, 0.0);
-    }
-    for(int r = 4; r < 9; ++r)
-    {
-        const int dz = r / 3 - 1, dy = r % 3 - 1;
-        const int z = cz + dz, y = cy + dy;
-        if(z >= (int)nz || y < 0 || y >= (int)ny)
-            continue;
-        bool left = cx > 0, right = cx + 1 < (int)nx;
-        if constexpr(PRUNE)
-        {
-            const double gy = dy < 0 ? gym : (dy > 0 ? gyp : 0.0);
-            const double gz = dz > 0 ? gzp : 0.0;
-            const double d2 = gy * gy + gz * gz;
-            if(d2 > r2)
-                continue;
-            left  = left && !(d2 + gxm * gxm > r2);
-            right = right && !(d2 + gxp * gxp > r2);
-        }
-        const uint32_t row = ((uint32_t)z * ny + (uint32_t)y) * nx;
-        const uint32_t t0 = r == 4 ? (uint32_t)s + 1 : cstart[row + (uint32_t)(left ? cx - 1 : cx)];
-        const uint32_t t1 = cstart[row + (uint32_t)(right ? cx + 2 : cx + 1)];
 #pragma unroll 2
-        for(uint32_t t = t0; t < t1; ++t)
+    for(uint32_t t = t0; t < t1; ++t)
+    {
+        if constexpr(PRE32)
+            if(pretest_rejects<PRE32>(pa32, spos32[t]))
+                continue;
+        if(exact_hit<STRICT>(pa, spos[t]))
         {
-            if constexpr(PRE32)
-                if(pretest_rejects<PRE32>(pa32, spos32[t]))
-                    continue;
-            if(exact_hit<STRICT>(pa, spos[t]))
-            {
-                record((uint32_t)s, t);
-                record(t, (uint32_t)s);
-            }
+            record_candidate(sids[s], t, pcount, slot);
+            record_candidate(sids[t], (uint32_t)s, pcount, slot);
         }
     }
 }
@@ -724,9 +727,9 @@ GB_D void warp_ranges(uint32_t t0, uint32_t t1, Visit&& visit)
 //     reach rL + r_max for large partners after it in the fine order.
 // Each unordered pair is tested once, with the same symmetric test
 // (pretest_rejects + exact_hit), and recorded for both particles into the
-// same slots and counts (by reference sorted position and id) as
-// k_pair_count: the fill pass's sort restores the reference's order, so
-// the pair list is the same, bit for bit.  A large particle's key is its
+// same slots and counts as k_pair_count (the partner by its reference sorted
+// position): the fill pass's sort restores the reference's order, so the
+// pair list is the same, bit for bit.  A large particle's key is its
 // fine cell plus nf (the fine cell count): the fine order holds the small
 // particles by cell, then the large ones by cell.
 struct FineGrid
@@ -787,70 +790,53 @@ __global__ void __launch_bounds__(kBlock)
     put_sorted(slot, (uint32_t)i, px, py, pz, rb_id, rcirc, fpos, fpos32);
 }
 
-// a hit between fine entries: both particles' slots and counts, by reference
-// sorted position and id, as k_pair_count records them
-GB_D void record_pair(uint32_t u, uint32_t id_u, uint32_t v, uint32_t id_v,
-                      uint32_t* __restrict__ count, uint32_t* __restrict__ pslot,
-                      uint32_t* __restrict__ slot)
-{
-    uint32_t k = atomicAdd(pslot + u, 1u);
-    if(k < kPairSlots)
-        slot[(size_t)u * kPairSlots + k] = v;
-    atomicAdd(count + id_u, 1u);
-    k = atomicAdd(pslot + v, 1u);
-    if(k < kPairSlots)
-        slot[(size_t)v * kPairSlots + k] = u;
-    atomicAdd(count + id_v, 1u);
-}
-
 // small particles: k_pair_count's half stencil on the fine grid (whose cells
-// hold small particles only); one thread per fine sorted position
+// hold small particles only); a thread per row of a fine sorted position
 template <typename S>
 __global__ void __launch_bounds__(kBlock, 6)
     k_pair_count_fine(int n, const uint32_t* __restrict__ fstart, FineGrid g,
                       const uint32_t* __restrict__ fskey, const uint32_t* __restrict__ fids,
                       const uint32_t* __restrict__ fref, const double4* __restrict__ fpos,
-                      const float4* __restrict__ fpos32, uint32_t* __restrict__ count,
-                      uint32_t* __restrict__ pslot, uint32_t* __restrict__ slot,
+                      const float4* __restrict__ fpos32, uint32_t* __restrict__ obs_count,
+                      uint32_t* __restrict__ pcount, uint32_t* __restrict__ slot,
                       ObsCand oc, const int* abort_flags)
 {
     grid_dep_sync();
     constexpr bool STRICT = is_strict<S>(), PRE32 = is_mixed<S>();
-    const int      f      = blockIdx.x * blockDim.x + threadIdx.x;
+    const int      r      = 4 + (int)(blockIdx.x % kHalfRows);
+    const int      f      = (int)(blockIdx.x / kHalfRows * blockDim.x + threadIdx.x);
     const uint32_t nx = g.nx, ny = g.ny, nz = g.nz;
     if(f >= n || step_aborted(abort_flags) || (uint32_t)f >= fstart[nx * ny * nz])
         return;
-    const uint32_t a = fids[f], sa = fref[f];
-    if(oc.n)
+    if(oc.n && r == 4)
     {
-        const int obs = obstacle_candidates(oc, a, sa);
+        const int obs = obstacle_candidates(oc, fids[f], fref[f]);
         if(obs)
-            atomicAdd(count + a, (uint32_t)obs);
+            obs_count[fids[f]] = (uint32_t)obs;
     }
     const uint32_t key = fskey[f];
-    const double4  pa  = fpos[f];
+    const int      cx = key % nx, cy = (key / nx) % ny, cz = key / (nx * ny);
+    const int      z = cz + r / 3 - 1, y = cy + r % 3 - 1;
+    if(z >= (int)nz || y < 0 || y >= (int)ny)
+        return;
+    const bool     left = cx > 0, right = cx + 1 < (int)nx;
+    const uint32_t row  = ((uint32_t)z * ny + (uint32_t)y) * nx;
+    const uint32_t t0 = r == 4 ? (uint32_t)f + 1 : fstart[row + (uint32_t)(left ? cx - 1 : cx)];
+    const uint32_t t1 = fstart[row + (uint32_t)(right ? cx + 2 : cx + 1)];
+    const double4  pa = fpos[f];
     float4         pa32;
     if constexpr(PRE32)
         pa32 = fpos32[f];
-    const int cx = key % nx, cy = (key / nx) % ny, cz = key / (nx * ny);
-    for(int r = 4; r < 9; ++r)
-    {
-        const int dz = r / 3 - 1, dy = r % 3 - 1;
-        const int z = cz + dz, y = cy + dy;
-        if(z >= (int)nz || y < 0 || y >= (int)ny)
-            continue;
-        const bool     left = cx > 0, right = cx + 1 < (int)nx;
-        const uint32_t row  = ((uint32_t)z * ny + (uint32_t)y) * nx;
-        const uint32_t t0 = r == 4 ? (uint32_t)f + 1 : fstart[row + (uint32_t)(left ? cx - 1 : cx)];
-        const uint32_t t1 = fstart[row + (uint32_t)(right ? cx + 2 : cx + 1)];
 #pragma unroll 2
-        for(uint32_t t = t0; t < t1; ++t)
+    for(uint32_t t = t0; t < t1; ++t)
+    {
+        if constexpr(PRE32)
+            if(pretest_rejects<PRE32>(pa32, fpos32[t]))
+                continue;
+        if(exact_hit<STRICT>(pa, fpos[t]))
         {
-            if constexpr(PRE32)
-                if(pretest_rejects<PRE32>(pa32, fpos32[t]))
-                    continue;
-            if(exact_hit<STRICT>(pa, fpos[t]))
-                record_pair(sa, a, fref[t], fids[t], count, pslot, slot);
+            record_candidate(fids[f], fref[t], pcount, slot);
+            record_candidate(fids[t], fref[f], pcount, slot);
         }
     }
 }
@@ -863,7 +849,7 @@ __global__ void __launch_bounds__(kBlock)
     k_pair_count_large(int n, const uint32_t* __restrict__ fstart, FineGrid g,
                        const uint32_t* __restrict__ fids, const uint32_t* __restrict__ fref,
                        const double4* __restrict__ fpos, const float4* __restrict__ fpos32,
-                       uint32_t* __restrict__ count, uint32_t* __restrict__ pslot,
+                       uint32_t* __restrict__ obs_count, uint32_t* __restrict__ pcount,
                        uint32_t* __restrict__ slot, ObsCand oc, const int* abort_flags)
 {
     grid_dep_sync();
@@ -878,7 +864,7 @@ __global__ void __launch_bounds__(kBlock)
     {
         const int obs = obstacle_candidates(oc, a, sa);
         if(obs)
-            atomicAdd(count + a, (uint32_t)obs);
+            obs_count[a] = (uint32_t)obs;
     }
     const double4 pa = fpos[f];
     float4        pa32;
@@ -917,7 +903,10 @@ __global__ void __launch_bounds__(kBlock)
                     if(pretest_rejects<PRE32>(pa32, fpos32[t]))
                         return;
                 if(exact_hit<STRICT>(pa, fpos[t]))
-                    record_pair(sa, a, fref[t], fids[t], count, pslot, slot);
+                {
+                    record_candidate(a, fref[t], pcount, slot);
+                    record_candidate(fids[t], sa, pcount, slot);
+                }
             });
         }
     }
@@ -1015,10 +1004,10 @@ GB_D void write_records(uint32_t a, const State<store_t<S>>& st, const Tables<S>
 }
 
 // Fill pass, one thread per particle id a (most have no candidate and read
-// only count[a]): the pair records of a at offset[a] -- its particle
-// candidates from the slots of its sorted position s = sorted_of[a], sorted
-// ascending (the enumeration order), or enumerated again in order when there
-// were more than kPairSlots -- then its obstacle candidates.  Every record's
+// only its two counts): the pair records of a at offset[a] -- its particle
+// candidates from its slots, sorted ascending (the enumeration order), or
+// enumerated again in order when there were more than kPairSlots -- then its
+// obstacle candidates.  Every record's
 // contact flag starts at 0, so that the narrow phase writes the records of
 // contacts only (outputs are read where the flag is set).
 template <typename S>
@@ -1026,12 +1015,11 @@ __global__ void __launch_bounds__(kBlock)
     k_pair_fill(int n, const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ sids,
                 const uint32_t* __restrict__ sorted_of, const double4* __restrict__ spos,
                 const float4* __restrict__ spos32, const uint32_t* __restrict__ cstart,
-                uint32_t nx, uint32_t ny, uint32_t nz, uint32_t* __restrict__ count,
-                const uint32_t* __restrict__ slot, ObsCand oc,
+                uint32_t nx, uint32_t ny, uint32_t nz, uint32_t* __restrict__ obs_count,
+                uint32_t* __restrict__ pcount, const uint32_t* __restrict__ slot, ObsCand oc,
                 const uint32_t* __restrict__ offset, uint32_t* __restrict__ pair_a,
                 uint32_t* __restrict__ pair_b, int64_t cap, int* __restrict__ flags,
-                uint32_t* __restrict__ gjk_count, uint32_t* __restrict__ pslot,
-                uint32_t* __restrict__ ovf_list, int ovf_phase, uint32_t* __restrict__ obs_queue,
+                uint32_t* __restrict__ gjk_count, uint32_t* __restrict__ ovf_list, int ovf_phase, uint32_t* __restrict__ obs_queue,
                 uint8_t* __restrict__ contact, State<store_t<S>> st, Tables<S> tb,
                 Records<store_t<S>> rec)
 {
@@ -1051,27 +1039,27 @@ __global__ void __launch_bounds__(kBlock)
     }
     if(a >= n || step_aborted(flags))
         return;
-    const uint32_t c = count[a];
-    if(c == 0)
+    const uint32_t cp = pcount[a], k_obs = oc.n ? obs_count[a] : 0u;
+    if(cp + k_obs == 0)
         return;
-    const int s = (int)sorted_of[a];
     int64_t out = offset[a];
-    if(out + c > cap)
+    if(out + cp + k_obs > cap)
     {
         atomicOr(flags, kFlagCapacity);
         return;
     }
     // the count pass's counters start the next step at zero (an aborted step
     // leaves them for the host's memset before its replay)
-    count[a] = 0u;
-    pslot[s] = 0u;
-    const uint32_t cp = c - (uint32_t)obstacle_candidates(oc, a, (uint32_t)s);
+    if(cp)
+        pcount[a] = 0u;
+    if(k_obs)
+        obs_count[a] = 0u;
     if(cp <= kPairSlots)
     {
         // the slots in registers (unused ones as 0xffffffff, above every
         // sorted position), sorted with static indices only, so nothing goes
         // to local memory
-        const uint4* mine = reinterpret_cast<const uint4*>(slot + (size_t)s * kPairSlots);
+        const uint4* mine = reinterpret_cast<const uint4*>(slot + (size_t)a * kPairSlots);
         uint32_t     t[kPairSlots];
 #pragma unroll
         for(int q = 0; q < kPairSlots / 4; ++q)
@@ -1113,19 +1101,18 @@ __global__ void __launch_bounds__(kBlock)
     }
     // the particle's obstacle records, contiguous after its particle pairs,
     // into the obstacle pass's queue
-    const uint32_t k_obs = c - cp;
     if(k_obs)
     {
         const uint32_t q = atomicAdd(gjk_count + 4 + ovf_phase, k_obs);
         for(uint32_t j = 0; j < k_obs; ++j)
             obs_queue[q + j] = (uint32_t)out + j;
+        for_each_obstacle_candidate(oc, a, sorted_of[a], [&](uint32_t o) {
+            pair_a[out]  = a;
+            pair_b[out]  = kObstacleBit | o;
+            contact[out] = 0;
+            ++out;
+        });
     }
-    for_each_obstacle_candidate(oc, a, (uint32_t)s, [&](uint32_t o) {
-        pair_a[out]  = a;
-        pair_b[out]  = kObstacleBit | o;
-        contact[out] = 0;
-        ++out;
-    });
     if(cp)
         write_records<S>((uint32_t)a, st, tb, rec);
 }
