@@ -77,6 +77,35 @@ int dalloc(T** p, size_t count)
     return GB_OK;
 }
 
+// Several device arrays in one allocation (each 256-byte aligned): a
+// cudaMalloc costs up to a millisecond, and a context needs some forty arrays.
+struct Arena
+{
+    struct Request
+    {
+        void** ptr;
+        size_t offset;
+    };
+    std::vector<Request> requests;
+    size_t               bytes = 0;
+
+    template <typename T>
+    void add(T** p, size_t count, size_t size = sizeof(T))
+    {
+        requests.push_back({(void**)p, bytes});
+        bytes += (std::max<size_t>(count, 1) * size + 255) & ~size_t(255);
+    }
+
+    // the allocation (`base`, to be freed as a whole), then every pointer
+    int allocate(char** base)
+    {
+        GB_CK(cudaMalloc((void**)base, std::max<size_t>(bytes, 256)));
+        for(const Request& r : requests)
+            *r.ptr = *base + r.offset;
+        return GB_OK;
+    }
+};
+
 template <typename T>
 void dfree(T*& p)
 {
@@ -147,6 +176,12 @@ struct gb_ctx
     // every body is a sphere)
     void* d_pose   = nullptr;
     void* d_sphere = nullptr;
+
+    // the allocations that hold the state, pair and fine-grid arrays
+    char* mem_state = nullptr;
+    char* mem_list  = nullptr; // the pair list and what the next step's history reads
+    char* mem_pairs = nullptr; // the other arrays of pair capacity
+    char* mem_fine  = nullptr;
 
     // state
     double*   d_pos = nullptr; // 3n
@@ -551,51 +586,50 @@ size_t count_stride(const gb_ctx* c)
 int alloc_state(gb_ctx* c)
 {
     const size_t n = c->n, ss = store_size(c->prec);
-    GB_TRY(dalloc(&c->d_pos, 3 * n));
-    GB_CK(cudaMalloc(&c->d_rot, std::max<size_t>(1, rot_count(c->prec) * n) * ss));
-    GB_CK(cudaMalloc(&c->d_vel, std::max<size_t>(1, 3 * n) * ss));
-    GB_CK(cudaMalloc(&c->d_omg, std::max<size_t>(1, 3 * n) * ss));
-    GB_CK(cudaMalloc(&c->d_frc, std::max<size_t>(1, 3 * n) * ss));
-    GB_CK(cudaMalloc(&c->d_trq, std::max<size_t>(1, 3 * n) * ss));
-    GB_CK(cudaMemset(c->d_frc, 0, std::max<size_t>(1, 3 * n) * ss));
-    GB_CK(cudaMemset(c->d_trq, 0, std::max<size_t>(1, 3 * n) * ss));
-    GB_TRY(dalloc(&c->d_rb_id, n));
-    GB_CK(cudaMemset(c->d_rb_id, 0, std::max<size_t>(1, n) * sizeof(uint32_t)));
-    GB_TRY(dalloc(&c->d_hash, n));
-    GB_TRY(dalloc(&c->d_iota, n));
+    Arena        m;
+    m.add(&c->d_pos, 3 * n);
+    m.add(&c->d_rot, rot_count(c->prec) * n, ss);
+    m.add(&c->d_vel, 3 * n, ss);
+    m.add(&c->d_omg, 3 * n, ss);
+    m.add(&c->d_frc, 3 * n, ss);
+    m.add(&c->d_trq, 3 * n, ss);
+    m.add(&c->d_rb_id, n);
+    m.add(&c->d_hash, n);
+    m.add(&c->d_iota, n);
     for(int b = 0; b < 2; ++b)
     {
-        GB_TRY(dalloc(&c->d_k[b], n));
-        GB_TRY(dalloc(&c->d_i[b], n));
-        GB_TRY(dalloc(&c->d_off[b], n + 1));
+        m.add(&c->d_k[b], n);
+        m.add(&c->d_i[b], n);
+        m.add(&c->d_off[b], n + 1);
     }
-    GB_TRY(dalloc(&c->d_spos, n));
-    GB_TRY(dalloc(&c->d_spos32, n));
-    GB_TRY(dalloc(&c->d_slot, (size_t)n * kPairSlots));
-    GB_TRY(dalloc(&c->d_sorted_of, n));
-    GB_TRY(dalloc(&c->d_obsmask_id, n));
-    GB_TRY(dalloc(&c->d_count, 2 * count_stride(c))); // obstacle, then particle candidates by id
-    GB_TRY(dalloc(&c->d_contacts, n));
-    GB_TRY(dalloc(&c->d_flags, 1));
-    GB_TRY(dalloc(&c->d_counters, 4));
+    m.add(&c->d_spos, n);
+    m.add(&c->d_spos32, n);
+    m.add(&c->d_slot, n * kPairSlots);
+    m.add(&c->d_sorted_of, n);
+    m.add(&c->d_obsmask_id, n);
+    m.add(&c->d_count, 2 * count_stride(c)); // obstacle, then particle candidates by id
+    m.add(&c->d_contacts, n);
+    m.add(&c->d_flags, 1);
+    m.add(&c->d_counters, 4);
     // [0], [1]: the GJK queues' lengths; [2], [3]: the fill pass's overflow
     // counts and [4], [5] its obstacle-record counts, alternating by step
-    GB_TRY(dalloc(&c->d_gjkn, 6));
+    m.add(&c->d_gjkn, 6);
+    m.add(&c->d_ovf, n);
+    m.add(&c->d_pcount, n);
+    m.add(&c->d_ticket, 1);
+    m.add(&c->d_done, 1);
+    GB_TRY(m.allocate(&c->mem_state));
+    GB_CK(cudaMemset(c->d_frc, 0, std::max<size_t>(1, 3 * n) * ss));
+    GB_CK(cudaMemset(c->d_trq, 0, std::max<size_t>(1, 3 * n) * ss));
+    GB_CK(cudaMemset(c->d_rb_id, 0, std::max<size_t>(1, n) * sizeof(uint32_t)));
     GB_CK(cudaMemset(c->d_gjkn, 0, 6 * sizeof(uint32_t)));
-    GB_TRY(dalloc(&c->d_ovf, n));
-    GB_TRY(dalloc(&c->d_pcount, n));
     GB_CK(cudaMemset(c->d_pcount, 0, (size_t)n * sizeof(uint32_t)));
-    if(!c->d_ticket)
-    {
-        GB_TRY(dalloc(&c->d_ticket, 1));
-        GB_CK(cudaMemset(c->d_ticket, 0, sizeof(unsigned long long)));
-        c->tickets = 0;
-    }
+    GB_CK(cudaMemset(c->d_ticket, 0, sizeof(unsigned long long)));
+    c->tickets = 0;
     GB_CK(cudaMemset(c->d_flags, 0, sizeof(int)));
     GB_CK(cudaMemset(c->d_counters, 0, 4 * sizeof(unsigned long long)));
     GB_CK(cudaMemset(c->d_contacts, 0, std::max<size_t>(1, n) * sizeof(int)));
     GB_CK(cudaMallocHost((void**)&c->h_pinned, 4 * sizeof(uint32_t)));
-    GB_TRY(dalloc(&c->d_done, 1));
     GB_CK(cudaMemset(c->d_done, 0, sizeof(unsigned int)));
     return GB_OK;
 }
@@ -608,20 +642,22 @@ int ensure_pairs(gb_ctx* c, int64_t need)
                                : std::max<int64_t>(need + need / 2, 1024);
     const size_t ss = store_size(c->prec);
     const bool   hist = c->cfg.contact_law == GB_LAW_HOOKE_HISTORY;
-    // the previous step's history buffers must survive the growth
+    Arena     m;
+    char*     mem = nullptr;
     uint32_t* npb[2] = {nullptr, nullptr};
     void*     nxi[2] = {nullptr, nullptr};
     uint8_t*  npc[2] = {nullptr, nullptr};
     for(int b = 0; b < 2; ++b)
     {
-        GB_TRY(dalloc(&npb[b], ncap));
-        if(hist || b == c->cur)
-            GB_TRY(dalloc(&npc[b], ncap));
+        m.add(&npb[b], ncap);
         if(hist)
-            GB_CK(cudaMalloc(&nxi[b], 3 * ncap * ss));
+            m.add(&nxi[b], 3 * ncap, ss);
+        if(hist || b == c->cur)
+            m.add(&npc[b], ncap);
     }
-    // (the previous step's pair count is on the device: copy the whole old
-    // capacity)
+    GB_TRY(m.allocate(&mem));
+    // the previous step's history buffers survive the growth (its pair count
+    // is on the device: the whole old capacity)
     const int prev = 1 - c->cur;
     if(c->have_prev && c->cap > 0)
     {
@@ -637,24 +673,21 @@ int ensure_pairs(gb_ctx* c, int64_t need)
     }
     for(int b = 0; b < 2; ++b)
     {
-        dfree(c->d_pb[b]);
         c->d_pb[b] = npb[b];
-        dfree(c->d_xi[b]);
         c->d_xi[b] = nxi[b];
-        dfree(c->d_pc[b]);
         c->d_pc[b] = npc[b];
     }
-    dfree(c->d_pa);
-    dfree(c->d_pf);
-    dfree(c->d_info);
-    dfree(c->d_gjkq);
-    GB_TRY(dalloc(&c->d_gjkq, 2 * ncap));
-    dfree(c->d_obsq);
-    GB_TRY(dalloc(&c->d_obsq, ncap));
-    GB_TRY(dalloc(&c->d_pa, ncap));
-    GB_CK(cudaMalloc(&c->d_pf, 9 * ncap * ss));
+    dfree(c->mem_list);
+    c->mem_list = mem;
+    dfree(c->mem_pairs);
+    Arena work;
+    work.add(&c->d_gjkq, 2 * ncap);
+    work.add(&c->d_obsq, ncap);
+    work.add(&c->d_pa, ncap);
+    work.add(&c->d_pf, 9 * ncap, ss);
     if(c->cfg.flags & GB_FLAG_RECORD_CONTACT_INFO)
-        GB_TRY(dalloc(&c->d_info, 7 * ncap));
+        work.add(&c->d_info, 7 * ncap);
+    GB_TRY(work.allocate(&c->mem_pairs));
     c->cap = ncap;
     return GB_OK;
 }
@@ -884,21 +917,19 @@ int fine_plan(gb_ctx* c)
     for(int i = 0; i < n; ++i)
         nlarge += r[i] > rs;
     // keys: the small particles' fine cells, then the large particles' (+ nf)
-    if(nf > c->fine_nf || !c->d_fcount)
+    if(nf > c->fine_nf || !c->mem_fine)
     {
-        dfree(c->d_fcount);
-        dfree(c->d_fstart);
-        GB_TRY(dalloc(&c->d_fcount, 2 * (size_t)nf + 1));
-        GB_TRY(dalloc(&c->d_fstart, 2 * (size_t)nf + 1));
-    }
-    if(!c->d_fkey)
-    {
-        GB_TRY(dalloc(&c->d_fkey, n));
-        GB_TRY(dalloc(&c->d_fskey, n));
-        GB_TRY(dalloc(&c->d_fids, n));
-        GB_TRY(dalloc(&c->d_fref, n));
-        GB_TRY(dalloc(&c->d_fpos, n));
-        GB_TRY(dalloc(&c->d_fpos32, n));
+        dfree(c->mem_fine);
+        Arena m;
+        m.add(&c->d_fcount, 2 * (size_t)nf + 1);
+        m.add(&c->d_fstart, 2 * (size_t)nf + 1);
+        m.add(&c->d_fkey, n);
+        m.add(&c->d_fskey, n);
+        m.add(&c->d_fids, n);
+        m.add(&c->d_fref, n);
+        m.add(&c->d_fpos, n);
+        m.add(&c->d_fpos32, n);
+        GB_TRY(m.allocate(&c->mem_fine));
     }
     GB_CK(cudaMemsetAsync(c->d_fcount, 0, (2 * (size_t)nf + 1) * sizeof(uint32_t), c->stream));
     c->fcount_zero = true;
@@ -1734,17 +1765,11 @@ int gb_destroy(gb_ctx* c)
         return GB_E_INVALID_ARG;
     if(c->stream)
         cudaStreamSynchronize(c->stream);
-    void* ptrs[] = {c->d_shape, c->d_inertia, c->d_verts, c->d_law, c->d_obs_shape, c->d_obs_tr,
-                    c->d_obs_mass, c->d_obs_plane, c->d_obs_vel, c->d_rcirc64, c->d_pos, c->d_rot, c->d_vel, c->d_omg, c->d_frc,
-                    c->d_trq, c->d_rb_id, c->d_hash, c->d_iota, c->d_k[0], c->d_k[1], c->d_i[0],
-                    c->d_i[1], c->d_hist, c->d_part, c->d_cstart, c->d_ccount, c->d_spos, c->d_spos32, c->d_slot, c->d_sorted_of, c->d_obsmask_id, c->d_count,
-                    c->d_off[0], c->d_off[1], c->d_pb[0], c->d_pb[1], c->d_pa, c->d_pf, c->d_pc[0], c->d_pc[1], c->d_pose, c->d_sphere,
-                    c->d_info, c->d_xi[0], c->d_xi[1], c->d_flags, c->d_counters, c->d_done,
-                    c->d_contacts,
-                    c->d_stage,     c->d_adj, c->d_tile_state, c->d_ticket, c->d_gjkq, c->d_gjkn,
-                    c->d_fkey, c->d_fcount, c->d_fstart, c->d_fskey, c->d_fids, c->d_fref,
-                    c->d_fpos, c->d_fpos32, c->d_ovf, c->d_pcount, c->d_cobs_start,
-                    c->d_cobs_ids, c->d_obsq};
+    void* ptrs[] = {c->d_shape,     c->d_inertia,    c->d_verts,   c->d_law,       c->d_obs_shape,
+                    c->d_obs_tr,    c->d_obs_mass,   c->d_obs_plane, c->d_obs_vel, c->d_rcirc64,
+                    c->d_hist,      c->d_part,       c->d_cstart,  c->d_ccount,    c->d_pose,
+                    c->d_sphere,    c->d_stage,      c->d_adj,     c->d_tile_state, c->d_cobs_start,
+                    c->d_cobs_ids,  c->mem_state,    c->mem_list,  c->mem_pairs,   c->mem_fine};
     for(void* p : ptrs)
         if(p)
             cudaFree(p);
