@@ -10,7 +10,7 @@
 // change.  State adjoints are 9 rows of n doubles: position, velocity,
 // angular velocity (x, y, z each).
 //
-// Deterministic: thread i gathers every contribution to particle i -- from
+// Deterministic: a lane pair gathers every contribution to particle i -- from
 // its own ordered pairs (i, j) and, recomputed, from the pairs (j, i) that
 // act on j -- and the law gradients are reduced in a fixed order.
 #pragma once
@@ -167,10 +167,16 @@ __global__ void __launch_bounds__(kBlock)
     }
 }
 
-// contacts: thread i adds to its adjoint the contributions of its own pairs
-// (i, j) and walls, and of the pairs (j, i) acting on its partners; block
-// partial sums of the law gradients go to partial[block][4 * laws.n]
-__global__ void __launch_bounds__(kBlock)
+// contacts: two lanes per particle i add to its adjoint the contributions of
+// its own pairs (i, j) and walls (the even lane) and of the pairs (j, i) acting
+// on its partners (the odd one); block partial sums of the law gradients go to
+// partial[block][4 * laws.n].  Latency-bound on a chain of partners per
+// particle, each two vector-Jacobian products: the lane pair halves it, and
+// blocks of 64 lanes keep a 50,000-grain packing on all SMs (256-thread blocks
+// with one lane per particle were 1.3 blocks per SM: 63 us a launch).
+constexpr int kAdjBlock = 64;
+
+__global__ void __launch_bounds__(kAdjBlock)
     k_adj_contacts(int n, State<double> st, const RBShape<double>* __restrict__ shape,
                    const RBInertia<double>* __restrict__ in, const uint32_t* __restrict__ off,
                    const uint32_t* __restrict__ pair_b, const uint8_t* __restrict__ contact,
@@ -178,11 +184,13 @@ __global__ void __launch_bounds__(kBlock)
                    const RBShape<double>* __restrict__ obs_shape, AdjLaws laws,
                    double* __restrict__ adj_prev, double* __restrict__ partial)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double    g_law[4 * kAdjMaxLaws];
+    const int  i   = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 1);
+    const bool own = (threadIdx.x & 1u) == 0u;
+    double     g_law[4 * kAdjMaxLaws];
 #pragma unroll
     for(int k = 0; k < 4 * kAdjMaxLaws; ++k)
         g_law[k] = 0.0;
+    V3<double> gx = zero3<double>(), gv = zero3<double>(), gw = zero3<double>();
     if(i < n)
     {
         double* const lf_[3] = {const_cast<double*>(lft), const_cast<double*>(lft) + n,
@@ -195,7 +203,6 @@ __global__ void __launch_bounds__(kBlock)
         const int        mat_i = shape[ri].material;
         const V3<double> xi = ld3(st.pos, i), vi = ld3(st.vel, i), wi = ld3(st.omg, i);
         const V3<double> lfi = ld3(lf_, i), lti = ld3(lt_, i);
-        V3<double>       gx = zero3<double>(), gv = zero3<double>(), gw = zero3<double>();
         for(uint32_t p = off[i]; p < off[i + 1]; ++p)
         {
             if(!contact[p])
@@ -203,6 +210,8 @@ __global__ void __launch_bounds__(kBlock)
             const uint32_t b = pair_b[p];
             if(b & kObstacleBit)
             {
+                if(!own)
+                    continue;
                 // sphere i against a Rectangle wall (closestPointsRectangle,
                 // CollisionDetection.cpp:53-90): s = rn . (xi - o) - r,
                 // vec = -s rn, pt = xi - r rn - s rn / 2
@@ -233,32 +242,32 @@ __global__ void __launch_bounds__(kBlock)
             const double     avm = m_i * m_j / (m_i + m_j);
             const V3<double> xj = ld3(st.pos, b), vj = ld3(st.vel, b), wj = ld3(st.omg, b);
             V3<double>       gxA, gxB, gvA, gwA, gvB, gwB;
-            // the pair (i, j): force on i
-            sphere_pair_vjp(xi, xj, r_i, r_j, laws.l[l], avm, vi, wi, vj, wj, lfi, lti, gxA, gxB,
-                            gvA, gwA, gvB, gwB, g_law + 4 * l);
-            gx = gx + gxA;
-            gv = gv + gvA;
-            gw = gw + gwA;
-            // the pair (j, i): force on j, its dependence on i (laws counted by j)
-            double scratch[4] = {0.0, 0.0, 0.0, 0.0};
-            sphere_pair_vjp(xj, xi, r_j, r_i, laws.l[l], avm, vj, wj, vi, wi, ld3(lf_, b),
-                            ld3(lt_, b), gxA, gxB, gvA, gwA, gvB, gwB, scratch);
-            gx = gx + gxB;
-            gv = gv + gvB;
-            gw = gw + gwB;
+            double           g4[4] = {0.0, 0.0, 0.0, 0.0};
+            // the pair (i, j), the force on i (laws counted by its lane), or
+            // the pair (j, i), the force on j and its dependence on i
+            sphere_pair_vjp(own ? xi : xj, own ? xj : xi, own ? r_i : r_j, own ? r_j : r_i,
+                            laws.l[l], avm, own ? vi : vj, own ? wi : wj, own ? vj : vi,
+                            own ? wj : wi, own ? lfi : ld3(lf_, b), own ? lti : ld3(lt_, b), gxA,
+                            gxB, gvA, gwA, gvB, gwB, g4);
+            gx = gx + (own ? gxA : gxB);
+            gv = gv + (own ? gvA : gvB);
+            gw = gw + (own ? gwA : gwB);
+            if(own)
+#pragma unroll
+                for(int q = 0; q < 4; ++q)
+                    g_law[4 * l + q] += g4[q];
         }
-        adj_prev[i]                 += gx.x;
-        adj_prev[(size_t)n + i]     += gx.y;
-        adj_prev[2 * (size_t)n + i] += gx.z;
-        adj_prev[3 * (size_t)n + i] += gv.x;
-        adj_prev[4 * (size_t)n + i] += gv.y;
-        adj_prev[5 * (size_t)n + i] += gv.z;
-        adj_prev[6 * (size_t)n + i] += gw.x;
-        adj_prev[7 * (size_t)n + i] += gw.y;
-        adj_prev[8 * (size_t)n + i] += gw.z;
+    }
+    const double g[9] = {gx.x, gx.y, gx.z, gv.x, gv.y, gv.z, gw.x, gw.y, gw.z};
+#pragma unroll
+    for(int k = 0; k < 9; ++k)
+    {
+        const double other = __shfl_xor_sync(0xffffffffu, g[k], 1);
+        if(own && i < n)
+            adj_prev[(size_t)k * n + i] += g[k] + other;
     }
     // block sums of the law gradients, in a fixed order: warp shuffles, then warps
-    __shared__ double red[kBlock / 32][4 * kAdjMaxLaws];
+    __shared__ double red[kAdjBlock / 32][4 * kAdjMaxLaws];
     const int         nv = 4 * laws.n;
     for(int k = 0; k < nv; ++k)
     {
@@ -270,26 +279,40 @@ __global__ void __launch_bounds__(kBlock)
             red[threadIdx.x >> 5][k] = v;
     }
     __syncthreads();
-    if(threadIdx.x < nv)
+    if((int)threadIdx.x < nv)
     {
         double v = 0.0;
-        for(int w = 0; w < kBlock / 32; ++w)
+        for(int w = 0; w < kAdjBlock / 32; ++w)
             v += red[w][threadIdx.x];
         partial[(size_t)blockIdx.x * nv + threadIdx.x] = v;
     }
 }
 
-// grad[k] += sum over blocks of partial[block][k], blocks in order
-__global__ void k_adj_reduce(int nblocks, int nv, const double* __restrict__ partial,
-                             double* __restrict__ grad)
+// grad[k] += the sum over blocks of partial[block][k]: one block per gradient,
+// its threads' strided sums, then warps, in a fixed order (one thread going
+// through all blocks took 15 us at 196 of them)
+__global__ void __launch_bounds__(kBlock)
+    k_adj_reduce(int nblocks, int nv, const double* __restrict__ partial,
+                 double* __restrict__ grad)
 {
-    const int k = threadIdx.x;
-    if(k >= nv)
-        return;
-    double v = 0.0;
-    for(int b = 0; b < nblocks; ++b)
+    const int         k = blockIdx.x;
+    __shared__ double red[kBlock / 32];
+    double            v = 0.0;
+    for(int b = threadIdx.x; b < nblocks; b += kBlock)
         v += partial[(size_t)b * nv + k];
-    grad[k] += v;
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1)
+        v += __shfl_down_sync(0xffffffffu, v, o);
+    if((threadIdx.x & 31) == 0)
+        red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if(threadIdx.x == 0)
+    {
+        double t = 0.0;
+        for(int w = 0; w < kBlock / 32; ++w)
+            t += red[w];
+        grad[k] += t;
+    }
 }
 
 } // namespace gb

@@ -2321,12 +2321,13 @@ int gb_adjoint_step(gb_ctx* c, const double* adj_next, double* adj_prev, double*
         laws.l[l] = {m.kn, m.en, m.etat, m.muc, L / std::sqrt(q), pi * pi / (q * std::sqrt(q)) / m.en};
     }
     const int    n  = c->n;
-    const int    nb = std::max(1, blocks(n, kBlock));
-    cudaStream_t s  = c->stream;
-    if(!c->d_adj || c->adj_cap < (size_t)(6 * n + nb * 4 * kAdjMaxLaws))
+    const int    nb  = std::max(1, blocks(n, kBlock));
+    const int    nba = std::max(1, blocks(2 * (int64_t)n, kAdjBlock)); // two lanes per particle
+    cudaStream_t s   = c->stream;
+    if(!c->d_adj || c->adj_cap < 6 * (size_t)n + (size_t)nba * 4 * kAdjMaxLaws)
     {
         dfree(c->d_adj);
-        c->adj_cap = (size_t)6 * n + (size_t)nb * 4 * kAdjMaxLaws;
+        c->adj_cap = 6 * (size_t)n + (size_t)nba * 4 * kAdjMaxLaws;
         GB_TRY(dalloc(&c->d_adj, c->adj_cap));
     }
     // the contacts of the current state; the accumulated torces are kept aside
@@ -2355,11 +2356,11 @@ int gb_adjoint_step(gb_ctx* c, const double* adj_next, double* adj_prev, double*
     const double h      = verlet && !c->verlet_started ? 0.5 * c->cfg.dt : c->cfg.dt;
     k_adj_integrate<<<nb, kBlock, 0, s>>>(n, c->cfg.dt, h, verlet ? 1 : 0, state, in, adj_next,
                                           adj_prev, lft);
-    k_adj_contacts<<<nb, kBlock, 0, s>>>(n, state, (const RBShape<double>*)c->d_shape, in,
+    k_adj_contacts<<<nba, kAdjBlock, 0, s>>>(n, state, (const RBShape<double>*)c->d_shape, in,
                                          c->d_off[c->cur], c->d_pb[c->cur], c->d_pc[c->cur], lft,
                                          c->d_obs_tr, (const RBShape<double>*)c->d_obs_shape,
                                          laws, adj_prev, part);
-    k_adj_reduce<<<1, 4 * kAdjMaxLaws, 0, s>>>(nb, 4 * nl, part, grad_laws);
+    k_adj_reduce<<<4 * nl, kBlock, 0, s>>>(nba, 4 * nl, part, grad_laws);
     c->launches += 3;
     GB_CK(cudaGetLastError());
     GB_CK(cudaMemcpyAsync(c->d_frc, c->d_stage, 3 * (size_t)n * sizeof(double),
