@@ -1216,12 +1216,11 @@ int build_pairs(gb_ctx* c)
     GB_TRY(scan_u32(c, pcount, off, n, off + n, c->d_flags, c->nob ? obs_count : nullptr));
     mark(c, 4);
     c->ovf_phase ^= 1;
-    GB_CK(launch(c->pdl, k_pair_fill<S>, nb, kBlock, s, n, c->d_skeys, c->d_sids, c->d_sorted_of,
-                 c->d_spos, spos32, c->d_cstart, c->dims[0], c->dims[1], c->dims[2], obs_count,
-                 pcount, c->d_slot, oc, off, c->d_pa, c->d_pb[c->cur], c->cap,
-                 c->d_flags, c->d_gjkn, c->d_ovf, c->ovf_phase, c->d_obsq,
-                 c->d_pc[c->cur], state_of<St>(c), tables_of<S>(c),
-                 records_of<St>(c)));
+    GB_CK(launch(c->pdl, k_pair_fill<S>, nb, kBlock, s, n, (const uint32_t*)c->d_sids,
+                 (const uint32_t*)c->d_sorted_of, obs_count, pcount, (const uint32_t*)c->d_slot,
+                 oc, (const uint32_t*)off, c->d_pa, c->d_pb[c->cur], c->cap, c->d_flags,
+                 c->d_gjkn, c->d_ovf, c->ovf_phase, c->d_obsq, c->d_pc[c->cur],
+                 state_of<St>(c), tables_of<S>(c), records_of<St>(c)));
     c->count_zero = true; // the fill pass zeroes each count it reads
     GB_CK(launch(c->pdl, k_pair_fill_overflow<S>, 4 * c->sms, 128, s,
                  (const uint32_t*)c->d_gjkn + 2 + c->ovf_phase, (const uint32_t*)c->d_ovf,

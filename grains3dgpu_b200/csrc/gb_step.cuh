@@ -1009,22 +1009,26 @@ GB_D void write_records(uint32_t a, const State<store_t<S>>& st, const Tables<S>
 // enumerated again in order when there were more than kPairSlots -- then its
 // obstacle candidates.  Every record's
 // contact flag starts at 0, so that the narrow phase writes the records of
-// contacts only (outputs are read where the flag is set).
+// contacts only (outputs are read where the flag is set).  A warp's particles
+// have consecutive ids and so nearly consecutive records: their sorted slots
+// are staged in shared memory and written out together, consecutive records
+// by consecutive lanes, where each lane writing its own few records cost a
+// partial sector per lane and array.
 template <typename S>
 __global__ void __launch_bounds__(kBlock)
-    k_pair_fill(int n, const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ sids,
-                const uint32_t* __restrict__ sorted_of, const double4* __restrict__ spos,
-                const float4* __restrict__ spos32, const uint32_t* __restrict__ cstart,
-                uint32_t nx, uint32_t ny, uint32_t nz, uint32_t* __restrict__ obs_count,
-                uint32_t* __restrict__ pcount, const uint32_t* __restrict__ slot, ObsCand oc,
+    k_pair_fill(int n, const uint32_t* __restrict__ sids, const uint32_t* __restrict__ sorted_of,
+                uint32_t* __restrict__ obs_count, uint32_t* __restrict__ pcount,
+                const uint32_t* __restrict__ slot, ObsCand oc,
                 const uint32_t* __restrict__ offset, uint32_t* __restrict__ pair_a,
                 uint32_t* __restrict__ pair_b, int64_t cap, int* __restrict__ flags,
-                uint32_t* __restrict__ gjk_count, uint32_t* __restrict__ ovf_list, int ovf_phase, uint32_t* __restrict__ obs_queue,
-                uint8_t* __restrict__ contact, State<store_t<S>> st, Tables<S> tb,
-                Records<store_t<S>> rec)
+                uint32_t* __restrict__ gjk_count, uint32_t* __restrict__ ovf_list, int ovf_phase,
+                uint32_t* __restrict__ obs_queue, uint8_t* __restrict__ contact,
+                State<store_t<S>> st, Tables<S> tb, Records<store_t<S>> rec)
 {
     grid_dep_sync();
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ uint32_t s_partner[kWarps][32 * kPairSlots]; // sorted positions ...
+    __shared__ uint8_t  s_owner[kWarps][32 * kPairSlots];   // ... and the lane they belong to
+    const int           a = blockIdx.x * blockDim.x + threadIdx.x;
     if(a == 0)
     {
         // the narrow phase's GJK queues of this step start empty: [0] the
@@ -1037,16 +1041,17 @@ __global__ void __launch_bounds__(kBlock)
         gjk_count[3 - ovf_phase] = 0;
         gjk_count[5 - ovf_phase] = 0;
     }
-    if(a >= n || step_aborted(flags))
+    if(step_aborted(flags)) // the same for the whole warp
         return;
-    const uint32_t cp = pcount[a], k_obs = oc.n ? obs_count[a] : 0u;
-    if(cp + k_obs == 0)
+    const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    uint32_t       cp = a < n ? pcount[a] : 0u, k_obs = a < n && oc.n ? obs_count[a] : 0u;
+    if(!__any_sync(0xffffffffu, cp + k_obs))
         return;
-    int64_t out = offset[a];
+    int64_t out = cp + k_obs ? offset[a] : 0;
     if(out + cp + k_obs > cap)
     {
         atomicOr(flags, kFlagCapacity);
-        return;
+        cp = k_obs = 0u;
     }
     // the count pass's counters start the next step at zero (an aborted step
     // leaves them for the host's memset before its replay)
@@ -1054,7 +1059,9 @@ __global__ void __launch_bounds__(kBlock)
         pcount[a] = 0u;
     if(k_obs)
         obs_count[a] = 0u;
-    if(cp <= kPairSlots)
+    const uint32_t m    = cp <= kPairSlots ? cp : 0u;
+    const uint32_t wmax = __reduce_max_sync(0xffffffffu, m);
+    if(wmax)
     {
         // the slots in registers (unused ones as 0xffffffff, above every
         // sorted position), sorted with static indices only, so nothing goes
@@ -1065,39 +1072,52 @@ __global__ void __launch_bounds__(kBlock)
         for(int q = 0; q < kPairSlots / 4; ++q)
         {
             uint4 x = make_uint4(~0u, ~0u, ~0u, ~0u);
-            if((uint32_t)(4 * q) < cp)
+            if((uint32_t)(4 * q) < m)
                 x = mine[q];
-            t[4 * q]     = (uint32_t)(4 * q) < cp ? x.x : ~0u;
-            t[4 * q + 1] = (uint32_t)(4 * q + 1) < cp ? x.y : ~0u;
-            t[4 * q + 2] = (uint32_t)(4 * q + 2) < cp ? x.z : ~0u;
-            t[4 * q + 3] = (uint32_t)(4 * q + 3) < cp ? x.w : ~0u;
+            t[4 * q]     = (uint32_t)(4 * q) < m ? x.x : ~0u;
+            t[4 * q + 1] = (uint32_t)(4 * q + 1) < m ? x.y : ~0u;
+            t[4 * q + 2] = (uint32_t)(4 * q + 2) < m ? x.z : ~0u;
+            t[4 * q + 3] = (uint32_t)(4 * q + 3) < m ? x.w : ~0u;
         }
         // a bitonic network over the warp's largest count (rounded up to 8,
         // 16 or 32 slots): one code path per warp, ~80 compare-exchanges for
         // the common 16 instead of 32 x 32 rank comparisons
-        const uint32_t wmax = __reduce_max_sync(__activemask(), cp);
         if(wmax <= 8)
             bitonic_sort<8>(t);
         else if(wmax <= 16)
             bitonic_sort<16>(t);
         else
             bitonic_sort<kPairSlots>(t);
+        const uint32_t incl  = warp_incl_scan(m);
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
 #pragma unroll
         for(int k = 0; k < kPairSlots; ++k)
-            if((uint32_t)k < cp)
+            if((uint32_t)k < m)
             {
-                pair_a[out + k]  = a;
-                pair_b[out + k]  = sids[t[k]];
-                contact[out + k] = 0;
+                s_partner[w][incl - m + k] = t[k];
+                s_owner[w][incl - m + k]   = (uint8_t)lane;
             }
-        out += cp;
+        __syncwarp();
+        const uint32_t shift = (uint32_t)out - (incl - m); // record minus staged index
+        for(uint32_t i0 = 0; i0 < total; i0 += 32)
+        {
+            const uint32_t i     = i0 + lane;
+            const unsigned owner = i < total ? s_owner[w][i] : 0u;
+            const uint32_t p     = __shfl_sync(0xffffffffu, shift, owner) + i;
+            if(i < total)
+            {
+                pair_a[p]  = (uint32_t)a - lane + owner;
+                pair_b[p]  = sids[s_partner[w][i]];
+                contact[p] = 0;
+            }
+        }
     }
-    else
+    out += cp;
+    if(cp > kPairSlots)
     {
         // more partners than slots (the largest grains of a polydisperse
         // packing): k_pair_fill_overflow writes them, a warp per particle
         ovf_list[atomicAdd(gjk_count + 2 + ovf_phase, 1u)] = (uint32_t)a;
-        out += cp;
     }
     // the particle's obstacle records, contiguous after its particle pairs,
     // into the obstacle pass's queue
