@@ -852,7 +852,10 @@ int redo_with_radix(gb_ctx* c)
 }
 
 // The finer candidate grid (k_pair_count_fine): r_s is the bounding radius
-// that 95% of the particles do not exceed; the grid is used where that is
+// that 97% of the particles do not exceed (a smaller share leaves more large
+// grains to their own pass, a larger one widens the cells; ten steps of the
+// 1M bed with 90, 95, 97 and 99%: 15.08, 14.42, 13.99 and 14.23 ms, of the
+// 130k bed in FP64 2.74, 2.73, 2.70 and 2.85 ms); the grid is used where that is
 // below 0.7 of the largest radius (a polydisperse packing), the rigid-body
 // ids are known on the host, and its cell count stays moderate.  The split
 // only decides which kernel tests a pair, never whether it is tested, so a
@@ -872,7 +875,7 @@ int fine_plan(gb_ctx* c)
     for(int i = 0; i < n; ++i)
         r[i] = bound_radius(c, c->h_rb_id[i]);
     std::vector<double> q(r);
-    const size_t k = (size_t)(0.95 * (n - 1));
+    const size_t k = (size_t)(0.97 * (n - 1));
     std::nth_element(q.begin(), q.begin() + k, q.end());
     const double rs = q[k];
     if(!(rs > 0.0) || !(rs < 0.7 * c->rmax))
