@@ -788,7 +788,7 @@ int broad_phase_radix(gb_ctx* c)
     k_gather_sorted<<<nb, kBlock, 0, s>>>(n, c->d_sids, c->d_pos, c->d_pos + n,
                                           c->d_pos + 2 * (size_t)n, c->d_rb_id, c->d_rcirc64,
                                           c->d_spos,
-                                          c->prec == GB_MIXED ? c->d_spos32 : nullptr,
+                                          c->d_spos32,
                                           c->d_sorted_of);
     c->launches += 2;
     GB_CK(cudaGetLastError());
@@ -825,7 +825,7 @@ int broad_phase_counting(gb_ctx* c)
     c->d_sids  = c->d_i[1];
     GB_CK(launch(c->pdl, k_cell_rank, nb, kBlock, s, n, c->d_i[0], c->d_hash, c->d_cstart,
                  c->d_skeys, c->d_sids, c->d_pos, c->d_pos + n, c->d_pos + 2 * (size_t)n,
-                 c->d_rb_id, c->d_rcirc64, c->d_spos, c->prec == GB_MIXED ? c->d_spos32 : nullptr,
+                 c->d_rb_id, c->d_rcirc64, c->d_spos, c->d_spos32,
                  c->d_sorted_of, c->d_flags));
     c->launches += 1;
     GB_CK(cudaGetLastError());
@@ -1146,7 +1146,8 @@ int build_pairs(gb_ctx* c)
         c->cur ^= 1; // last step's pair list becomes the history
     GB_TRY(ensure_pairs(c, c->cap_hint));
     uint32_t*       off    = c->d_off[c->cur];
-    const float4*   spos32 = c->prec == GB_MIXED ? c->d_spos32 : nullptr;
+    const float4*   spos32 = c->d_spos32;
+    constexpr bool  STRICT = is_strict<S>();
     if(c->nob && !c->mask_valid)
     {
         GB_CK(launch(c->pdl, k_obstacle_mask<S>, nb, kBlock, s, n, state_of<St>(c),
@@ -1159,11 +1160,6 @@ int build_pairs(gb_ctx* c)
     uint32_t* const pcount    = c->d_count + count_stride(c);
     if(!c->count_zero)
         GB_CK(cudaMemsetAsync(c->d_count, 0, 2 * count_stride(c) * sizeof(uint32_t), s));
-    CellGeometry geo;
-    for(int k = 0; k < 3; ++k)
-        geo.mn[k] = c->cfg.origin[k];
-    geo.cell = c->cell;
-    geo.rmax = c->rmax;
     if(!c->fine_planned)
         GB_TRY(fine_plan(c));
     if(!c->cobs_valid)
@@ -1179,7 +1175,7 @@ int build_pairs(gb_ctx* c)
     {
         // the finer grid of the small particles, then the count passes
         const FineGrid& g   = c->fine_g;
-        float4*         f32 = c->prec == GB_MIXED ? c->d_fpos32 : nullptr;
+        float4*         f32 = c->d_fpos32;
         if(!c->fcount_zero)
             GB_CK(cudaMemsetAsync(c->d_fcount, 0, (2 * (size_t)c->fine_nf + 1) * sizeof(uint32_t),
                                   s));
@@ -1196,13 +1192,13 @@ int build_pairs(gb_ctx* c)
                      (const uint32_t*)c->d_sorted_of, c->d_fskey, c->d_fids, c->d_fref, c->d_fpos,
                      f32, (const int*)c->d_flags));
         c->fcount_zero = true; // each particle took back the count it added
-        GB_CK(launch(c->pdl, k_pair_count_fine<S>, kHalfRows * nb, kBlock, s, n,
+        GB_CK(launch(c->pdl, k_pair_count_fine<STRICT>, kHalfRows * nb, kBlock, s, n,
                      (const uint32_t*)c->d_fstart, g, (const uint32_t*)c->d_fskey,
                      (const uint32_t*)c->d_fids, (const uint32_t*)c->d_fref,
                      (const double4*)c->d_fpos, (const float4*)f32, obs_count, pcount, c->d_slot,
                      oc, (const int*)c->d_flags));
         const int nbl = std::max(1, blocks((int64_t)c->fine_nlarge * 32, kBlock));
-        GB_CK(launch(c->pdl, k_pair_count_large<S>, nbl, kBlock, s, n,
+        GB_CK(launch(c->pdl, k_pair_count_large<STRICT>, nbl, kBlock, s, n,
                      (const uint32_t*)c->d_fstart, g, (const uint32_t*)c->d_fids,
                      (const uint32_t*)c->d_fref, (const double4*)c->d_fpos, (const float4*)f32,
                      obs_count, pcount, c->d_slot, oc, (const int*)c->d_flags));
@@ -1210,8 +1206,8 @@ int build_pairs(gb_ctx* c)
     }
     else
     {
-        GB_CK(launch(c->pdl, k_pair_count<S>, kHalfRows * nb, kBlock, s, n, c->d_skeys, c->d_sids,
-                     c->d_spos, spos32, c->d_cstart, c->dims[0], c->dims[1], c->dims[2], geo,
+        GB_CK(launch(c->pdl, k_pair_count<STRICT>, kHalfRows * nb, kBlock, s, n, c->d_skeys, c->d_sids,
+                     c->d_spos, spos32, c->d_cstart, c->dims[0], c->dims[1], c->dims[2],
                      obs_count, pcount, c->d_slot, oc, (const int*)c->d_flags));
         c->launches += 1;
     }
@@ -1225,7 +1221,7 @@ int build_pairs(gb_ctx* c)
                  c->d_gjkn, c->d_ovf, c->ovf_phase, c->d_obsq, c->d_pc[c->cur],
                  state_of<St>(c), tables_of<S>(c), records_of<St>(c)));
     c->count_zero = true; // the fill pass zeroes each count it reads
-    GB_CK(launch(c->pdl, k_pair_fill_overflow<S>, 4 * c->sms, 128, s,
+    GB_CK(launch(c->pdl, k_pair_fill_overflow<STRICT>, 4 * c->sms, 128, s,
                  (const uint32_t*)c->d_gjkn + 2 + c->ovf_phase, (const uint32_t*)c->d_ovf,
                  (const uint32_t*)c->d_skeys, (const uint32_t*)c->d_sids,
                  (const uint32_t*)c->d_sorted_of, (const double4*)c->d_spos, spos32,

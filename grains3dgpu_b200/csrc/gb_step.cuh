@@ -273,10 +273,10 @@ GB_D Law<S> load_law(const Law<store_t<S>>* t, int ma, int mb)
 // The three cells x-1, x, x+1 of one (y, z) row have consecutive keys, so
 // their particles are one contiguous range of the sorted order: the walk is
 // nine ranges, visiting the candidates in the same order as the 27 cells.
-// PRE32 (the mixed mode): a conservative FP32 test on spos32 (put_sorted
-// inflates its radii by a bound on the FP32 rounding, so an FP32 rejection
-// implies an FP64 rejection) skips most non-candidates before the FP64 test:
-// the candidate set is the FP64 test's.  The FP64 modes test in FP64 only.
+// A conservative FP32 test on spos32 (put_sorted inflates its radii by a bound
+// on the FP32 rounding, so an FP32 rejection implies an FP64 rejection) skips
+// most non-candidates before the FP64 test, in every mode: the candidate set
+// is the FP64 test's.
 // Candidates kept per particle by the count pass: 32 covers all but ~1e-4 of
 // the particles of a dense polydisperse bed (mean ~7, 99.9th percentile ~25);
 // the fill pass enumerates the rest again.
@@ -473,22 +473,16 @@ GB_D constexpr bool is_strict()
 
 // The candidate test of sorted particles a and b: |d| - (rA + rB) < 0 in
 // FP64 (ComponentManagerCPU.cpp:372-380; the strict mode in the reference's
-// operation order), behind the FP32 pre-test of the mixed mode, whose
-// rejection is certified (put_sorted inflates the FP32 radii).  The
+// operation order), behind the FP32 pre-test, whose rejection is certified
+// (put_sorted inflates the FP32 radii).  The
 // products and sums are written as explicit round-to-nearest operations, so
 // that every kernel that enumerates candidates -- the count pass and the
 // re-enumeration of the fill pass -- takes the same decisions.
-template <bool PRE32>
 GB_D bool pretest_rejects(const float4& a32, const float4& q)
 {
-    if constexpr(PRE32)
-    {
-        const float fx = __fsub_rn(q.x, a32.x), fy = __fsub_rn(q.y, a32.y);
-        const float fz = __fsub_rn(q.z, a32.z), fr = __fadd_rn(a32.w, q.w);
-        return __fmaf_rn(fz, fz, __fmaf_rn(fy, fy, __fmul_rn(fx, fx))) >= __fmul_rn(fr, fr);
-    }
-    else
-        return false;
+    const float fx = __fsub_rn(q.x, a32.x), fy = __fsub_rn(q.y, a32.y);
+    const float fz = __fsub_rn(q.z, a32.z), fr = __fadd_rn(a32.w, q.w);
+    return __fmaf_rn(fz, fz, __fmaf_rn(fy, fy, __fmul_rn(fx, fx))) >= __fmul_rn(fr, fr);
 }
 
 template <bool STRICT>
@@ -527,37 +521,6 @@ GB_D void neighbour_row(const uint32_t* __restrict__ cstart, uint32_t nx, uint32
     end                = cstart[row + (uint32_t)x1 + 1];
 }
 
-template <bool STRICT, bool PRE32, typename Hit>
-GB_D void for_each_candidate(int s, const uint32_t* __restrict__ skeys,
-                             const double4* __restrict__ spos,
-                             const float4* __restrict__ spos32,
-                             const uint32_t* __restrict__ cstart, uint32_t nx, uint32_t ny,
-                             uint32_t nz, Hit&& hit)
-{
-    const uint32_t key = skeys[s];
-    const double4  pa  = spos[s];
-    float4         pa32;
-    if constexpr(PRE32)
-        pa32 = spos32[s];
-    const int cx = key % nx, cy = (key / nx) % ny, cz = key / (nx * ny);
-    for(int r = 0; r < 9; ++r)
-    {
-        uint32_t t0, t1;
-        neighbour_row(cstart, nx, ny, nz, cx, cy, cz, r, t0, t1);
-        // the particle itself passes every test below and is dropped
-        // only on a hit, which keeps the common path short
-#pragma unroll 2
-        for(uint32_t t = t0; t < t1; ++t)
-        {
-            if constexpr(PRE32)
-                if(pretest_rejects<PRE32>(pa32, spos32[t]))
-                    continue;
-            if(exact_hit<STRICT>(pa, spos[t]) && t != (uint32_t)s)
-                hit(t);
-        }
-    }
-}
-
 // Count pass over half of the stencil, five threads per sorted particle s,
 // one per row.  The candidate test is symmetric bit for bit (b - a is
 // -(a - b) exactly, and the radius sum commutes), so each unordered pair is
@@ -577,26 +540,11 @@ GB_D void for_each_candidate(int s, const uint32_t* __restrict__ skeys,
 // dependent loads (row bounds, then candidates): one thread per particle
 // waited through five chains in turn, and a small packing left the chip idle.
 //
-// Reach: a particle b hashed to a neighbour cell lies beyond the cell faces
-// that separate that cell from a's (a centre clamped into the grid lies
-// further out still), so |a - b| is at least the distance from a to those
-// faces, and a candidate needs |a - b| < rA + rB <= rA + rmax.  The rows and
-// the end cells of a row that are farther than that, with a margin far above
-// the rounding of the hash and of the faces, hold no pair that the exact test
-// accepts and are not walked; the pair set is unchanged.  The FP64 modes
-// prune so (their exact test on every candidate is the costly part); the
-// mixed mode does not, since its FP32 pre-test is cheap and a warp walks the
-// longest range among its lanes anyway: pruning measured slower there.
-//
-// Latency-bound on L1 hits: the mixed instantiation runs at full occupancy
-// (32 registers), which measured 5% faster than 40 registers at six blocks
-// per SM.
-struct CellGeometry
-{
-    double mn[3]; // grid origin
-    double cell;  // cell edge
-    double rmax;  // largest bounding radius of any particle
-};
+// The FP32 test passes one candidate in some 5 to 15, so in nearly every round
+// a few lanes of a warp have a hit; tested and recorded where they are found,
+// the FP64 test and the two atomics ran in nearly every round for those few
+// lanes and were most of the instructions.  The hits of a warp are queued in
+// shared memory instead and taken 32 at a time.
 
 // Candidate v (a sorted position) of particle id u: its slot and the count.
 GB_D void record_candidate(uint32_t id_u, uint32_t v, uint32_t* __restrict__ pcount,
@@ -607,73 +555,104 @@ GB_D void record_candidate(uint32_t id_u, uint32_t v, uint32_t* __restrict__ pco
         slot[(size_t)id_u * kPairSlots + k] = v;
 }
 
+// A warp's FP32 hits (s, t): at most 31 left over and two rounds of 32.
+struct HitQueue
+{
+    uint32_t s[96], t[96];
+};
+
+GB_D void push_hit(HitQueue& q, unsigned& n, bool hit, uint32_t s, uint32_t t)
+{
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    if(hit)
+    {
+        const unsigned k = n + __popc(m & ((1u << (threadIdx.x & 31u)) - 1u));
+        q.s[k]           = s;
+        q.t[k]           = t;
+    }
+    n += __popc(m);
+}
+
+// record(s, t) for the queued hits that the FP64 test keeps, while a whole
+// round of them is queued, or all of them (`flush`)
+template <bool STRICT, typename Record>
+GB_D void take_hits(HitQueue& q, unsigned& n, bool flush, const double4* __restrict__ pos,
+                    Record&& record)
+{
+    while(n >= 32u || (flush && n))
+    {
+        const unsigned lane = threadIdx.x & 31u, k = n < 32u ? n : 32u;
+        n -= k;
+        __syncwarp();
+        if(lane < k)
+        {
+            const uint32_t s = q.s[n + lane], t = q.t[n + lane];
+            if(exact_hit<STRICT>(pos[s], pos[t]))
+                record(s, t);
+        }
+        __syncwarp();
+    }
+}
+
+// A warp walks its lanes' candidate ranges [t0, t1) of the lanes' particles s
+// (an empty range on the lanes without one).
+template <bool STRICT, typename Record>
+GB_D void walk_rows(uint32_t s, uint32_t t0, uint32_t t1, const double4* __restrict__ pos,
+                    const float4* __restrict__ pos32, HitQueue& q, Record&& record)
+{
+    const uint32_t len    = t1 > t0 ? t1 - t0 : 0u;
+    const uint32_t rounds = __reduce_max_sync(0xffffffffu, len);
+    if(!rounds)
+        return;
+    const float4 a32 = len ? pos32[s] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    unsigned     n   = 0; // queued hits, warp-uniform
+    for(uint32_t k = 0; k < rounds; k += 2)
+    {
+        const bool h0 = k < len && !pretest_rejects(a32, pos32[t0 + k]);
+        const bool h1 = k + 1 < len && !pretest_rejects(a32, pos32[t0 + k + 1]);
+        push_hit(q, n, h0, s, t0 + k);
+        push_hit(q, n, h1, s, t0 + k + 1);
+        take_hits<STRICT>(q, n, k + 2 >= rounds, pos, record);
+    }
+}
+
 constexpr int kHalfRows = 5; // the rows of the half stencil, one thread each
 
-template <typename S>
-__global__ void __launch_bounds__(kBlock, sizeof(store_t<S>) == 4 ? 8 : 6)
+template <bool STRICT>
+__global__ void __launch_bounds__(kBlock, 8)
     k_pair_count(int n, const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ sids,
                  const double4* __restrict__ spos, const float4* __restrict__ spos32,
                  const uint32_t* __restrict__ cstart, uint32_t nx, uint32_t ny, uint32_t nz,
-                 CellGeometry geo, uint32_t* __restrict__ obs_count,
-                 uint32_t* __restrict__ pcount, uint32_t* __restrict__ slot, ObsCand oc,
-                 const int* abort_flags)
+                 uint32_t* __restrict__ obs_count, uint32_t* __restrict__ pcount,
+                 uint32_t* __restrict__ slot, ObsCand oc, const int* abort_flags)
 {
     grid_dep_sync();
-    constexpr bool STRICT = is_strict<S>(), PRE32 = is_mixed<S>();
-    const int      r      = 4 + (int)(blockIdx.x % kHalfRows); // row r of the 3 x 3 (dz, dy)
-    const int      s      = (int)(blockIdx.x / kHalfRows * blockDim.x + threadIdx.x);
-    if(s >= n || step_aborted(abort_flags))
+    __shared__ HitQueue s_hits[kWarps];
+    const int           r = 4 + (int)(blockIdx.x % kHalfRows); // row r of the 3 x 3 (dz, dy)
+    const int           s = (int)(blockIdx.x / kHalfRows * blockDim.x + threadIdx.x);
+    if(step_aborted(abort_flags))
         return;
-    if(oc.n && r == 4)
+    uint32_t t0 = 0, t1 = 0;
+    if(s < n)
     {
-        const uint32_t a   = sids[s];
-        const int      obs = obstacle_candidates(oc, a, (uint32_t)s);
-        if(obs)
-            obs_count[a] = (uint32_t)obs;
-    }
-    const uint32_t key = skeys[s];
-    const int      cx = key % nx, cy = (key / nx) % ny, cz = key / (nx * ny);
-    const int      dz = r / 3 - 1, dy = r % 3 - 1;
-    const int      z = cz + dz, y = cy + dy;
-    if(z >= (int)nz || y < 0 || y >= (int)ny)
-        return;
-    const double4 pa = spos[s];
-    bool          left = cx > 0, right = cx + 1 < (int)nx;
-    if constexpr(!PRE32)
-    {
-        // distances from a to the faces of its cell (0 if a lies outside it)
-        const double reach = (pa.w + geo.rmax) * (1.0 + 1e-6) + 1e-6 * geo.cell;
-        const double r2    = reach * reach;
-        const double gxm   = fmax(pa.x - (geo.mn[0] + cx * geo.cell), 0.0);
-        const double gxp   = fmax(geo.mn[0] + (cx + 1) * geo.cell - pa.x, 0.0);
-        const double gy    = dy < 0   ? fmax(pa.y - (geo.mn[1] + cy * geo.cell), 0.0)
-                             : dy > 0 ? fmax(geo.mn[1] + (cy + 1) * geo.cell - pa.y, 0.0)
-                                      : 0.0;
-        const double gz    = dz > 0 ? fmax(geo.mn[2] + (cz + 1) * geo.cell - pa.z, 0.0) : 0.0;
-        const double d2    = gy * gy + gz * gz;
-        if(d2 > r2)
-            return;
-        left  = left && !(d2 + gxm * gxm > r2);
-        right = right && !(d2 + gxp * gxp > r2);
-    }
-    const uint32_t row = ((uint32_t)z * ny + (uint32_t)y) * nx;
-    const uint32_t t0 = r == 4 ? (uint32_t)s + 1 : cstart[row + (uint32_t)(left ? cx - 1 : cx)];
-    const uint32_t t1 = cstart[row + (uint32_t)(right ? cx + 2 : cx + 1)];
-    float4         pa32;
-    if constexpr(PRE32)
-        pa32 = spos32[s];
-#pragma unroll 2
-    for(uint32_t t = t0; t < t1; ++t)
-    {
-        if constexpr(PRE32)
-            if(pretest_rejects<PRE32>(pa32, spos32[t]))
-                continue;
-        if(exact_hit<STRICT>(pa, spos[t]))
+        if(oc.n && r == 4)
         {
-            record_candidate(sids[s], t, pcount, slot);
-            record_candidate(sids[t], (uint32_t)s, pcount, slot);
+            const uint32_t a   = sids[s];
+            const int      obs = obstacle_candidates(oc, a, (uint32_t)s);
+            if(obs)
+                obs_count[a] = (uint32_t)obs;
         }
+        const uint32_t key = skeys[s];
+        const int      cx = key % nx, cy = (key / nx) % ny, cz = key / (nx * ny);
+        neighbour_row(cstart, nx, ny, nz, cx, cy, cz, r, t0, t1);
+        if(r == 4)
+            t0 = (uint32_t)s + 1;
     }
+    walk_rows<STRICT>((uint32_t)s, t0, t1, spos, spos32, s_hits[threadIdx.x >> 5],
+                      [&](uint32_t u, uint32_t v) {
+                          record_candidate(sids[u], v, pcount, slot);
+                          record_candidate(sids[v], u, pcount, slot);
+                      });
 }
 
 // A warp walks the concatenation of up to 32 ranges [t0, t1) of sorted
@@ -792,8 +771,8 @@ __global__ void __launch_bounds__(kBlock)
 
 // small particles: k_pair_count's half stencil on the fine grid (whose cells
 // hold small particles only); a thread per row of a fine sorted position
-template <typename S>
-__global__ void __launch_bounds__(kBlock, 6)
+template <bool STRICT>
+__global__ void __launch_bounds__(kBlock, 8)
     k_pair_count_fine(int n, const uint32_t* __restrict__ fstart, FineGrid g,
                       const uint32_t* __restrict__ fskey, const uint32_t* __restrict__ fids,
                       const uint32_t* __restrict__ fref, const double4* __restrict__ fpos,
@@ -802,49 +781,37 @@ __global__ void __launch_bounds__(kBlock, 6)
                       ObsCand oc, const int* abort_flags)
 {
     grid_dep_sync();
-    constexpr bool STRICT = is_strict<S>(), PRE32 = is_mixed<S>();
-    const int      r      = 4 + (int)(blockIdx.x % kHalfRows);
-    const int      f      = (int)(blockIdx.x / kHalfRows * blockDim.x + threadIdx.x);
-    const uint32_t nx = g.nx, ny = g.ny, nz = g.nz;
-    if(f >= n || step_aborted(abort_flags) || (uint32_t)f >= fstart[nx * ny * nz])
+    __shared__ HitQueue s_hits[kWarps];
+    const int           r = 4 + (int)(blockIdx.x % kHalfRows);
+    const int           f = (int)(blockIdx.x / kHalfRows * blockDim.x + threadIdx.x);
+    if(step_aborted(abort_flags))
         return;
-    if(oc.n && r == 4)
+    uint32_t t0 = 0, t1 = 0;
+    if(f < n && (uint32_t)f < fstart[g.nx * g.ny * g.nz])
     {
-        const int obs = obstacle_candidates(oc, fids[f], fref[f]);
-        if(obs)
-            obs_count[fids[f]] = (uint32_t)obs;
-    }
-    const uint32_t key = fskey[f];
-    const int      cx = key % nx, cy = (key / nx) % ny, cz = key / (nx * ny);
-    const int      z = cz + r / 3 - 1, y = cy + r % 3 - 1;
-    if(z >= (int)nz || y < 0 || y >= (int)ny)
-        return;
-    const bool     left = cx > 0, right = cx + 1 < (int)nx;
-    const uint32_t row  = ((uint32_t)z * ny + (uint32_t)y) * nx;
-    const uint32_t t0 = r == 4 ? (uint32_t)f + 1 : fstart[row + (uint32_t)(left ? cx - 1 : cx)];
-    const uint32_t t1 = fstart[row + (uint32_t)(right ? cx + 2 : cx + 1)];
-    const double4  pa = fpos[f];
-    float4         pa32;
-    if constexpr(PRE32)
-        pa32 = fpos32[f];
-#pragma unroll 2
-    for(uint32_t t = t0; t < t1; ++t)
-    {
-        if constexpr(PRE32)
-            if(pretest_rejects<PRE32>(pa32, fpos32[t]))
-                continue;
-        if(exact_hit<STRICT>(pa, fpos[t]))
+        if(oc.n && r == 4)
         {
-            record_candidate(fids[f], fref[t], pcount, slot);
-            record_candidate(fids[t], fref[f], pcount, slot);
+            const int obs = obstacle_candidates(oc, fids[f], fref[f]);
+            if(obs)
+                obs_count[fids[f]] = (uint32_t)obs;
         }
+        const uint32_t key = fskey[f];
+        const int cx = key % g.nx, cy = (key / g.nx) % g.ny, cz = key / (g.nx * g.ny);
+        neighbour_row(fstart, g.nx, g.ny, g.nz, cx, cy, cz, r, t0, t1);
+        if(r == 4)
+            t0 = (uint32_t)f + 1;
     }
+    walk_rows<STRICT>((uint32_t)f, t0, t1, fpos, fpos32, s_hits[threadIdx.x >> 5],
+                      [&](uint32_t u, uint32_t v) {
+                          record_candidate(fids[u], fref[v], pcount, slot);
+                          record_candidate(fids[v], fref[u], pcount, slot);
+                      });
 }
 
 // large particles (keys past the small ones'), one warp each: small partners
 // from the fine cells within reach rL + r_s, then large partners after it in
 // the fine order from the large particles' cells within reach rL + r_max
-template <typename S>
+template <bool STRICT>
 __global__ void __launch_bounds__(kBlock)
     k_pair_count_large(int n, const uint32_t* __restrict__ fstart, FineGrid g,
                        const uint32_t* __restrict__ fids, const uint32_t* __restrict__ fref,
@@ -853,7 +820,9 @@ __global__ void __launch_bounds__(kBlock)
                        uint32_t* __restrict__ slot, ObsCand oc, const int* abort_flags)
 {
     grid_dep_sync();
-    constexpr bool STRICT = is_strict<S>(), PRE32 = is_mixed<S>();
+    __shared__ HitQueue s_hits[kWarps];
+    HitQueue&           hits  = s_hits[threadIdx.x >> 5];
+    unsigned            nhits = 0;
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t nf   = g.nx * g.ny * g.nz;
     const int64_t  f    = (int64_t)fstart[nf] + ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
@@ -867,9 +836,11 @@ __global__ void __launch_bounds__(kBlock)
             obs_count[a] = (uint32_t)obs;
     }
     const double4 pa = fpos[f];
-    float4        pa32;
-    if constexpr(PRE32)
-        pa32 = fpos32[f];
+    const float4  pa32 = fpos32[f];
+    auto          record = [&](uint32_t u, uint32_t v) {
+        record_candidate(fids[u], fref[v], pcount, slot);
+        record_candidate(fids[v], fref[u], pcount, slot);
+    };
     for(int large = 0; large < 2; ++large)
     {
         // the fine cells of the box [x - reach, x + reach]
@@ -897,19 +868,12 @@ __global__ void __launch_bounds__(kBlock)
                     t0 = (uint32_t)f + 1; // each large pair once
             }
             warp_ranges(t0, t1, [&](uint32_t t, bool valid) {
-                if(!valid)
-                    return;
-                if constexpr(PRE32)
-                    if(pretest_rejects<PRE32>(pa32, fpos32[t]))
-                        return;
-                if(exact_hit<STRICT>(pa, fpos[t]))
-                {
-                    record_candidate(a, fref[t], pcount, slot);
-                    record_candidate(fids[t], sa, pcount, slot);
-                }
+                push_hit(hits, nhits, valid && !pretest_rejects(pa32, fpos32[t]), (uint32_t)f, t);
+                take_hits<STRICT>(hits, nhits, false, fpos, record);
             });
         }
     }
+    take_hits<STRICT>(hits, nhits, true, fpos, record);
 }
 
 // Ascending sort of t[0, N) in registers by a bitonic network (Batcher, 1968):
@@ -1142,7 +1106,7 @@ __global__ void __launch_bounds__(kBlock)
 // for_each_candidate walks them), 32 candidates a round, the hits of a round
 // written in lane order (ballot + prefix count), so the list is the one
 // for_each_candidate writes.
-template <typename S>
+template <bool STRICT>
 __global__ void __launch_bounds__(128)
     k_pair_fill_overflow(const uint32_t* __restrict__ ovf_count,
                          const uint32_t* __restrict__ ovf_list, const uint32_t* __restrict__ skeys,
@@ -1154,7 +1118,6 @@ __global__ void __launch_bounds__(128)
                          const int* __restrict__ flags)
 {
     grid_dep_sync();
-    constexpr bool STRICT = is_strict<S>(), PRE32 = is_mixed<S>();
     if(step_aborted(flags))
         return;
     const unsigned lane  = threadIdx.x & 31u;
@@ -1167,9 +1130,7 @@ __global__ void __launch_bounds__(128)
         uint32_t       out = offset[a];
         const uint32_t key = skeys[s];
         const double4  pa  = spos[s];
-        float4         pa32;
-        if constexpr(PRE32)
-            pa32 = spos32[s];
+        const float4   pa32 = spos32[s];
         const int cx = key % nx, cy = (key / nx) % ny, cz = key / (nx * ny);
         // the 9 rows of 3 cells, lane r holding row r, walked as one sequence
         uint32_t t0 = 0, t1 = 0;
@@ -1177,8 +1138,7 @@ __global__ void __launch_bounds__(128)
             neighbour_row(cstart, nx, ny, nz, cx, cy, cz, (int)lane, t0, t1);
         warp_ranges(t0, t1, [&](uint32_t t, bool valid) {
             bool hit = valid && t != s;
-            if constexpr(PRE32)
-                hit = hit && !pretest_rejects<PRE32>(pa32, spos32[t]);
+            hit = hit && !pretest_rejects(pa32, spos32[t]);
             hit                 = hit && exact_hit<STRICT>(pa, spos[t]);
             const unsigned bits = __ballot_sync(0xffffffffu, hit);
             if(hit)
