@@ -551,20 +551,11 @@ GB_D GjkResult<S> gjk_jh(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
 {
     unsigned bits = 0, last = 0, last_bit = 0, all_bits = 0;
     V3<S>    p[4], q[4];
+    // the tables need no initial values: a subset of all_bits has had its
+    // determinants computed when the last of its points came in, and points
+    // are read through `bits` and `all_bits` only (clearing the tables was a
+    // kilobyte of local memory per lane and solve)
     JH<S>    jh;
-#pragma unroll
-    for(int i = 0; i < 16; ++i)
-#pragma unroll
-        for(int j = 0; j < 4; ++j)
-            jh.det[i][j] = S(0.0);
-#pragma unroll
-    for(int i = 0; i < 4; ++i)
-    {
-#pragma unroll
-        for(int j = 0; j < 4; ++j)
-            jh.dp[i][j] = S(0.0);
-        p[i] = q[i] = jh.y[i] = zero3<S>();
-    }
     S       mu = S(0.0);
     int     num_iterations = 0;
     const S rel_error      = k_loweps<S>();

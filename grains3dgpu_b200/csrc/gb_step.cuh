@@ -175,7 +175,8 @@ GB_D Contact<float> closest_spheres_mixed(double rA, double rB, const double xa[
     const double     nd = norm(d64), overlap = nd - rA - rB;
     if(!(overlap < 0.0))
         return no_contact<float>();
-    const V3<double> u = d64 / nd;
+    // one FP64 division (the result is rounded to FP32)
+    const V3<double> u = (1.0 / nd) * d64;
     Contact<double>  c;
     c.pt      = (rA + 0.5 * overlap) * u;
     c.vec     = overlap * u;
@@ -657,11 +658,13 @@ __global__ void __launch_bounds__(kBlock, 8)
 
 // A warp walks the concatenation of up to 32 ranges [t0, t1) of sorted
 // positions, lane r holding range r (lanes past the last range hold empty
-// ones), 32 entries a round in range order: visit(t, valid) runs on every
-// lane each round (warp-uniform).  All ranges' bounds are loaded at once, by
+// ones), ROUNDS x 32 entries at a time in range order: visit(t, valid) with
+// the lane's ROUNDS entries (entry k of a lane is the k-th group of 32's) runs
+// on every lane (warp-uniform).  All ranges' bounds are loaded at once, by
 // their lanes, and short ranges share rounds, where a range-at-a-time walk
-// pays a dependent load pair and a mostly idle round per range.
-template <typename Visit>
+// pays a dependent load pair and a mostly idle round per range.  More rounds
+// at a time put more loads in flight where a warp works alone.
+template <int ROUNDS, typename Visit>
 GB_D void warp_ranges(uint32_t t0, uint32_t t1, Visit&& visit)
 {
     const unsigned lane = threadIdx.x & 31u;
@@ -676,18 +679,25 @@ GB_D void warp_ranges(uint32_t t0, uint32_t t1, Visit&& visit)
     }
     const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
     const uint32_t exc   = inc - len;
-    for(uint32_t base = 0; base < total; base += 32)
+    for(uint32_t base = 0; base < total; base += 32 * ROUNDS)
     {
-        const uint32_t idx = base + lane;
-        // the last range that starts at or before idx (exclusive prefixes
-        // do not decrease; an empty range shares its start with the next)
-        unsigned r = 0;
+        uint32_t t[ROUNDS];
+        bool     valid[ROUNDS];
 #pragma unroll
-        for(unsigned step = 16; step >= 1; step >>= 1)
-            if(__shfl_sync(0xffffffffu, exc, r + step) <= idx)
-                r += step;
-        const uint32_t t = __shfl_sync(0xffffffffu, t0, r) + (idx - __shfl_sync(0xffffffffu, exc, r));
-        visit(t, idx < total);
+        for(int k = 0; k < ROUNDS; ++k)
+        {
+            const uint32_t idx = base + 32u * k + lane;
+            // the last range that starts at or before idx (exclusive prefixes
+            // do not decrease; an empty range shares its start with the next)
+            unsigned r = 0;
+#pragma unroll
+            for(unsigned step = 16; step >= 1; step >>= 1)
+                if(__shfl_sync(0xffffffffu, exc, r + step) <= idx)
+                    r += step;
+            t[k] = __shfl_sync(0xffffffffu, t0, r) + (idx - __shfl_sync(0xffffffffu, exc, r));
+            valid[k] = idx < total;
+        }
+        visit(t, valid);
     }
 }
 
@@ -867,8 +877,11 @@ __global__ void __launch_bounds__(kBlock)
                 if(large && t0 < (uint32_t)f + 1)
                     t0 = (uint32_t)f + 1; // each large pair once
             }
-            warp_ranges(t0, t1, [&](uint32_t t, bool valid) {
-                push_hit(hits, nhits, valid && !pretest_rejects(pa32, fpos32[t]), (uint32_t)f, t);
+            warp_ranges<2>(t0, t1, [&](const uint32_t(&t)[2], const bool(&valid)[2]) {
+                const bool h0 = valid[0] && !pretest_rejects(pa32, fpos32[t[0]]);
+                const bool h1 = valid[1] && !pretest_rejects(pa32, fpos32[t[1]]);
+                push_hit(hits, nhits, h0, (uint32_t)f, t[0]);
+                push_hit(hits, nhits, h1, (uint32_t)f, t[1]);
                 take_hits<STRICT>(hits, nhits, false, fpos, record);
             });
         }
@@ -1102,10 +1115,9 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 // The particle pairs of the particles whose partners overflowed their slots,
-// one warp per particle: the 27 cells in the reference's order (as
-// for_each_candidate walks them), 32 candidates a round, the hits of a round
-// written in lane order (ballot + prefix count), so the list is the one
-// for_each_candidate writes.
+// one warp per particle: the 27 cells in the reference's order,
+// four rounds of 32 candidates at a time (a particle is one chain of dependent
+// rounds), the hits of a round written in lane order (ballot + prefix count).
 template <bool STRICT>
 __global__ void __launch_bounds__(128)
     k_pair_fill_overflow(const uint32_t* __restrict__ ovf_count,
@@ -1136,19 +1148,25 @@ __global__ void __launch_bounds__(128)
         uint32_t t0 = 0, t1 = 0;
         if(lane < 9)
             neighbour_row(cstart, nx, ny, nz, cx, cy, cz, (int)lane, t0, t1);
-        warp_ranges(t0, t1, [&](uint32_t t, bool valid) {
-            bool hit = valid && t != s;
-            hit = hit && !pretest_rejects(pa32, spos32[t]);
-            hit                 = hit && exact_hit<STRICT>(pa, spos[t]);
-            const unsigned bits = __ballot_sync(0xffffffffu, hit);
-            if(hit)
+        warp_ranges<4>(t0, t1, [&](const uint32_t(&t)[4], const bool(&valid)[4]) {
+            bool hit[4];
+#pragma unroll
+            for(int k = 0; k < 4; ++k)
+                hit[k] = valid[k] && t[k] != s && !pretest_rejects(pa32, spos32[t[k]]);
+#pragma unroll
+            for(int k = 0; k < 4; ++k)
             {
-                const uint32_t k = out + __popc(bits & ((1u << lane) - 1u));
-                pair_a[k]        = a;
-                pair_b[k]        = sids[t];
-                contact[k]       = 0;
+                const bool     h    = hit[k] && exact_hit<STRICT>(pa, spos[t[k]]);
+                const unsigned bits = __ballot_sync(0xffffffffu, h);
+                if(h)
+                {
+                    const uint32_t q = out + __popc(bits & ((1u << lane) - 1u));
+                    pair_a[q]        = a;
+                    pair_b[q]        = sids[t[k]];
+                    contact[q]       = 0;
+                }
+                out += __popc(bits);
             }
-            out += __popc(bits);
         });
     }
 }
