@@ -106,9 +106,10 @@ GB_D S sgn(S x)
 GB_D V3<double> support_sq_log(const Body<double>& b, const V3<double>& v)
 {
     const double abvx = fabs(v.x), abvy = fabs(v.y), abvz = fabs(v.z);
-    const double la = b.k[4] * log2(b.k[0] * abvy / abvx);              // log2 alpha
-    const double lt = log2(1.0 + exp2(b.p[4] * la));                     // log2 temp
-    const double lb = b.k[5] * lt + b.k[3] * log2(b.k[1] * abvz / abvx); // log2 beta
+    const double rx = 1.0 / abvx;
+    const double la = b.k[4] * log2(b.k[0] * abvy * rx);              // log2 alpha
+    const double lt = log2(1.0 + exp2(b.p[4] * la));                   // log2 temp
+    const double lb = b.k[5] * lt + b.k[3] * log2(b.k[1] * abvz * rx); // log2 beta
     const double xt = exp2(-b.k[7] * log2(exp2(b.k[6] * lt) + exp2(b.p[3] * lb)));
     return mk<double>(sgn(v.x) * b.p[0] * xt, sgn(v.y) * exp2(la) * b.p[1] * xt,
                       sgn(v.z) * exp2(lb) * b.p[2] * xt);
@@ -193,6 +194,32 @@ GB_D V3<S> support(const Body<S>& b, const V3<S>& v)
                          S(0.0));
         default:
             return mk<S>(S(0.0), S(0.0), S(0.0));
+    }
+}
+
+// support(b, 0), where every GJK starts, without evaluating it: the signs of a
+// superquadric's components are those of 0, a box or rectangle takes its
+// positive corner, a polyhedron's first vertex is never beaten, and a
+// sphere's quotient is 0/0.  (For a superquadric it was a whole log-domain
+// chain, for a polyhedron a loop over its vertices.)
+template <typename S>
+GB_D V3<S> support_zero(const Body<S>& b)
+{
+    switch(b.type)
+    {
+        case GB_POLYHEDRON:
+        {
+            const Vert<store_t<S>> q = b.verts[0];
+            return mk<S>(S(q.x), S(q.y), S(q.z));
+        }
+        case GB_BOX:
+            return mk<S>(b.p[0], b.p[1], b.p[2]);
+        case GB_SPHERE:
+            return mk<S>(S(NAN), S(NAN), S(NAN));
+        case GB_RECTANGLE:
+            return mk<S>(b.p[0], b.p[1], S(0.0));
+        default: // GB_SUPERQUADRIC
+            return zero3<S>();
     }
 }
 
@@ -561,9 +588,7 @@ GB_D GjkResult<S> gjk_jh(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
     const S rel_error      = k_loweps<S>();
     const S abs_error      = S(1.e-4) * rel_error;
 
-    V3<S> s0A, s0B;
-    support2<PAIRED>(A, zero3<S>(), B, zero3<S>(), s0A, s0B);
-    V3<S> v    = s0A - apply(b2a, s0B);
+    V3<S> v    = support_zero(A) - apply(b2a, support_zero(B));
     V3<S> w    = v;
     S     dist = norm(v);
     bool  run  = active && dist > k_higheps<S>();
@@ -652,6 +677,26 @@ GB_D unsigned sv_other(unsigned j, unsigned k)
     return k + (k >= j ? 1u : 0u);
 }
 
+// weights C / m: the strict mode divides as the reference does, the others
+// multiply by one reciprocal (a division is some 25 dependent instructions)
+template <int N, typename S>
+GB_D void sv_weights(const S C[N], S m, S l[N])
+{
+    if constexpr(std::is_same<S, dstrict>::value)
+    {
+#pragma unroll
+        for(int i = 0; i < N; ++i)
+            l[i] = C[i] / m;
+    }
+    else
+    {
+        const S r = S(1.0) / m;
+#pragma unroll
+        for(int i = 0; i < N; ++i)
+            l[i] = C[i] * r;
+    }
+}
+
 // s1d (GJK_AY.cpp:15-84) on the segment (A, B), in slot order: the used
 // vertices (bit 0: A, bit 1: B) and their weights
 template <typename S>
@@ -675,8 +720,11 @@ GB_D unsigned sv_edge(const V3<S>& A, const V3<S>& B, S& la, S& lb)
     const unsigned sc0 = sv_same_sign(neg_tI, C0), sc1 = sv_same_sign(neg_tI, C1);
     if(sc0 + sc1 == 2)
     {
-        la = C0 / neg_tI;
-        lb = C1 / neg_tI;
+        const S C[2] = {C0, C1};
+        S       l[2];
+        sv_weights<2>(C, neg_tI, l);
+        la = l[0];
+        lb = l[1];
         return 3u;
     }
     if(sc0)
@@ -728,9 +776,7 @@ GB_D unsigned sv_face(const V3<S> Y[3], S l[3])
         open |= (1u - sv_same_sign(mu_max, C[j])) << j;
     if(!open)
     {
-#pragma unroll
-        for(int j = 0; j < 3; ++j)
-            l[j] = C[j] / mu_max;
+        sv_weights<3>(C, mu_max, l);
         return 7u;
     }
     S        d    = S(100000.0);
@@ -780,11 +826,7 @@ GB_D unsigned sv_tetrahedron(const V3<S> y[4], S lambdas[4])
     for(unsigned i = 0; i < 4; ++i)
         open |= (1u - sv_same_sign(dM, C[i])) << i;
     if(!open)
-    {
-#pragma unroll
-        for(int i = 0; i < 4; ++i)
-            lambdas[i] = C[i] / dM;
-    }
+        sv_weights<4>(C, dM, lambdas);
     return open;
 }
 
@@ -924,9 +966,7 @@ GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
     bool    momentum       = NESTEROV;
     const S rel_error      = k_loweps<S>();
     const S abs_error      = S(1.e-4) * rel_error;
-    V3<S>   s0A, s0B;
-    support2<PAIRED>(A, zero3<S>(), B, zero3<S>(), s0A, s0B);
-    V3<S>   v = s0A - apply(b2a, s0B);
+    V3<S>   v = support_zero(A) - apply(b2a, support_zero(B));
     V3<S>   w = v, d = v, s_prev = v;
     S       dist = norm(v);
     bool    run  = active && dist > k_higheps<S>();

@@ -611,8 +611,11 @@ GB_D void walk_rows(uint32_t s, uint32_t t0, uint32_t t1, const double4* __restr
     {
         const bool h0 = k < len && !pretest_rejects(a32, pos32[t0 + k]);
         const bool h1 = k + 1 < len && !pretest_rejects(a32, pos32[t0 + k + 1]);
-        push_hit(q, n, h0, s, t0 + k);
-        push_hit(q, n, h1, s, t0 + k + 1);
+        if(__any_sync(0xffffffffu, h0 || h1))
+        {
+            push_hit(q, n, h0, s, t0 + k);
+            push_hit(q, n, h1, s, t0 + k + 1);
+        }
         take_hits<STRICT>(q, n, k + 2 >= rounds, pos, record);
     }
 }
@@ -1404,8 +1407,7 @@ GB_D bool gjk_first_iteration_separates(const Body<float>& A, const Body<float>&
     const M3<float> RAt = transpose(RA);
     b2a.R               = mul(RAt, RB);
     b2a.o               = mul(RAt, d);
-    const V3<float> s0A = support(A, zero3<float>()), s0B = support(B, zero3<float>());
-    const V3<float> v    = s0A - apply(b2a, s0B);
+    const V3<float> v    = support_zero(A) - apply(b2a, support_zero(B));
     const float     dist = norm(v);
     const V3<float> pa = support_first(A, -v), qb = support_first(B, mul_t(b2a.R, v));
     const V3<float> w  = pa - apply(b2a, qb);
@@ -1527,7 +1529,7 @@ GB_D bool gjk_fp32_separates(const Body<float>& A, const Body<float>& B, const M
     b2a.o               = mul(RAt, d);
     const float ct      = A.crust + B.crust;
     const float margin  = 1e-4f * s + 1e-9f;
-    V3<float>   y0 = support(A, zero3<float>()) - apply(b2a, support(B, zero3<float>()));
+    V3<float>   y0 = support_zero(A) - apply(b2a, support_zero(B));
     V3<float>   y1 = y0, y2 = y0;
     int         n  = 1;
     V3<float>   v  = y0;
