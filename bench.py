@@ -819,9 +819,9 @@ LIMITER = {"integration": "issue and memory latency: 40% warps active (64 regist
            "broad_phase": "launch and tail latency of short dependent passes (hash 10 us, "
                           "scan, scatter 9 us, rank 20 us at 600k grains); 73 B per particle "
                           "read from DRAM",
-           "pair_count": "memory latency of the neighbour walk on the finer grid: 17 "
-                         "long-scoreboard stalls per issue at 46% warps active",
-           "narrow": "FP32 issue in the cull (42% issue slots, 24 of 32 lanes, 96 registers) "
+           "pair_count": "memory latency of the neighbour walk on the finer grid: 16 "
+                         "long-scoreboard stalls per issue at 59% warps active",
+           "narrow": "FP32 issue in the cull (42% issue slots, 30 of 32 lanes, 96 registers) "
                      "and FP64 GJK chains at 10-15% warps active (220 registers, 168 in "
                      "its three-block form for long queues)"}
 

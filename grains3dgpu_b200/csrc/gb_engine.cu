@@ -1354,8 +1354,26 @@ int run_detect(gb_ctx* c, int phases)
             // 0.441 ms; 200k polyhedra: 0.199 -> 0.206 ms).  Both forms are
             // launched; the queue length, on the device, picks the one that
             // works.
+            if constexpr(!JH)
+                if(!c->poly_bodies)
+                {
+                    // The signed-volume GJKs: a queue that four lanes per pair
+                    // take in one round runs so (a tetrahedron's faces side by
+                    // side), a longer one two lanes per pair, as above (20 steps
+                    // of the 2k column 3734 -> 3617 us, 10 of the 10k column in
+                    // FP64 2171 -> 2062 us).  Not with polyhedra, whose supports
+                    // are the larger part: the second launch cost 20 steps of
+                    // the 100k polyhedra 3846 -> 3908 us.
+                    constexpr int  LONG  = is_mixed<S>() ? 3 : 1;
+                    const uint32_t split = (uint32_t)(
+                        one_wave((const void*)k_narrow_gjk<S, VAR | kGjkQuad>, 128) * 128 / 4);
+                    GB_TRY(launch_gjk(k_narrow_gjk<S, VAR | kGjkQuad>, 0u, split));
+                    GB_TRY(launch_gjk(k_narrow_gjk<S, VAR, LONG>, split, UINT32_MAX));
+                    c->launches += 4;
+                    return GB_OK;
+                }
             uint32_t split = UINT32_MAX;
-            if constexpr(is_mixed<S>())
+            if constexpr(is_mixed<S>() && JH)
                 if(!c->poly_bodies)
                 {
                     split = (uint32_t)(one_wave((const void*)k_narrow_gjk<S, VAR>, 128) * 128 / 2);

@@ -265,6 +265,16 @@ GB_D V3<S> support_first(const Body<S>& b, const V3<S>& v)
 // in parallel, and they exchange them by shuffles.  (A support is the longest
 // dependent chain of an iteration: ~2,000 cycles for an FP64 superquadric.)
 constexpr int kGjkPaired = 8;
+// ... on four lanes instead of two (signed-volume GJKs on a short queue, whose
+// time is that of the longest pair's chain of iterations): each lane of the
+// four takes one open face of a tetrahedron
+constexpr int kGjkQuad = 16;
+
+// the lanes that run a pair under a variant
+constexpr int gjk_lanes(int var)
+{
+    return var & kGjkPaired ? (var & kGjkQuad ? 4 : 2) : 1;
+}
 
 // A GJK's loop condition.  PAIRED: the whole warp (all 32 lanes call the
 // GJK, lanes without a pair with run = false) goes round until its last pair
@@ -304,6 +314,7 @@ GB_D void support2(const Body<S>& A, const V3<S>& va, const Body<S>& B, const V3
 {
     if constexpr(PAIRED)
     {
+        // (four lanes are two such pairs with the same data)
         const unsigned lane   = threadIdx.x & 31u;
         const unsigned even   = lane & ~1u;
         const unsigned mask   = 3u << even;
@@ -661,7 +672,8 @@ GB_D unsigned sv_same_sign(S a, S b)
 
 // The sub-algorithm below keeps the simplex in registers: slots, faces and
 // edges are picked by selects on their index, since an indexed local array
-// costs a round trip to memory per access.
+// costs a round trip to memory per access (with the shared faces, ten steps of
+// the 10k column FP64 3313 -> 2545 us).
 
 // vertex i (0..3) of y
 template <typename S>
@@ -831,11 +843,12 @@ GB_D unsigned sv_tetrahedron(const V3<S> y[4], S lambdas[4])
 }
 
 // sv_subalgorithm (GJK_AY.cpp:340-368): new simplex, weights and closest
-// point.  PAIRED (kGjkPaired): the two lanes of a pair share a tetrahedron's
-// open faces, the even lane the first and third, the odd one the second and
-// fourth, and agree on the nearest (the first one on ties, as one lane going
-// through all of them finds it); a triangle is one face, which both evaluate.
-template <bool PAIRED, typename S>
+// point.  LANES (gjk_lanes): two lanes share a tetrahedron's open faces, the
+// even lane the first and third, the odd one the second and fourth; four lanes
+// take one each; they agree on the nearest (the first one on ties, as one lane
+// going through all of them finds it).  A triangle is one face, which all
+// evaluate.
+template <int LANES, typename S>
 GB_D V3<S> sv_subalgorithm(const V3<S> y[4], unsigned& bits, S lambdas[4])
 {
     const unsigned num_used = __popc(bits);
@@ -862,13 +875,17 @@ GB_D V3<S> sv_subalgorithm(const V3<S> y[4], unsigned& bits, S lambdas[4])
         unsigned   open     = triangle ? 15u ^ bits : sv_tetrahedron(y, lambdas);
         if(open)
         {
-            const bool share = PAIRED && !triangle;
+            const bool share = LANES > 1 && !triangle;
             if(share) // this lane's faces
             {
                 const unsigned first = open & (0u - open), rest = open ^ first;
                 const unsigned second = rest & (0u - rest), rest2 = rest ^ second;
                 const unsigned third  = rest2 & (0u - rest2);
-                open = threadIdx.x & 1u ? second | (rest2 ^ third) : first | third;
+                if constexpr(LANES == 4)
+                    open = threadIdx.x & 2u ? (threadIdx.x & 1u ? rest2 ^ third : third)
+                                            : (threadIdx.x & 1u ? second : first);
+                else
+                    open = threadIdx.x & 1u ? second | (rest2 ^ third) : first | third;
             }
             S        d    = S(100000.0);
             unsigned used = 0, best = 4;
@@ -898,20 +915,26 @@ GB_D V3<S> sv_subalgorithm(const V3<S> y[4], unsigned& bits, S lambdas[4])
             }
             if(share)
             {
-                const unsigned lane = threadIdx.x & 31u, peer = lane ^ 1u;
-                const unsigned mask = 3u << (lane & ~1u);
-                const S        dp   = lane_shfl(mask, d, peer);
-                const unsigned bp   = __shfl_sync(mask, best, peer);
-                const unsigned up   = __shfl_sync(mask, used, peer);
-                const bool     theirs = dp < d || (dp == d && bp < best);
+                const unsigned lane = threadIdx.x & 31u;
+                const unsigned mask = ((1u << LANES) - 1u) << (lane & ~(LANES - 1u));
 #pragma unroll
-                for(int k = 0; k < 3; ++k)
+                for(unsigned o = 1; o < (unsigned)LANES; o <<= 1)
                 {
-                    const S lp = lane_shfl(mask, l[k], peer);
-                    l[k]       = theirs ? lp : l[k];
+                    const unsigned peer   = lane ^ o;
+                    const S        dp     = lane_shfl(mask, d, peer);
+                    const unsigned bp     = __shfl_sync(mask, best, peer);
+                    const unsigned up     = __shfl_sync(mask, used, peer);
+                    const bool     theirs = dp < d || (dp == d && bp < best);
+#pragma unroll
+                    for(int k = 0; k < 3; ++k)
+                    {
+                        const S lp = lane_shfl(mask, l[k], peer);
+                        l[k]       = theirs ? lp : l[k];
+                    }
+                    d    = theirs ? dp : d;
+                    best = theirs ? bp : best;
+                    used = theirs ? up : used;
                 }
-                best = theirs ? bp : best;
-                used = theirs ? up : used;
             }
             bits = 0;
             if(best < 4)
@@ -952,10 +975,11 @@ GB_D bool sv_degenerate(unsigned bits, const V3<S> y[4], const V3<S>& w)
 //   y_k = delta_k x_k + (1 - delta_k) s_{k-1},   delta_k = (k + 1)/(k + 3),
 //   d_k = delta_k d_{k-1}/|d_{k-1}| + (1 - delta_k) y_k/|y_k|.
 // Without NESTEROV it is computeClosestPoints_GJK_AY (GJK_AY.cpp:392-469).
-template <typename S, bool NESTEROV, bool PAIRED = false>
+template <typename S, bool NESTEROV, int LANES = 1>
 GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
                          bool active = true)
 {
+    constexpr bool PAIRED = LANES > 1;
     unsigned bits = 0, last = 0;
     V3<S>    p[4], q[4], y[4];
     S        lambdas[4] = {S(0.0), S(0.0), S(0.0), S(0.0)};
@@ -1020,7 +1044,7 @@ GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
         q[last] = qn;
         bits |= 1u << last;
         ++num_iterations;
-        v    = sv_subalgorithm<PAIRED>(y, bits, lambdas);
+        v    = sv_subalgorithm<LANES>(y, bits, lambdas);
         dist = norm(v);
         s_prev = w;
         run    = bits < 15 && dist > k_higheps<S>() && num_iterations < 1000;
@@ -1046,14 +1070,14 @@ GB_D GjkResult<S> gjk_sv(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a,
 template <int VAR, typename S>
 GB_D GjkResult<S> gjk(const Body<S>& A, const Body<S>& B, const Tr<S>& b2a, bool active)
 {
-    constexpr bool PAIRED = (VAR & kGjkPaired) != 0;
-    constexpr int  KIND   = VAR & ~kGjkPaired;
+    constexpr int LANES = gjk_lanes(VAR);
+    constexpr int KIND  = VAR & ~(kGjkPaired | kGjkQuad);
     if constexpr(KIND == GB_GJK_SV)
-        return gjk_sv<S, false, PAIRED>(A, B, b2a, active);
+        return gjk_sv<S, false, LANES>(A, B, b2a, active);
     else if constexpr(KIND == GB_GJK_NESTEROV)
-        return gjk_sv<S, true, PAIRED>(A, B, b2a, active);
+        return gjk_sv<S, true, LANES>(A, B, b2a, active);
     else
-        return gjk_jh<S, PAIRED>(A, B, b2a, active);
+        return gjk_jh<S, (LANES > 1)>(A, B, b2a, active);
 }
 
 } // namespace gb

@@ -539,13 +539,15 @@ GB_D void neighbour_row(const uint32_t* __restrict__ cstart, uint32_t nx, uint32
 //
 // The rows are walked by threads of their own because the walk is a chain of
 // dependent loads (row bounds, then candidates): one thread per particle
-// waited through five chains in turn, and a small packing left the chip idle.
+// waited through five chains in turn, and a small packing left the chip idle
+// (12k spheres 32 -> 14 us a launch).
 //
 // The FP32 test passes one candidate in some 5 to 15, so in nearly every round
 // a few lanes of a warp have a hit; tested and recorded where they are found,
 // the FP64 test and the two atomics ran in nearly every round for those few
 // lanes and were most of the instructions.  The hits of a warp are queued in
-// shared memory instead and taken 32 at a time.
+// shared memory instead and taken 32 at a time (1M bed: fine-grid count 252 ->
+// 164 us, large grains 162 -> 67 us; 1M spheres' count 112 -> 90 us).
 
 // Candidate v (a sorted position) of particle id u: its slot and the count.
 GB_D void record_candidate(uint32_t id_u, uint32_t v, uint32_t* __restrict__ pcount,
@@ -993,7 +995,7 @@ GB_D void write_records(uint32_t a, const State<store_t<S>>& st, const Tables<S>
 // have consecutive ids and so nearly consecutive records: their sorted slots
 // are staged in shared memory and written out together, consecutive records
 // by consecutive lanes, where each lane writing its own few records cost a
-// partial sector per lane and array.
+// partial sector per lane and array (1M bed 114 -> 74 us a launch).
 template <typename S>
 __global__ void __launch_bounds__(kBlock)
     k_pair_fill(int n, const uint32_t* __restrict__ sids, const uint32_t* __restrict__ sorted_of,
@@ -1677,8 +1679,8 @@ GB_D void narrow_pair(int64_t p, uint32_t a, uint32_t b, const State<store_t<S>>
         else
             ci = closest_points<VAR>(A, B, RA, RB, oA, oB, d, &iters, active);
     }
-    // a lane pair (kGjkPaired) holds the same results: its even lane stores them
-    if((VAR & kGjkPaired) && (!active || (threadIdx.x & 1u)))
+    // the lanes of a pair hold the same results: the first one stores them
+    if((VAR & kGjkPaired) && (!active || (threadIdx.x & (gjk_lanes(VAR) - 1))))
         return;
     if(ci.overlap < S(0.0))
         pair_contact<S>(p, a, b, load_law<S>(tb.law, tb.shape[ra].material, tb.shape[rb].material),
@@ -1710,7 +1712,7 @@ GB_D void for_each_pair(int64_t npairs, F&& f)
 }
 
 // The same for passes that whole warps run together: f(p, valid) on every lane
-// of the warp, `step` (1 or 2) lanes per pair, lanes without a pair with
+// of the warp, STEP (1, 2 or 4) lanes per pair, lanes without a pair with
 // valid = false and a p that may be read (npairs > 0).
 template <int STEP, typename F>
 GB_D void for_each_pair_converged(int64_t npairs, F&& f)
@@ -1731,7 +1733,9 @@ GB_D void for_each_pair_converged(int64_t npairs, F&& f)
 // The narrow phase of a run whose bodies are all spheres: every record's
 // closed form and law in one pass, one thread per record, from the sphere
 // records of the fill pass (two to three sectors a particle, where the
-// structure-of-arrays state costs a sector per component).
+// structure-of-arrays state costs a sector per component).  Issue-bound on the
+// FP64 closed form (48% of issue slots); a launch, against the general kernel
+// on the state arrays: 1M spheres mixed 254 -> 160 us, 400k FP64 246 -> 91 us.
 template <typename S>
 __global__ void __launch_bounds__(kBlock)
     k_narrow_spheres(const uint32_t* __restrict__ total, const int* __restrict__ flags,
@@ -1875,7 +1879,11 @@ GB_D bool warp_pop(const WarpQueue& q, unsigned& n, uint32_t& p, uint32_t& a, ui
 // record p (k_narrow_gjk32).  Decisions are certified (obb_apart,
 // gjk_first_iteration_separates), so every mode, the bit-exact one included,
 // keeps the contacts of its own FP64 tests, which the last pass repeats for
-// each record it solves.
+// each record it solves.  Bound by FP32 issue and the latency of the records
+// (42% of issue slots at five blocks per SM; six gave the 1M bed 1% and cost
+// the 100k polyhedra 2%).  A launch, against a thread per ordered record in
+// the mode's own precision: 1M bed mixed 398 -> 176 us, 130k bed FP64 242 ->
+// 30 us, 400k drum 334 -> 107 us, 100k polyhedra 149 -> 60 us.
 template <typename S, bool JH_RULE, bool SPHERES>
 __global__ void __launch_bounds__(128, 5)
     k_narrow(const uint32_t* __restrict__ total, const int* __restrict__ flags,
@@ -1973,7 +1981,11 @@ __global__ void __launch_bounds__(128, 5)
 // The FP32 GJK stage over the cull's queue: a pair that gjk_fp32_separates
 // decides has no contact (its certificate, a lower bound on the distance,
 // holds for every GJK variant and for both records); of every other pair both
-// records go to the FP64 GJK's queue.
+// records go to the FP64 GJK's queue.  Bound by issue with 5 to 12 of 32 lanes
+// active (lanes of a warp need different numbers of iterations); a launch on
+// the 1M bed 210 us for each record on its own, 112 us now.  Four blocks per
+// SM: two cost the bed 4% and the polyhedra 15% of a step, five the 10k column
+// 3% (spills).
 template <typename St>
 __global__ void __launch_bounds__(128)
     k_narrow_gjk32(const uint32_t* __restrict__ gjk_count, const int* __restrict__ flags,
@@ -2032,7 +2044,7 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS)
     const int64_t nq     = *gjk_count;
     if(nq < (int64_t)min_queue || nq >= (int64_t)max_queue)
         return;
-    for_each_pair_converged<2>(nq, [&](int64_t q, bool valid) {
+    for_each_pair_converged<gjk_lanes(VAR | kGjkPaired)>(nq, [&](int64_t q, bool valid) {
         const uint32_t p = gjk_queue[q];
         narrow_pair<S, VAR | kGjkPaired>(p, pair_a[p], pair_b[p], st, tb, po, law_kind, has_kr,
                                          dt, counters, valid);

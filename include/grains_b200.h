@@ -70,7 +70,8 @@ extern "C" {
 #define GB_MAX_POLY_VERTICES 64
 
 /* ---- run modes -------------------------------------------------------------- */
-#define GB_FP64 0        /* every kernel in double precision, FMA contraction on  */
+#define GB_FP64 0        /* results in double precision, FMA contraction on (pairs that
+                            certified FP32 bounds separate are not solved, in any mode) */
 #define GB_MIXED 1       /* FP32 bulk; FP64 positions and candidate tests, FP64 GJK */
 #define GB_FP64_STRICT 2 /* FP64 in the reference's IEEE operation order (no FMA
                             contraction): the parity mode                          */
@@ -175,8 +176,8 @@ typedef struct gb_stats {
     int64_t candidate_pairs;  /* ordered pairs passing the bounding-sphere test */
     int64_t contacts;         /* ordered particle pairs with overlap < 0         */
     int64_t obstacle_contacts;
-    int64_t gjk_calls;        /* particle pairs past the bounding tests and GJK's first
-                                 iteration (queued for the GJK pass)           */
+    int64_t gjk_calls;        /* particle pairs (both orders counted) that the bounding tests
+                                 and GJK's first iteration leave open          */
     int64_t gjk_iterations;   /* summed over the steps of the last gb_step call */
     int32_t status_flags; /* bit i set: device-side error (1 << -GB_E_x)    */
     int32_t n_cells;
@@ -185,8 +186,8 @@ typedef struct gb_stats {
     double cell_size;
     double grid_max[3];      /* linked-cell max corner actually used */
     int64_t kernel_launches; /* kernels launched by this context so far */
-    int64_t gjk_fp64_calls;  /* particle pairs solved by the FP64 GJK (GB_MIXED: those its
-                                FP32 stage leaves open; otherwise gjk_calls) */
+    int64_t gjk_fp64_calls;  /* particle pairs solved by the FP64 GJK: those its FP32 stage
+                                leaves open */
     int64_t fine_grid_cells; /* cells of the finer candidate grid of a polydisperse packing
                                 (0: candidates from the linked cells alone) */
     int64_t obstacle_candidates; /* particle-obstacle records of the last detect (the obstacles
