@@ -1883,7 +1883,8 @@ GB_D bool warp_pop(const WarpQueue& q, unsigned& n, uint32_t& p, uint32_t& a, ui
 // (42% of issue slots at five blocks per SM; six gave the 1M bed 1% and cost
 // the 100k polyhedra 2%).  A launch, against a thread per ordered record in
 // the mode's own precision: 1M bed mixed 398 -> 176 us, 130k bed FP64 242 ->
-// 30 us, 400k drum 334 -> 107 us, 100k polyhedra 149 -> 60 us.
+// 30 us, 400k drum 334 -> 107 us, 100k polyhedra 149 -> 94 us (and less since
+// support(0) is not evaluated).
 template <typename S, bool JH_RULE, bool SPHERES>
 __global__ void __launch_bounds__(128, 5)
     k_narrow(const uint32_t* __restrict__ total, const int* __restrict__ flags,
