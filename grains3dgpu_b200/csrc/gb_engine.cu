@@ -387,10 +387,15 @@ Tables<S> tables_of(gb_ctx* c)
 
 bool crust_bounds(const gb_ctx* c) { return (c->cfg.flags & GB_FLAG_CRUST_BOUNDS) != 0; }
 
-// the bounding radius of rigid body i in the candidate test and the cell size
+// the bounding radius of a rigid body in the candidate test and the cell size
+double bound_radius(const gb_ctx* c, const gb_rigid_body_desc& rb, const gb_rigid_body_props& p)
+{
+    return p.circumscribed_radius + (crust_bounds(c) ? rb.crust_thickness : 0.0);
+}
+
 double bound_radius(const gb_ctx* c, int i)
 {
-    return c->props[i].circumscribed_radius + (crust_bounds(c) ? c->rbs[i].crust_thickness : 0.0);
+    return bound_radius(c, c->rbs[i], c->props[i]);
 }
 
 template <typename St>
@@ -1132,6 +1137,54 @@ int alloc_records(gb_ctx* c)
     return GB_OK;
 }
 
+// the bodies' device side: the cell arrays of their grid, their tables in
+// every precision that the run mode reads, and the records of their particles
+int upload_bodies(gb_ctx* c)
+{
+    dfree(c->d_cstart);
+    GB_TRY(dalloc(&c->d_cstart, (size_t)c->ncells + 1));
+    dfree(c->d_ccount);
+    c->ccount_zero = false;
+    GB_TRY(dalloc(&c->d_ccount, (size_t)c->ncells + 1));
+    if(c->d_shape64 && c->d_shape64 != c->d_shape)
+    {
+        cudaFree(c->d_shape64);
+        cudaFree(c->d_verts64);
+    }
+    if(c->prec != GB_MIXED)
+    {
+        cudaFree(c->d_shape32);
+        cudaFree(c->d_verts32);
+    }
+    c->d_shape32 = c->d_verts32 = nullptr;
+    c->d_shape64 = c->d_verts64 = nullptr;
+    const int st = upload_tables<double>(c);
+    c->d_shape64 = c->d_shape;
+    c->d_verts64 = c->d_verts;
+    GB_TRY(st);
+    if(c->prec == GB_MIXED)
+    {
+        c->d_shape = c->d_verts = nullptr; // keep the FP64 copies, add FP32 ones
+        const int st32          = upload_tables<float>(c);
+        c->d_shape32            = c->d_shape;
+        c->d_verts32            = c->d_verts;
+        GB_TRY(st32);
+    }
+    else if(!c->all_spheres)
+    {
+        // the FP64 modes' FP32 copies, rounded on the device
+        const int nv = std::max((int)(c->verts.size() / 3), 1);
+        GB_TRY(dalloc((RBShape<float>**)&c->d_shape32, c->nrb));
+        GB_TRY(dalloc((Vert<float>**)&c->d_verts32, nv));
+        k_tables_to_float<<<blocks(std::max(c->nrb, nv), kBlock), kBlock>>>(
+            c->nrb, (const RBShape<double>*)c->d_shape, (RBShape<float>*)c->d_shape32, nv,
+            (const Vert<double>*)c->d_verts, (Vert<float>*)c->d_verts32);
+        GB_CK(cudaGetLastError());
+        GB_CK(cudaStreamSynchronize(0));
+    }
+    return c->prec == GB_MIXED ? alloc_records<float>(c) : alloc_records<double>(c);
+}
+
 // candidate pairs (particles, then obstacles): count -> scan -> fill, with no
 // host round trip: the total stays on the device (off[n]); a total beyond the
 // capacity aborts the step (kFlagCapacity) and the host replays it larger
@@ -1852,21 +1905,19 @@ int gb_set_rigid_bodies(gb_ctx* c, const gb_rigid_body_desc* rbs, const double* 
 {
     if(!c || !rbs || n_vertices < 0 || (n_vertices && !vertices))
         return GB_E_INVALID_ARG;
-    c->rbs.assign(rbs, rbs + c->nrb);
-    c->fine_planned = false;
-    c->cobs_valid   = false; // the cell size may change
-    c->verts.assign(vertices, vertices + 3 * n_vertices);
-    c->props.resize(c->nrb);
-    double rmax = 0.0;
-    c->poly_bodies  = false;
-    c->all_spheres  = true;
-    c->some_spheres = false;
+    // Everything that the table decides is worked out and checked here first:
+    // a refused table leaves the context with the bodies that it had.
+    std::vector<gb_rigid_body_props> props(c->nrb);
+    double rmax         = 0.0;
+    bool   poly_bodies  = false;
+    bool   all_spheres  = true;
+    bool   some_spheres = false;
     for(int i = 0; i < c->nrb; ++i)
     {
         const gb_convex& cv = rbs[i].convex;
-        c->poly_bodies  = c->poly_bodies || cv.type == GB_POLYHEDRON;
-        c->all_spheres  = c->all_spheres && cv.type == GB_SPHERE;
-        c->some_spheres = c->some_spheres || cv.type == GB_SPHERE;
+        poly_bodies  = poly_bodies || cv.type == GB_POLYHEDRON;
+        all_spheres  = all_spheres && cv.type == GB_SPHERE;
+        some_spheres = some_spheres || cv.type == GB_SPHERE;
         if(cv.type == GB_POLYHEDRON
            && (cv.first_vertex < 0 || cv.first_vertex + cv.n_vertices > n_vertices))
             return GB_E_INVALID_ARG;
@@ -1874,75 +1925,57 @@ int gb_set_rigid_bodies(gb_ctx* c, const gb_rigid_body_desc* rbs, const double* 
             return GB_E_UNSUPPORTED;
         if(rbs[i].material < 0 || rbs[i].material >= c->nmat)
             return GB_E_INVALID_ARG;
-        GB_TRY(gb_rigid_body_properties(&rbs[i], vertices, &c->props[i]));
-        rmax = std::max(rmax, bound_radius(c, i)); // Grains.cpp:226-231
+        GB_TRY(gb_rigid_body_properties(&rbs[i], vertices, &props[i]));
+        rmax = std::max(rmax, bound_radius(c, rbs[i], props[i])); // Grains.cpp:226-231
     }
     // linked cell: cell = factor * 2 * max circumscribed radius (Grains.cpp:233-246)
     double coeff = c->cfg.cell_size_factor;
     if(coeff < 1.0)
         coeff = 1.0;
-    c->cell = coeff * 2.0 * rmax;
-    c->rmax = rmax;
+    const double cell = coeff * 2.0 * rmax;
+    double       lc_max[3];
+    uint32_t     dims[3];
     for(int k = 0; k < 3; ++k)
     {
-        c->lc_max[k] = c->cfg.max_coordinate[k] + (c->cfg.pad_grid ? c->cell : 0.0);
-        double t     = 1.e-10; // LinkedCell.cpp:23-28
-        t += c->lc_max[k] - c->cfg.origin[k];
-        t /= c->cell;
+        lc_max[k] = c->cfg.max_coordinate[k] + (c->cfg.pad_grid ? cell : 0.0);
+        double t  = 1.e-10; // LinkedCell.cpp:23-28
+        t += lc_max[k] - c->cfg.origin[k];
+        t /= cell;
         if(!(t >= 1.0) || t > 4.0e9)
             return GB_E_INVALID_ARG;
-        c->dims[k] = (uint32_t)t;
+        dims[k] = (uint32_t)t;
     }
-    const uint64_t nc = (uint64_t)c->dims[0] * c->dims[1] * c->dims[2];
+    const uint64_t nc = (uint64_t)dims[0] * dims[1] * dims[2];
     if(nc == 0 || nc > kMaxCells)
         return GB_E_INVALID_ARG;
+    // From here only the device can fail, and then the context has no bodies
+    // until a later call gives it some.
+    c->rb_set       = false;
+    c->rbs.assign(rbs, rbs + c->nrb);
+    c->verts.assign(vertices, vertices + 3 * n_vertices);
+    c->props        = std::move(props);
+    c->poly_bodies  = poly_bodies;
+    c->all_spheres  = all_spheres;
+    c->some_spheres = some_spheres;
+    c->fine_planned = false;
+    c->cobs_valid   = false; // the cell size may change
+    c->cell         = cell;
+    c->rmax         = rmax;
+    for(int k = 0; k < 3; ++k)
+    {
+        c->lc_max[k] = lc_max[k];
+        c->dims[k]   = dims[k];
+    }
     c->ncells   = (uint32_t)nc;
     c->key_bits = 0;
     while(c->key_bits < 32 && (1ull << c->key_bits) < nc)
         ++c->key_bits;
-    dfree(c->d_cstart);
-    GB_TRY(dalloc(&c->d_cstart, (size_t)nc + 1));
-    dfree(c->d_ccount);
-    c->ccount_zero = false;
-    GB_TRY(dalloc(&c->d_ccount, (size_t)nc + 1));
-    if(c->d_shape64 && c->d_shape64 != c->d_shape)
+    const int st = upload_bodies(c);
+    if(st != GB_OK)
     {
-        cudaFree(c->d_shape64);
-        cudaFree(c->d_verts64);
-    }
-    if(c->prec != GB_MIXED)
-    {
-        cudaFree(c->d_shape32);
-        cudaFree(c->d_verts32);
-    }
-    c->d_shape32 = c->d_verts32 = nullptr;
-    c->d_shape64 = c->d_verts64 = nullptr;
-    int st       = upload_tables<double>(c);
-    c->d_shape64 = c->d_shape;
-    c->d_verts64 = c->d_verts;
-    if(st == GB_OK && c->prec == GB_MIXED)
-    {
-        c->d_shape = c->d_verts = nullptr; // keep the FP64 copies, add FP32 ones
-        st                      = upload_tables<float>(c);
-        c->d_shape32            = c->d_shape;
-        c->d_verts32            = c->d_verts;
-    }
-    else if(st == GB_OK && !c->all_spheres)
-    {
-        // the FP64 modes' FP32 copies, rounded on the device
-        const int nv = std::max((int)(c->verts.size() / 3), 1);
-        GB_TRY(dalloc((RBShape<float>**)&c->d_shape32, c->nrb));
-        GB_TRY(dalloc((Vert<float>**)&c->d_verts32, nv));
-        k_tables_to_float<<<blocks(std::max(c->nrb, nv), kBlock), kBlock>>>(
-            c->nrb, (const RBShape<double>*)c->d_shape, (RBShape<float>*)c->d_shape32, nv,
-            (const Vert<double>*)c->d_verts, (Vert<float>*)c->d_verts32);
-        GB_CK(cudaGetLastError());
-        GB_CK(cudaStreamSynchronize(0));
-    }
-    if(st == GB_OK)
-        st = c->prec == GB_MIXED ? alloc_records<float>(c) : alloc_records<double>(c);
-    if(st)
+        c->links_valid = c->detect_valid = false; // the cell arrays may be gone
         return st;
+    }
     c->rb_set     = true;
     c->mask_valid = false;
     return GB_OK;

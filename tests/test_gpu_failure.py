@@ -16,6 +16,8 @@ import pytest
 
 from grains3dgpu_b200 import abi, scenes
 
+from test_gpu_cull import packing
+
 pytestmark = pytest.mark.gpu
 
 
@@ -64,3 +66,55 @@ def test_out_of_domain_is_reported(gb):
     s.set_transforms(scene.transforms)
     assert gb.step(s.ctx, 1) == abi.GB_OK
     s.close()
+
+
+def _refused_tables(rbs, nmat):
+    """Tables of as many bodies that gb_set_rigid_bodies refuses, each for a
+    body after ones of other types than the scene's, or for its grid."""
+    n = len(rbs)
+
+    def table(kinds, last=None, **fields):
+        t = rbs.copy()
+        t["type"] = kinds
+        t["p"] = 1e-3
+        t["n_vertices"] = t["first_vertex"] = 0
+        if last is not None:
+            t["type"][-1] = last
+        for k, v in fields.items():
+            t[k][-1] = v
+        return t
+
+    tiny = table(abi.GB_SPHERE)
+    tiny["p"] = 1e-13  # more linked cells than the grid can have
+    for first in (abi.GB_SPHERE, abi.GB_BOX):
+        yield table(first, material=nmat), abi.GB_E_INVALID_ARG
+        yield table(first, last=abi.GB_CONE), abi.GB_E_UNSUPPORTED
+        yield (table(first, last=abi.GB_POLYHEDRON, n_vertices=8, first_vertex=10 ** 6),
+               abi.GB_E_INVALID_ARG)
+    assert n > 1
+    yield tiny, abi.GB_E_INVALID_ARG
+
+
+@pytest.mark.parametrize("precision", [abi.GB_FP64_STRICT, abi.GB_MIXED])
+@pytest.mark.parametrize("bodies", [(0, 1), (2, 3), (0, 2)])
+def test_refused_bodies_leave_the_context_as_it_was(gb, bodies, precision):
+    """A refused gb_set_rigid_bodies changes nothing: the steps after it are
+    those of a context that never saw the call, whatever shapes the refused
+    table held."""
+    scene = packing(150, bodies)
+    seen = scenes.System(gb, scene, precision=precision)
+    twin = scenes.System(gb, scene, precision=precision)
+    for s in (seen, twin):
+        s.step(2)
+    verts = np.ascontiguousarray(scene.vertices, dtype=np.float64)
+    for rbs, status in _refused_tables(scene.rbs, scene.config["n_materials"]):
+        assert gb.set_rigid_bodies(seen.ctx, rbs.ctypes.data_as(abi.C.POINTER(abi.RigidBodyDesc)),
+                                   abi.dptr(verts) if verts.size else None,
+                                   verts.shape[0]) == status
+        assert bytes(seen.rb_props(1)) == bytes(twin.rb_props(1))
+        for s in (seen, twin):
+            s.step(2)
+        assert np.array_equal(seen.transforms(), twin.transforms())
+        assert np.array_equal(seen.velocities(), twin.velocities())
+        a, b = seen.stats(), twin.stats()
+        assert (a.cell_size, a.n_cells, a.contacts) == (b.cell_size, b.n_cells, b.contacts)
