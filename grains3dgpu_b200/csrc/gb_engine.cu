@@ -1993,10 +1993,13 @@ int gb_set_contact_models(gb_ctx* c, const gb_contact_model* table)
 {
     if(!c || !table)
         return GB_E_INVALID_ARG;
-    c->laws.assign(table, table + c->nmat * (c->nmat + 1) / 2);
-    for(auto& m : c->laws)
+    // a refused table leaves the context with the laws that it had
+    const std::vector<gb_contact_model> laws(table, table + c->nmat * (c->nmat + 1) / 2);
+    for(auto& m : laws)
         if(!(m.kn >= 0.0) || !(m.en > 0.0 && m.en <= 1.0))
             return GB_E_INVALID_ARG;
+    c->law_set = false;
+    c->laws    = laws;
     int st = c->prec == GB_MIXED ? upload_laws<float>(c) : upload_laws<double>(c);
     if(st)
         return st;
@@ -2008,9 +2011,8 @@ int gb_set_obstacles(gb_ctx* c, const gb_rigid_body_desc* obst, const double* tr
 {
     if(!c || (c->nob && (!obst || !transforms)))
         return GB_E_INVALID_ARG;
-    c->obs.assign(obst, obst + c->nob);
-    c->obs_tr.assign(transforms, transforms + 12 * (size_t)c->nob);
-    c->obs_props.resize(c->nob);
+    // refused obstacles leave the context with those that it had
+    std::vector<gb_rigid_body_props> props(c->nob);
     for(int i = 0; i < c->nob; ++i)
     {
         if(obst[i].convex.type == GB_POLYHEDRON || obst[i].convex.type == GB_CYLINDER
@@ -2020,8 +2022,12 @@ int gb_set_obstacles(gb_ctx* c, const gb_rigid_body_desc* obst, const double* tr
             return GB_E_INVALID_ARG;
         if(obst[i].material < 0 || obst[i].material >= c->nmat)
             return GB_E_INVALID_ARG;
-        GB_TRY(gb_rigid_body_properties(&obst[i], nullptr, &c->obs_props[i]));
+        GB_TRY(gb_rigid_body_properties(&obst[i], nullptr, &props[i]));
     }
+    c->obs_set = false;
+    c->obs.assign(obst, obst + c->nob);
+    c->obs_tr.assign(transforms, transforms + 12 * (size_t)c->nob);
+    c->obs_props = std::move(props);
     if(c->d_obs_shape64 && c->d_obs_shape64 != c->d_obs_shape)
         cudaFree(c->d_obs_shape64);
     c->d_obs_shape64 = nullptr;

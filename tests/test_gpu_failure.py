@@ -68,6 +68,10 @@ def test_out_of_domain_is_reported(gb):
     s.close()
 
 
+def _rb_pointer(rbs):
+    return rbs.ctypes.data_as(abi.C.POINTER(abi.RigidBodyDesc))
+
+
 def _refused_tables(rbs, nmat):
     """Tables of as many bodies that gb_set_rigid_bodies refuses, each for a
     body after ones of other types than the scene's, or for its grid."""
@@ -108,7 +112,7 @@ def test_refused_bodies_leave_the_context_as_it_was(gb, bodies, precision):
         s.step(2)
     verts = np.ascontiguousarray(scene.vertices, dtype=np.float64)
     for rbs, status in _refused_tables(scene.rbs, scene.config["n_materials"]):
-        assert gb.set_rigid_bodies(seen.ctx, rbs.ctypes.data_as(abi.C.POINTER(abi.RigidBodyDesc)),
+        assert gb.set_rigid_bodies(seen.ctx, _rb_pointer(rbs),
                                    abi.dptr(verts) if verts.size else None,
                                    verts.shape[0]) == status
         assert bytes(seen.rb_props(1)) == bytes(twin.rb_props(1))
@@ -118,3 +122,48 @@ def test_refused_bodies_leave_the_context_as_it_was(gb, bodies, precision):
         assert np.array_equal(seen.velocities(), twin.velocities())
         a, b = seen.stats(), twin.stats()
         assert (a.cell_size, a.n_cells, a.contacts) == (b.cell_size, b.n_cells, b.contacts)
+
+
+def test_refused_obstacles_leave_the_context_as_it_was(gb):
+    """After refused obstacles (shrunk pegs elsewhere, the last one of an
+    unknown material), bodies set again -- which makes the obstacle bins
+    anew -- meet the obstacles of a context that never saw the call."""
+    scene = scenes.peg_board()
+    seen, twin = (scenes.System(gb, scene, precision=abi.GB_FP64) for _ in range(2))
+    obs = np.ascontiguousarray(scene.obstacles).copy()
+    obs["p"] *= 0.1
+    obs["material"][-1] = scene.config["n_materials"]
+    tr = np.ascontiguousarray(scene.obstacle_transforms, dtype=np.float64) + 0.01
+    assert gb.set_obstacles(seen.ctx, _rb_pointer(obs), abi.dptr(tr)) == abi.GB_E_INVALID_ARG
+    rbs = np.ascontiguousarray(scene.rbs)
+    for s in (seen, twin):
+        assert gb.set_rigid_bodies(s.ctx, _rb_pointer(rbs), None, 0) == abi.GB_OK
+        s.step(2)
+    assert seen.stats().obstacle_contacts == twin.stats().obstacle_contacts > 100
+    assert np.array_equal(seen.transforms(), twin.transforms())
+
+
+def test_refused_contact_models_leave_the_context_as_it_was(gb):
+    """The adjoint reads the laws' host copy: after refused laws (other
+    stiffnesses, a negative one last) its gradients are those of a context
+    that never saw the call."""
+    import torch
+    scene = scenes.sphere_bed()
+    n, nl = scene.n, len(scene.contact_models)
+    adj = torch.ones((9, n), dtype=torch.float64, device="cuda")
+    out = []
+    for refused in (False, True):
+        s = scenes.System(gb, scene, precision=abi.GB_FP64)
+        if refused:
+            laws = [dict(m, kn=2.0 * m["kn"]) for m in scene.contact_models]
+            laws[-1]["kn"] = -1.0
+            assert gb.set_contact_models(s.ctx, abi.contact_model_array(laws)) \
+                == abi.GB_E_INVALID_ARG
+        prev = torch.empty_like(adj)
+        grad = torch.zeros(4 * nl, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        ptr = [abi.C.cast(abi.C.c_void_p(t.data_ptr()), abi._D) for t in (adj, prev, grad)]
+        assert gb.adjoint_step(s.ctx, *ptr) == abi.GB_OK
+        out.append((prev.cpu().numpy(), grad.cpu().numpy()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    assert np.abs(out[0][1]).max() > 0.0
