@@ -29,6 +29,7 @@ thread_local cudaError_t g_last_cuda = cudaSuccess;
         if(e_ != cudaSuccess)                  \
         {                                      \
             g_last_cuda = e_;                  \
+            (void)cudaGetLastError(); /* reported here, not by the next call */ \
             return e_ == cudaErrorMemoryAllocation ? GB_E_OUT_OF_MEMORY : GB_E_CUDA; \
         }                                      \
     } while(0)
@@ -252,7 +253,8 @@ struct gb_ctx
     uint8_t*  d_pc[2] = {nullptr, nullptr}; // contact flags, double-buffered with the list
     double*   d_info = nullptr;
     void*     d_xi[2] = {nullptr, nullptr}; // 3 * cap each
-    int64_t   cap = 0;
+    int64_t   cap = 0;      // pair capacity of the step's arrays
+    int64_t   list_cap = 0; // ... of the list (cap, or cap is 0: ensure_pairs)
     int64_t   cap_hint = 0; // capacity the next step allocates up front (grows after an overflow)
     int       cur = 0;
     int64_t   npairs = 0; // of the last detect (read back after it)
@@ -639,19 +641,20 @@ int alloc_state(gb_ctx* c)
     return GB_OK;
 }
 
-int ensure_pairs(gb_ctx* c, int64_t need)
+// The pair list in arrays of capacity ncap, its contents carried over as far
+// as both hold them (the next step's history, a loaded contact set; the
+// records' number is on the device, so the whole capacity).  Without memory
+// nothing changes.
+int resize_list(gb_ctx* c, int64_t ncap)
 {
-    if(need <= c->cap)
-        return GB_OK;
-    int64_t ncap = c->cap == 0 ? std::max<int64_t>(need, 1024)
-                               : std::max<int64_t>(need + need / 2, 1024);
-    const size_t ss = store_size(c->prec);
-    const bool   hist = c->cfg.contact_law == GB_LAW_HOOKE_HISTORY;
-    Arena     m;
-    char*     mem = nullptr;
-    uint32_t* npb[2] = {nullptr, nullptr};
-    void*     nxi[2] = {nullptr, nullptr};
-    uint8_t*  npc[2] = {nullptr, nullptr};
+    const size_t  ss   = store_size(c->prec);
+    const bool    hist = c->cfg.contact_law == GB_LAW_HOOKE_HISTORY;
+    const int64_t keep = std::min(ncap, c->list_cap);
+    Arena         m;
+    char*         mem = nullptr;
+    uint32_t*     npb[2] = {nullptr, nullptr};
+    void*         nxi[2] = {nullptr, nullptr};
+    uint8_t*      npc[2] = {nullptr, nullptr};
     for(int b = 0; b < 2; ++b)
     {
         m.add(&npb[b], ncap);
@@ -661,20 +664,24 @@ int ensure_pairs(gb_ctx* c, int64_t need)
             m.add(&npc[b], ncap);
     }
     GB_TRY(m.allocate(&mem));
-    // the previous step's history buffers survive the growth (its pair count
-    // is on the device: the whole old capacity)
-    const int prev = 1 - c->cur;
-    if(c->have_prev && c->cap > 0)
-    {
-        GB_CK(cudaMemcpy(npb[prev], c->d_pb[prev], c->cap * sizeof(uint32_t),
-                         cudaMemcpyDeviceToDevice));
-        if(hist)
-            GB_CK(cudaMemcpy(npc[prev], c->d_pc[prev], c->cap, cudaMemcpyDeviceToDevice));
-        if(hist)
-            for(int k = 0; k < 3; ++k)
-                GB_CK(cudaMemcpy((char*)nxi[prev] + k * ncap * ss,
-                                 (char*)c->d_xi[prev] + k * c->cap * ss, c->cap * ss,
+    auto carry_over = [&]() -> int {
+        for(int b = 0; b < 2; ++b)
+        {
+            GB_CK(cudaMemcpy(npb[b], c->d_pb[b], keep * sizeof(uint32_t),
+                             cudaMemcpyDeviceToDevice));
+            if(npc[b])
+                GB_CK(cudaMemcpy(npc[b], c->d_pc[b], keep, cudaMemcpyDeviceToDevice));
+            for(int k = 0; hist && k < 3; ++k)
+                GB_CK(cudaMemcpy((char*)nxi[b] + k * ncap * ss,
+                                 (char*)c->d_xi[b] + k * c->list_cap * ss, keep * ss,
                                  cudaMemcpyDeviceToDevice));
+        }
+        return GB_OK;
+    };
+    if(const int st = keep > 0 ? carry_over() : GB_OK)
+    {
+        cudaFree(mem);
+        return st;
     }
     for(int b = 0; b < 2; ++b)
     {
@@ -684,17 +691,49 @@ int ensure_pairs(gb_ctx* c, int64_t need)
     }
     dfree(c->mem_list);
     c->mem_list = mem;
-    dfree(c->mem_pairs);
-    Arena work;
-    work.add(&c->d_gjkq, 2 * ncap);
-    work.add(&c->d_obsq, ncap);
-    work.add(&c->d_pa, ncap);
-    work.add(&c->d_pf, 9 * ncap, ss);
-    if(c->cfg.flags & GB_FLAG_RECORD_CONTACT_INFO)
-        work.add(&c->d_info, 7 * ncap);
-    GB_TRY(work.allocate(&c->mem_pairs));
-    c->cap = ncap;
+    c->list_cap = ncap;
     return GB_OK;
+}
+
+// The other arrays of pair capacity, as many records as the list's, in place
+// of the old ones (freed first: they are the larger part, and hold nothing
+// between detects).  Without memory the context has none (cap 0).
+int resize_work(gb_ctx* c)
+{
+    dfree(c->mem_pairs);
+    c->d_gjkq = c->d_obsq = c->d_pa = nullptr;
+    c->d_pf   = nullptr;
+    c->d_info = nullptr;
+    c->cap    = 0;
+    Arena work;
+    work.add(&c->d_gjkq, 2 * c->list_cap);
+    work.add(&c->d_obsq, c->list_cap);
+    work.add(&c->d_pa, c->list_cap);
+    work.add(&c->d_pf, 9 * c->list_cap, store_size(c->prec));
+    if(c->cfg.flags & GB_FLAG_RECORD_CONTACT_INFO)
+        work.add(&c->d_info, 7 * c->list_cap);
+    GB_TRY(work.allocate(&c->mem_pairs));
+    c->cap = c->list_cap;
+    return GB_OK;
+}
+
+// Pair capacity for `need` records.  Growth that fails leaves the capacity
+// and the list as they were; the last detect's forces are gone by then.
+int ensure_pairs(gb_ctx* c, int64_t need)
+{
+    if(need <= c->cap)
+        return GB_OK;
+    const int64_t old = c->list_cap;
+    if(need > old)
+        GB_TRY(resize_list(c, std::max<int64_t>(old == 0 ? need : need + need / 2, 1024)));
+    const int st = resize_work(c);
+    if(st != GB_OK)
+    {
+        c->detect_valid = false;
+        if(old > 0 && resize_list(c, old) == GB_OK)
+            (void)resize_work(c);
+    }
+    return st;
 }
 
 // exclusive scan of n uint32 (in place allowed); *d_total (device) gets the sum
@@ -1639,7 +1678,17 @@ int run_steps(gb_ctx* c, int32_t n_steps, int phases, int32_t* result)
         for(int32_t k = done; k < n_steps; ++k)
         {
             snaps.push_back(snap(c));
-            GB_TRY(dispatch(c, [&](auto z) { return run_detect<decltype(z)>(c, phases); }));
+            const int st = dispatch(
+                c, [&](auto z) { return run_detect<decltype(z)>(c, phases); });
+            if(st != GB_OK)
+            {
+                // not launched whole (no memory for its pairs): the context
+                // is back before this step, with no valid detect
+                restore(c, snaps.back());
+                c->cap_hint    = c->cap > 0 ? c->cap : c->cap_hint;
+                c->links_valid = c->detect_valid = c->in_step = false;
+                return st;
+            }
             if(phases & PHASE_MOVE)
             {
                 // the first step adds to a torce left by separate calls, then resets it

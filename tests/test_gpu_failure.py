@@ -167,3 +167,77 @@ def test_refused_contact_models_leave_the_context_as_it_was(gb):
         out.append((prev.cpu().numpy(), grad.cpu().numpy()))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
     assert np.abs(out[0][1]).max() > 0.0
+
+
+@pytest.mark.parametrize("law,fails", [(abi.GB_LAW_HOOKE, "work"),
+                                       (abi.GB_LAW_HOOKE_HISTORY, "work"),
+                                       (abi.GB_LAW_HOOKE_HISTORY, "list")])
+def test_growth_without_memory_is_reported(gb, law, fails):
+    """A contact set too large for the device (a header that claims so; nothing
+    past it is read) makes the pair arrays' growth fail.  The call says so, no
+    array of the failed growth is read, and the steps after it, springs of
+    the history law included, are those of a context that never saw it."""
+    import torch
+    scene = packing(150, (0, 1))
+    kw = dict(precision=abi.GB_FP64_STRICT, contact_law=law,
+              flags=abi.GB_FLAG_RECORD_CONTACT_INFO)
+    seen, twin = (scenes.System(gb, scene, **kw) for _ in range(2))
+    for s in (seen, twin):
+        s.step(3)
+    before = seen.dump(abi.GB_DUMP_CONTACT_PAIRS)
+    # bytes per record of the list (58 with the springs) and of the other
+    # arrays (144 with the contact information), half as many records again
+    total = torch.cuda.get_device_properties(0).total_memory
+    pairs = int(1.25 * total / (1.5 * (58 if fails == "list" else 144)))
+    buf = torch.zeros(4096, dtype=torch.int64, device="cuda")
+    buf[0], buf[1] = scene.n, pairs
+    torch.cuda.synchronize()
+    assert gb.load_contacts(seen.ctx, buf.data_ptr()) == abi.GB_E_OUT_OF_MEMORY
+    if fails == "list":
+        assert np.array_equal(seen.dump(abi.GB_DUMP_CONTACT_PAIRS), before)
+    else:
+        count = abi.C.c_int64(0)
+        assert gb.debug_dump(seen.ctx, abi.GB_DUMP_CONTACT_PAIRS, None, 0,
+                             abi.C.byref(count)) == abi.GB_E_NOT_READY
+    for s in (seen, twin):
+        assert s.step(3) == abi.GB_OK
+    assert np.array_equal(seen.dump(abi.GB_DUMP_CONTACT_INFO), twin.dump(abi.GB_DUMP_CONTACT_INFO))
+    assert np.array_equal(seen.transforms(), twin.transforms())
+    assert np.array_equal(seen.velocities(), twin.velocities())
+
+
+def test_springs_survive_growth(gb):
+    """The pair arrays grow in a step whose history holds springs: most grains
+    are far apart at first and come into one packing afterwards, so that the
+    candidates pass the capacity while earlier contacts last.  The trajectory
+    is that of a context that never grew, and not that of one without the
+    springs."""
+    scene = packing(400, (0, 1))
+    dense = scene.transforms.copy()
+    top = scene.config["max_coordinate"][2]
+    scene.config["max_coordinate"] = (*scene.config["max_coordinate"][:2], 1.0)
+    tr = scene.obstacle_transforms
+    tr[np.isclose(tr[:, 11], top), 11] = 1.0
+    apart = dense.copy()
+    up = np.argsort(dense[:, 11], kind="stable")[100:]
+    apart[up, 11] = 0.03 + 3e-3 * np.arange(len(up))
+    scene.transforms = apart
+    ends = []
+    for capacity, history in ((1, True), (100_000, True), (100_000, False)):
+        s = scenes.System(gb, scene, precision=abi.GB_FP64_STRICT, pair_capacity=capacity,
+                          contact_law=abi.GB_LAW_HOOKE_HISTORY)
+        s.step(5)
+        assert 0 < s.stats().contacts <= s.stats().candidate_pairs < 1024
+        kin = s.velocities()
+        lower = s.transforms()
+        if not history:
+            s = scenes.System(gb, scene, precision=abi.GB_FP64_STRICT,
+                              contact_law=abi.GB_LAW_HOOKE_HISTORY)
+            s.set_velocities(kin)
+        lower[up] = dense[up]
+        s.set_transforms(lower)
+        s.step(3)
+        assert s.stats().candidate_pairs > 1024
+        ends.append((s.transforms(), s.velocities()))
+    assert all(np.array_equal(a, b) for a, b in zip(ends[0], ends[1]))
+    assert not np.array_equal(ends[1][1], ends[2][1])
