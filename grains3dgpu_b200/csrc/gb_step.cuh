@@ -1023,7 +1023,9 @@ __global__ void __launch_bounds__(kBlock)
         gjk_count[3 - ovf_phase] = 0;
         gjk_count[5 - ovf_phase] = 0;
     }
-    if(step_aborted(flags)) // the same for the whole warp
+    // (this pass sets the capacity flag itself, so the lanes of a warp may read
+    // it apart: one answer for all of them, who go on together from here)
+    if(__any_sync(0xffffffffu, step_aborted(flags)))
         return;
     const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     uint32_t       cp = a < n ? pcount[a] : 0u, k_obs = a < n && oc.n ? obs_count[a] : 0u;
