@@ -1414,12 +1414,13 @@ int run_detect(gb_ctx* c, int phases)
             constexpr int  VAR = decltype(var)::value;
             constexpr bool JH  = VAR == GB_GJK_JH;
             const auto*    pose = (const PoseRec<St>*)c->d_pose;
-            const uint32_t* off = c->d_off[c->cur];
+            const uint32_t* off       = c->d_off[c->cur];
+            const uint32_t* sorted_of = c->d_sorted_of;
             auto            cull = [&](auto kernel) -> int {
                 GB_CK(launch(c->pdl, kernel, one_wave((const void*)kernel, 128), 128, s, total,
                              (const int*)c->d_flags, (const uint32_t*)c->d_pa,
-                             (const uint32_t*)c->d_pb[c->cur], off, pose, st, tb, po, law, kr,
-                             S(c->cfg.dt), c->d_counters, c->d_gjkq, c->d_gjkn));
+                             (const uint32_t*)c->d_pb[c->cur], off, sorted_of, pose, st, tb, po, law,
+                             kr, S(c->cfg.dt), c->d_counters, c->d_gjkq, c->d_gjkn));
                 return GB_OK;
             };
             if(c->some_spheres)
@@ -1429,8 +1430,8 @@ int run_detect(gb_ctx* c, int phases)
             GB_CK(launch(c->pdl, k_narrow_gjk32<St>, one_wave((const void*)k_narrow_gjk32<St>, 128),
                          128, s, (const uint32_t*)c->d_gjkn, (const int*)c->d_flags,
                          (const uint32_t*)c->d_gjkq, (const uint32_t*)c->d_pa,
-                         (const uint32_t*)c->d_pb[c->cur], off, pose, tb.shape32, tb.verts32,
-                         c->d_gjkq + c->cap, c->d_gjkn + 1));
+                         (const uint32_t*)c->d_pb[c->cur], off, sorted_of, pose, tb.shape32,
+                         tb.verts32, c->d_gjkq + c->cap, c->d_gjkn + 1));
             const uint32_t* q64 = c->d_gjkq + c->cap;
             const uint32_t* n64 = c->d_gjkn + 1;
             auto launch_gjk = [&](auto kernel, uint32_t lo, uint32_t hi) -> int {

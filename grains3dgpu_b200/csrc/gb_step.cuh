@@ -1819,13 +1819,33 @@ GB_D V3<float> centre_difference(const Pose32& A, const Pose32& B)
 }
 
 // the record (b, a) of record (a, b): b's records hold the mirror of each of
-// a's (the candidate test is symmetric); kNoRecord, never expected, if not
-constexpr uint32_t kNoRecord = 0xffffffffu;
+// a's (the candidate test is symmetric); kNoRecord, never expected, if not.
+// They ascend in the partner's sorted position, obstacles after them (the fill
+// pass), so a long list is halved first: a large grain among small ones has
+// thousands of records, and each of its pairs looks through them (a detect of
+// 60,000 grains around one, mixed 25.2 -> 15.3 ms, of 1,350 0.48 -> 0.40 ms).
+// Where halving stops matters little (8, 32 and 128 records: the same within
+// 1%); lists of up to 32, all but a few in other packings, read no positions.
+constexpr uint32_t kNoRecord     = 0xffffffffu;
+constexpr uint32_t kMirrorLinear = 32; // records looked through one by one
 
 GB_D uint32_t mirror_record(const uint32_t* __restrict__ off, const uint32_t* __restrict__ pair_b,
-                            uint32_t a, uint32_t b)
+                            const uint32_t* __restrict__ sorted_of, uint32_t a, uint32_t b)
 {
-    for(uint32_t k = off[b], e = off[b + 1]; k < e; ++k)
+    uint32_t k = off[b], e = off[b + 1];
+    if(e - k > kMirrorLinear)
+    {
+        const uint32_t s = sorted_of[a];
+        while(e - k > kMirrorLinear)
+        {
+            const uint32_t m = k + (e - k) / 2, q = pair_b[m];
+            if(!(q & kObstacleBit) && sorted_of[q] <= s)
+                k = m;
+            else
+                e = m;
+        }
+    }
+    for(; k < e; ++k)
         if(pair_b[k] == a)
             return k;
     return kNoRecord;
@@ -1891,9 +1911,10 @@ template <typename S, bool JH_RULE, bool SPHERES>
 __global__ void __launch_bounds__(128, 5)
     k_narrow(const uint32_t* __restrict__ total, const int* __restrict__ flags,
              const uint32_t* __restrict__ pair_a, const uint32_t* __restrict__ pair_b,
-             const uint32_t* __restrict__ off, const PoseRec<store_t<S>>* __restrict__ pose,
-             State<store_t<S>> st, Tables<S> tb, PairOut<store_t<S>> po, int law_kind, int has_kr,
-             S dt, unsigned long long* __restrict__ counters, uint32_t* __restrict__ gjk_queue,
+             const uint32_t* __restrict__ off, const uint32_t* __restrict__ sorted_of,
+             const PoseRec<store_t<S>>* __restrict__ pose, State<store_t<S>> st, Tables<S> tb,
+             PairOut<store_t<S>> po, int law_kind, int has_kr, S dt,
+             unsigned long long* __restrict__ counters, uint32_t* __restrict__ gjk_queue,
              uint32_t* __restrict__ gjk_count)
 {
     grid_dep_sync();
@@ -1969,7 +1990,7 @@ __global__ void __launch_bounds__(128, 5)
                 uint32_t p = 0, a = 0, b = 0;
                 if(warp_pop(sphere, nsphere, p, a, b))
                 {
-                    const uint32_t pm = mirror_record(off, pair_b, a, b);
+                    const uint32_t pm = mirror_record(off, pair_b, sorted_of, a, b);
                     for(int k = 0; k < (pm == kNoRecord ? 1 : 2); ++k)
                         narrow_pair<S, GB_GJK_JH, true>(k ? pm : p, k ? b : a, k ? a : b, st, tb,
                                                         po, law_kind, has_kr, dt, counters);
@@ -1994,9 +2015,9 @@ __global__ void __launch_bounds__(128)
     k_narrow_gjk32(const uint32_t* __restrict__ gjk_count, const int* __restrict__ flags,
                    const uint32_t* __restrict__ gjk_queue, const uint32_t* __restrict__ pair_a,
                    const uint32_t* __restrict__ pair_b, const uint32_t* __restrict__ off,
-                   const PoseRec<St>* __restrict__ pose, const RBShape<float>* __restrict__ shape,
-                   const Vert<float>* __restrict__ verts, uint32_t* __restrict__ queue64,
-                   uint32_t* __restrict__ count64)
+                   const uint32_t* __restrict__ sorted_of, const PoseRec<St>* __restrict__ pose,
+                   const RBShape<float>* __restrict__ shape, const Vert<float>* __restrict__ verts,
+                   uint32_t* __restrict__ queue64, uint32_t* __restrict__ count64)
 {
     grid_dep_sync();
     if(step_aborted(flags))
@@ -2011,7 +2032,7 @@ __global__ void __launch_bounds__(128)
                                                      A.r + B.r, valid);
         if(valid && open)
         {
-            const uint32_t pm = mirror_record(off, pair_b, a, b);
+            const uint32_t pm = mirror_record(off, pair_b, sorted_of, a, b);
             const uint32_t k  = atomicAdd(count64, pm == kNoRecord ? 1u : 2u);
             queue64[k]        = p;
             if(pm != kNoRecord)

@@ -8,7 +8,7 @@ import pytest
 
 from grains3dgpu_b200 import abi, scenes
 
-from conftest import rel_err
+from conftest import rel_err, share_props
 from test_gpu_parity import pair
 
 pytestmark = pytest.mark.gpu
@@ -95,3 +95,75 @@ def test_spheres_alone(gb, oracle, n, law):
         assert rel_err(g.velocities(), o.velocities()) <= tol
         if n > 2:
             assert g.stats().contacts > 0
+
+
+def big_grain(shape, first, n=1350, seed=9):
+    """One large grain among n small ones that touch it: small spheres (and a
+    tenth boxes) on the shell of a large sphere, or small boxes lying on the
+    faces of a large box.  The large grain is the first or the last particle,
+    which decides in whose list the other's record is looked up."""
+    rng = np.random.default_rng(seed)
+    R, r = 4e-3, 0.2e-3
+    rbs = np.zeros(4, scenes.RB_DTYPE)
+    rbs["density"] = 2500.0
+    rbs["crust"] = 5e-5
+    rbs["type"] = [abi.GB_SPHERE, abi.GB_SPHERE, abi.GB_BOX, abi.GB_BOX]
+    rbs["p"][0, 0], rbs["p"][1, 0] = R, r
+    rbs["p"][2, :3], rbs["p"][3, :3] = R, r
+    if shape == "sphere":
+        k = np.arange(n) + 0.5
+        phi, z = np.pi * (1 + 5 ** 0.5) * k, 1 - 2 * k / n
+        u = np.stack([np.sqrt(1 - z * z) * np.cos(phi), np.sqrt(1 - z * z) * np.sin(phi), z], 1)
+        pos = u * (R + r * rng.uniform(0.8, 1.05, n))[:, None]
+        ids = np.where(rng.random(n) < 0.1, 3, 1)
+    else:
+        m = int(np.ceil(np.sqrt(n / 6)))
+        s = (np.arange(m) - (m - 1) / 2) * (2 * (R - r) / (m - 1))
+        u, v = (x.ravel() for x in np.meshgrid(s, s, indexing="ij"))
+        h = R + r + rng.uniform(0.5e-5, 0.9e-4, (6, m * m))
+        faces = []
+        for f in range(6):
+            q = np.zeros((m * m, 3))
+            q[:, f % 3] = h[f] * (1 if f < 3 else -1)
+            q[:, (f + 1) % 3], q[:, (f + 2) % 3] = u, v
+            faces.append(q)
+        pos = np.concatenate(faces)[:n]
+        ids = np.full(n, 3)
+    rot = np.tile(np.eye(3).ravel(), (n + 1, 1))
+    ang = rng.uniform(-0.05, 0.05, n + 1)
+    rot[:, 0], rot[:, 1], rot[:, 3], rot[:, 4] = np.cos(ang), -np.sin(ang), np.sin(ang), np.cos(ang)
+    at = 0 if first else n
+    side = 0.03
+    tr = np.zeros((n + 1, 12))
+    tr[:, :9] = rot
+    tr[:, 9:] = np.insert(pos, at, 0.0, axis=0) + 0.5 * side
+    ids = np.insert(ids, at, 0 if shape == "sphere" else 2).astype(np.uint32)
+    walls, wtr = scenes.box_walls((side,) * 3)
+    cfg = dict(n_particles=n + 1, n_rigid_bodies=4, n_obstacles=6, n_materials=2,
+               origin=(0, 0, 0), max_coordinate=(side,) * 3, dt=1e-6, gravity=(0, 0, -9.81))
+    vel = rng.normal(0.0, 0.05, (n + 1, 6))
+    return scenes.Scene("big-grain", cfg, rbs, np.zeros((0, 3)), ids, tr, vel, walls, wtr,
+                        [scenes.law(etat=0.3)] * 3)
+
+
+@pytest.mark.parametrize("first", [True, False])
+@pytest.mark.parametrize("shape", ["sphere", "box"])
+def test_mirror_records_of_a_long_list(gb, oracle, shape, first):
+    """Records looked up in a list of a thousand (the closed form of two
+    spheres, the queue of the FP64 GJK): both orders of every contact, bit for
+    bit."""
+    s = big_grain(shape, first)
+    kw = dict(gjk_variant=abi.GB_GJK_SV, contact_law=abi.GB_LAW_HOOKE)
+    g = scenes.System(gb, s, precision=abi.GB_FP64_STRICT, **kw,
+                      flags=abi.GB_FLAG_CRUST_BOUNDS | abi.GB_FLAG_RECORD_CONTACT_INFO)
+    o = scenes.System(oracle, s, flags=abi.GB_FLAG_CRUST_BOUNDS, **kw)
+    share_props(g, o, oracle)
+    g.detect()
+    o.detect()
+    contacts = g.dump(abi.GB_DUMP_CONTACT_PAIRS)
+    big = 0 if first else s.n - 1
+    assert (contacts[:, 0] == big).sum() > 300
+    assert np.array_equal(contacts, o.dump(abi.GB_DUMP_CONTACT_PAIRS))
+    assert np.array_equal(g.dump(abi.GB_DUMP_CONTACT_INFO), o.dump(abi.GB_DUMP_CONTACT_INFO),
+                          equal_nan=True)
+    assert np.array_equal(g.torces(), o.torces(), equal_nan=True)
