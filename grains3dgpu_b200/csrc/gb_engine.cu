@@ -901,12 +901,54 @@ int redo_with_radix(gb_ctx* c)
 // 1M bed with 90, 95, 97 and 99%: 15.08, 14.42, 13.99 and 14.23 ms, of the
 // 130k bed in FP64 2.74, 2.73, 2.70 and 2.85 ms); the grid is used where that is
 // below 0.7 of the largest radius (a polydisperse packing), the rigid-body
-// ids are known on the host, and its cell count stays moderate.  The split
+// ids are known on the host, and its cell count stays moderate.  Where more
+// than 3% of the particles are of a size well above the rest's, the 97th
+// percentile is that size and says nothing about the small ones: then, in
+// crowded cells, it is the 95th.  The split
 // only decides which kernel tests a pair, never whether it is tested, so a
 // stale plan costs time, not results.
-// the mean reference-cell occupancy seen by a particle above which the finer
-// grid pays for its extra passes (~27 x 8 = 216 candidates per particle)
+// The mean reference-cell occupancy seen by a particle above which the finer
+// grid pays for its extra passes (~27 x 8 = 216 candidates per particle) ...
 constexpr double kFineCrowding = 8.0;
+// ... above which it does with the 95th percentile, where the 97th makes none:
+// spheres of two radii, 3 to 5% of them 2 to 6 times as large, at 28 and
+// more 1.0 to 1.5 times as fast with it as without (1M, 4% of three times the
+// radius, occupancy 49: 1.50 -> 1.24 ms a step), at 24 0.99 to 1.17, at 9 to 20
+// 0.7 to 0.98; ...
+constexpr double kFineCrowding95 = 28.0;
+// ... and above which the 95th is better where the 97th is a further size
+// (kFineStep times the 95th's or more): 4.5% of the spheres in two larger sizes
+// at occupancy 61 and 102 1.09 times as fast, at 30 0.93; sizes 1.3 apart 0.99.
+constexpr double kFineCrowdingStep = 40.0;
+constexpr double kFineStep         = 1.4;
+
+// the grid for a given r_s (false: there is none)
+bool fine_grid(const gb_ctx* c, double rs, FineGrid* grid, uint64_t* cells)
+{
+    if(!(rs > 0.0) || !(rs < 0.7 * c->rmax))
+        return false;
+    FineGrid g{};
+    g.rs   = rs;
+    g.rmax = c->rmax;
+    g.h    = 2.0 * rs * (1.0 + 1e-9);
+    uint64_t nf = 1;
+    uint32_t dim[3];
+    for(int a = 0; a < 3; ++a)
+    {
+        g.mn[a]      = c->cfg.origin[a];
+        const double e = std::ceil((c->lc_max[a] - c->cfg.origin[a]) / g.h);
+        if(!(e >= 1.0) || e > 4.0e9)
+            return false;
+        dim[a] = (uint32_t)e;
+        nf *= dim[a];
+    }
+    if(2 * nf + 1 > kMaxCells || nf > 16ull * (uint64_t)c->n + 4096)
+        return false;
+    g.nx = dim[0], g.ny = dim[1], g.nz = dim[2];
+    *grid  = g;
+    *cells = nf;
+    return true;
+}
 
 int fine_plan(gb_ctx* c)
 {
@@ -919,34 +961,22 @@ int fine_plan(gb_ctx* c)
     for(int i = 0; i < n; ++i)
         r[i] = bound_radius(c, c->h_rb_id[i]);
     std::vector<double> q(r);
-    const size_t k = (size_t)(0.97 * (n - 1));
-    std::nth_element(q.begin(), q.begin() + k, q.end());
-    const double rs = q[k];
-    if(!(rs > 0.0) || !(rs < 0.7 * c->rmax))
+    const size_t k97 = (size_t)(0.97 * (n - 1)), k95 = (size_t)(0.95 * (n - 1));
+    std::nth_element(q.begin(), q.begin() + k97, q.end());
+    const double r97 = q[k97];
+    std::nth_element(q.begin(), q.begin() + k95, q.begin() + k97 + 1);
+    const double r95 = q[k95];
+    FineGrid     g{}, g95{};
+    uint64_t     nf = 0, nf95 = 0;
+    const bool   has97 = fine_grid(c, r97, &g, &nf);
+    const bool   has95 = (!has97 || r97 > kFineStep * r95) && fine_grid(c, r95, &g95, &nf95);
+    if(!has97 && !has95)
         return GB_OK;
-    FineGrid g{};
-    g.rs   = rs;
-    g.rmax = c->rmax;
-    g.h    = 2.0 * rs * (1.0 + 1e-9);
-    uint64_t nf = 1;
-    uint32_t dim[3];
-    for(int a = 0; a < 3; ++a)
-    {
-        g.mn[a]      = c->cfg.origin[a];
-        const double e = std::ceil((c->lc_max[a] - c->cfg.origin[a]) / g.h);
-        if(!(e >= 1.0) || e > 4.0e9)
-            return GB_OK;
-        dim[a] = (uint32_t)e;
-        nf *= dim[a];
-    }
-    if(2 * nf + 1 > kMaxCells || nf > 16ull * (uint64_t)n + 4096)
-        return GB_OK;
-    g.nx = dim[0], g.ny = dim[1], g.nz = dim[2];
+    double crowding = INFINITY; // (forced on)
     if(c->fine_mode < 0)
     {
-        // worth it where the reference cells are crowded: a particle shares
-        // its cell with sum(n_c^2) / n others on average (the cell starts of
-        // this step's sort, read once per plan)
+        // a particle shares its reference cell with sum(n_c^2) / n others on
+        // average (the cell starts of this step's sort, read once per plan)
         std::vector<uint32_t> cs((size_t)c->ncells + 1);
         GB_CK(cudaMemcpyAsync(cs.data(), c->d_cstart, cs.size() * sizeof(uint32_t),
                               cudaMemcpyDeviceToHost, c->stream));
@@ -957,12 +987,18 @@ int fine_plan(gb_ctx* c)
             const double m = cs[k + 1] >= cs[k] ? double(cs[k + 1] - cs[k]) : 0.0;
             sq += m * m;
         }
-        if(sq < kFineCrowding * (double)n)
-            return GB_OK;
+        crowding = sq / (double)n;
     }
+    if(has95 && crowding >= (has97 ? kFineCrowdingStep : kFineCrowding95))
+    {
+        g  = g95;
+        nf = nf95;
+    }
+    else if(!has97 || crowding < kFineCrowding)
+        return GB_OK;
     uint32_t nlarge = 0;
     for(int i = 0; i < n; ++i)
-        nlarge += r[i] > rs;
+        nlarge += r[i] > g.rs;
     // keys: the small particles' fine cells, then the large particles' (+ nf)
     if(nf > c->fine_nf || !c->mem_fine)
     {

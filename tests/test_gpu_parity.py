@@ -337,3 +337,49 @@ def test_mixed_precision_single_step_dense_polydisperse(gb):
     assert e["contacts_ref"] > 1000
     assert e["matched"] == e["contacts_ref"] == e["contacts_run"], e
     assert e["force"]["max"] <= 1e-5 and e["torque"]["max"] <= 1e-5, e
+
+
+def graded_spheres(sizes, shares, pitch, n=20_000, seed=8):
+    """Spheres of the given radii (mm) in the given shares on a jittered cubic
+    lattice (mm), in a box that holds it."""
+    rng = np.random.default_rng(seed)
+    rbs = np.zeros(len(sizes), scenes.RB_DTYPE)
+    rbs["type"] = abi.GB_SPHERE
+    rbs["p"][:, 0] = 1e-3 * np.array(sizes)
+    rbs["crust"], rbs["density"] = 1e-5, 2500.0
+    m = int(np.ceil(n ** (1 / 3)))
+    k = np.arange(n)
+    pos = np.stack([k % m, k // m % m, k // (m * m)], 1) * pitch + max(sizes)
+    tr = np.zeros((n, 12))
+    tr[:, :9] = scenes.random_rotations(rng, n)
+    tr[:, 9:] = 1e-3 * (pos + rng.uniform(-0.05, 0.05, (n, 3)) * pitch)
+    box = (1e-3 * (m * pitch + 2 * max(sizes)),) * 3
+    walls, wtr = scenes.box_walls(box)
+    cfg = dict(n_particles=n, n_rigid_bodies=len(sizes), n_obstacles=6, n_materials=2,
+               origin=(0, 0, 0), max_coordinate=box, dt=1e-6, gravity=(0, 0, -9.81))
+    ids = rng.choice(len(sizes), size=n, p=shares).astype(np.uint32)
+    return scenes.Scene("graded-spheres", cfg, rbs, np.zeros((0, 3)), ids, tr,
+                        np.zeros((n, 6)), walls, wtr, [scenes.law()] * 3)
+
+
+@pytest.mark.parametrize("sizes,shares,pitch,rs", [
+    ([1.0, 3.0], [0.96, 0.04], 1.6, 1.0),             # the 97th percentile is the large size
+    ([1.0, 3.0], [0.96, 0.04], 2.6, None),            # ... in cells too empty for the 95th
+    ([1.0, 2.0, 3.0], [0.955, 0.03, 0.015], 1.6, 1.0),  # the 97th is a further size
+    ([1.0, 2.0, 3.0], [0.955, 0.03, 0.015], 2.2, 2.0),  # ... in less crowded cells
+    ([1.0, 1.3, 3.0], [0.955, 0.03, 0.015], 1.6, 1.3),  # ... not much further
+])
+def test_fine_grid_of_graded_packings(gb, oracle, sizes, shares, pitch, rs):
+    """The radius that splits small from large grains (in mm; None: no finer
+    grid) where 3 to 5% of the grains are of larger sizes; the pair lists are
+    the oracle's."""
+    scene = graded_spheres(sizes, shares, pitch)
+    g, o = pair(gb, oracle, scene)
+    g.detect()
+    o.detect()
+    st = g.stats()
+    want = 0 if rs is None else np.prod([np.ceil((st.grid_max[k] - 0.0) / (2e-3 * rs * (1 + 1e-9)))
+                                         for k in range(3)])
+    assert st.fine_grid_cells == want
+    for kind in (abi.GB_DUMP_CANDIDATE_PAIRS, abi.GB_DUMP_CONTACT_PAIRS):
+        assert np.array_equal(g.dump(kind), o.dump(kind))
