@@ -180,7 +180,11 @@ __device__ __forceinline__ void put_sorted(uint32_t s, uint32_t e, const double*
     if(out32)
     {
         const double slack = 0x1p-19 * (fabs(p.x) + fabs(p.y) + fabs(p.z) + p.w);
-        out32[s] = make_float4((float)p.x, (float)p.y, (float)p.z, __double2float_ru(p.w + slack));
+        // (a square past FP32's range would reject everything: NaN, which
+        // rejects nothing, for radii that long)
+        const double r32 = p.w + slack;
+        out32[s] = make_float4((float)p.x, (float)p.y, (float)p.z,
+                               r32 < 0x1p60 ? __double2float_ru(r32) : NAN);
     }
 }
 

@@ -383,3 +383,23 @@ def test_fine_grid_of_graded_packings(gb, oracle, sizes, shares, pitch, rs):
     assert st.fine_grid_cells == want
     for kind in (abi.GB_DUMP_CANDIDATE_PAIRS, abi.GB_DUMP_CONTACT_PAIRS):
         assert np.array_equal(g.dump(kind), o.dump(kind))
+
+
+@pytest.mark.parametrize("precision", [abi.GB_FP64, abi.GB_FP64_STRICT])
+def test_lengths_past_the_square_root_of_fp32(gb, oracle, precision):
+    """The FP64 modes keep the candidates of grains whose radii have no square
+    in FP32 (the pre-test's arithmetic)."""
+    scene = graded_spheres([1.0, 1.2], [0.5, 0.5], 1.9, n=60)
+    scale = 1e23
+    for a in (scene.rbs["p"], scene.rbs["crust"], scene.transforms[:, 9:],
+              scene.obstacles["p"], scene.obstacle_transforms[:, 9:]):
+        a *= scale
+    scene.config["max_coordinate"] = tuple(scale * x for x in scene.config["max_coordinate"])
+    g, o = pair(gb, oracle, scene, precision=precision)
+    g.detect()
+    o.detect()
+    want = o.dump(abi.GB_DUMP_CANDIDATE_PAIRS)
+    assert want.shape[0] > 100
+    assert np.array_equal(g.dump(abi.GB_DUMP_CANDIDATE_PAIRS), want)
+    assert np.array_equal(g.dump(abi.GB_DUMP_CONTACT_PAIRS), o.dump(abi.GB_DUMP_CONTACT_PAIRS))
+    assert g.stats().contacts > 100
