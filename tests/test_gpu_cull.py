@@ -167,3 +167,58 @@ def test_mirror_records_of_a_long_list(gb, oracle, shape, first):
     assert np.array_equal(g.dump(abi.GB_DUMP_CONTACT_INFO), o.dump(abi.GB_DUMP_CONTACT_INFO),
                           equal_nan=True)
     assert np.array_equal(g.torces(), o.torces(), equal_nan=True)
+
+
+@pytest.mark.parametrize("variant", [abi.GB_GJK_JH, abi.GB_GJK_SV])
+def test_mixture_of_several_rounds(gb, oracle, variant):
+    """A list several times as long as the cull's threads (five blocks of 128 a
+    multiprocessor: 94,720 records at a time), so that what a stage leaves in a
+    warp's queues is carried over from round to round."""
+    g, o = pair(gb, oracle, packing(40_000, MIXTURE), gjk_variant=variant)
+    g.detect()
+    o.detect()
+    assert g.stats().candidate_pairs > 300_000
+    assert np.array_equal(g.dump(abi.GB_DUMP_CONTACT_PAIRS), o.dump(abi.GB_DUMP_CONTACT_PAIRS))
+    assert np.array_equal(g.dump(abi.GB_DUMP_CONTACT_INFO), o.dump(abi.GB_DUMP_CONTACT_INFO),
+                          equal_nan=True)
+    assert np.array_equal(g.torces(), o.torces(), equal_nan=True)
+
+
+def loose_boxes(n=20_000, stretch=1.2, crust=2e-4):
+    """Boxes alone, far enough apart that nearly all of them meet in their
+    crusts; no polyhedron in the table of bodies."""
+    s = packing(n, (2,))
+    s.rbs, s.vertices = s.rbs[:3].copy(), np.zeros((0, 3))
+    s.rbs["crust"] = crust
+    s.config["n_rigid_bodies"] = 3
+    s.config["max_coordinate"] = tuple(stretch * x for x in s.config["max_coordinate"])
+    for a in (s.transforms[:, 9:], s.obstacle_transforms[:, 9:], s.obstacles["p"]):
+        a *= stretch
+    return s
+
+
+@pytest.mark.parametrize("variant", [abi.GB_GJK_SV, abi.GB_GJK_NESTEROV])
+def test_long_queue_of_signed_volume_solves(gb, oracle, variant):
+    """More FP64 solves than a wave of four-lane pairs holds (at most four
+    blocks of 128 a multiprocessor: 18,944), which the two-lane form takes:
+    FP64-strict bit for bit as the oracle; in the mixed mode the same contacts,
+    and forces within 1e-5 but for the grains whose cores all but intersect."""
+    s = loose_boxes()
+    kw = dict(gjk_variant=variant, flags=abi.GB_FLAG_CRUST_BOUNDS)
+    o = scenes.System(oracle, s, **kw)
+    g, m, f = (scenes.System(gb, s, precision=p, **kw)
+               for p in (abi.GB_FP64_STRICT, abi.GB_MIXED, abi.GB_FP64))
+    share_props(g, o, oracle)
+    for y in (o, g, m, f):
+        y.detect()
+    assert min(y.stats().gjk_fp64_calls for y in (g, m, f)) > 20_000
+    want = o.dump(abi.GB_DUMP_CONTACT_PAIRS)
+    assert want.shape[0] > 20_000
+    for y in (g, m, f):
+        assert np.array_equal(y.dump(abi.GB_DUMP_CONTACT_PAIRS), want)
+    assert np.array_equal(g.torces(), o.torces(), equal_nan=True)
+    a, b = (y.dump(abi.GB_DUMP_CONTACT_FORCES)[:, :3] for y in (m, f))
+    ok = np.isfinite(a).all(1) & np.isfinite(b).all(1)
+    assert ok.mean() > 0.97
+    err = np.linalg.norm(a[ok] - b[ok], axis=1) / np.linalg.norm(b[ok], axis=1)
+    assert np.quantile(err, 0.99) <= 1e-5

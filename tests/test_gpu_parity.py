@@ -115,7 +115,7 @@ def test_broad_phase_and_pairs_bit_exact_polyhedra_200k(gb, oracle):
 @pytest.mark.parametrize("workload,knob", [("bed", None), ("dilute", "1"), ("bed", "0")])
 def test_fine_grid_pairs_bit_exact(gb, oracle, monkeypatch, workload, knob):
     """Candidates of a polydisperse packing on the finer grid (cell twice the
-    95th-percentile bounding radius; the largest 5 % of grains by warp): the
+    97th-percentile bounding radius; the largest 3 % of grains by warp): the
     dense bed of the headline workload (200,000 of its grains on the 2.2 mm
     lattice) takes it by itself, the dilute packing when forced, and the bed
     can be held to the linked cells alone.  Either way the cell starts,
