@@ -750,6 +750,7 @@ int scan_u32(gb_ctx* c, const uint32_t* in, uint32_t* out, int64_t n, uint32_t* 
         // growing the state mid-step: wait for the scans that may still read it
         GB_CK(cudaStreamSynchronize(c->stream));
         dfree(c->d_tile_state);
+        c->tile_cap = 0; // (should there be no memory)
         GB_TRY(dalloc(&c->d_tile_state, nb));
         GB_CK(cudaMemset(c->d_tile_state, 0, nb * sizeof(unsigned long long)));
         c->tile_cap = nb;
@@ -804,6 +805,7 @@ int broad_phase_radix(gb_ctx* c)
         if(hn > c->hist_cap)
         {
             dfree(c->d_hist);
+            c->hist_cap = 0;
             GB_TRY(dalloc(&c->d_hist, hn));
             c->hist_cap = hn;
         }
