@@ -1390,11 +1390,14 @@ GB_D void narrow_obstacle(int64_t p, uint32_t a, int o, const State<store_t<S>>&
 //     iteration and returns |v|; if that exceeds the crusts: no contact.
 // Every other pair (in particular every contact) takes the full GJK.  It is
 // evaluated in FP32 in every mode (supports, frames and dot products), with a
-// margin of 1e-4 of the bounding radii, some 20 times a bound on the FP32
-// error of g (support values are Lipschitz in the direction with constant
-// |x| <= R_circ, so the FP32 direction error of ~3e-7 moves them by < 1e-9 m;
-// the FP32 supports and frames add a few 1e-9 m): a pair decided here is one
-// that the FP64 GJK also finds out of contact, so the contact set and the
+// margin of 1e-4 of the bounding radii, some eleven times a bound on the FP32
+// error of g: a support value is short by up to 7.8e-6 of its radius
+// (support_sq_log32), and the direction's error of ~3e-7 (support values are
+// Lipschitz in the direction with constant |x| <= R_circ) and the frames' add
+// 1e-6.  A pair decided here is one that the FP64 GJK also finds out of
+// contact, so long as it converges (a signed-volume iteration that breaks down
+// on a separated pair ends at distance 0, a contact with a 0/0 normal; such a
+// pair is none here), so the contact set and the
 // contact geometry stay those of the FP64 GJK.  Both rules are the same for
 // (A, B) and (B, A): the pair of the other order has v and w mirrored, so
 // each unordered pair is decided once, for both its records.
