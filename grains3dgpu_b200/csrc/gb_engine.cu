@@ -164,6 +164,7 @@ struct gb_ctx
     double*  d_obs_vel   = nullptr;
     double*  d_rcirc64 = nullptr;
     double   rmax      = 0.0;     // the largest circumscribed radius (the candidate test's radius)
+    double   rmid      = 0.0;     // the (lower) median of the bodies' radii
     // FP64 shape tables: aliases of the above in the FP64 modes, separate
     // copies in the mixed mode (read by its FP64 GJK)
     void* d_shape64 = nullptr;
@@ -1389,6 +1390,22 @@ PairOut<store_t<S>> pair_out(gb_ctx* c)
     return po;
 }
 
+// Whether grains have many contacts, for the mixed per-particle pass: its plain
+// loop over a grain's records keeps several in flight, a loop of single
+// records leaves more registers to the rest.  Of spheres alone nearly every
+// candidate is a contact (1M spheres, a step: 460.6 us plain, 461.9 single; 200k
+// of two sizes up to 8% apart), and a grain more than kManySizes times as
+// large as the median body has hundreds of partners (1,350 around one: 109 us a
+// launch against 254; 20k spheres and boxes among some of 8 and 12 times their
+// size 1.05 to 1.23 times as fast).  Other packings have few contacts per grain
+// (1M bed 917 us plain, 910 single; dilute 257 and 248; 200k polyhedra 141, 139).
+constexpr double kManySizes = 8.0;
+
+bool many_contacts(const gb_ctx* c)
+{
+    return c->all_spheres || c->rmax > kManySizes * c->rmid;
+}
+
 template <typename S>
 int launch_particles(gb_ctx* c, const State<store_t<S>>& st, const Tables<S>& tb,
                       const PairOut<store_t<S>>& po, const StepParams<S>& sp, int* contacts_out)
@@ -1398,9 +1415,16 @@ int launch_particles(gb_ctx* c, const State<store_t<S>>& st, const Tables<S>& tb
     // after a detect with obstacles the stream waits on the auxiliary one:
     // a plain launch there
     const bool pdl = c->pdl && !(c->nob && (sp.phases & PHASE_DETECT));
-    GB_CK(launch(pdl, k_particles<S>, nb, kBlock, c->stream, c->n, st, tb, c->d_off[c->cur], po,
-                 sp, contacts_out, move && c->nob ? c->d_obsmask_id : nullptr, c->d_flags,
-                 c->d_done));
+    auto go = [&](auto kernel) -> int {
+        GB_CK(launch(pdl, kernel, nb, kBlock, c->stream, c->n, st, tb, c->d_off[c->cur], po, sp,
+                     contacts_out, move && c->nob ? c->d_obsmask_id : nullptr, c->d_flags,
+                     c->d_done));
+        return GB_OK;
+    };
+    if constexpr(is_mixed<S>())
+        GB_TRY(many_contacts(c) ? go(k_particles<S, true>) : go(k_particles<S, false>));
+    else
+        GB_TRY(go(k_particles<S, false>));
     c->launches += 1;
     if(move)
         c->mask_valid = c->nob > 0;
@@ -1997,6 +2021,7 @@ int gb_set_rigid_bodies(gb_ctx* c, const gb_rigid_body_desc* rbs, const double* 
     // a refused table leaves the context with the bodies that it had.
     std::vector<gb_rigid_body_props> props(c->nrb);
     double rmax         = 0.0;
+    std::vector<double> radii;
     bool   poly_bodies  = false;
     bool   all_spheres  = true;
     bool   some_spheres = false;
@@ -2015,7 +2040,13 @@ int gb_set_rigid_bodies(gb_ctx* c, const gb_rigid_body_desc* rbs, const double* 
             return GB_E_INVALID_ARG;
         GB_TRY(gb_rigid_body_properties(&rbs[i], vertices, &props[i]));
         rmax = std::max(rmax, bound_radius(c, rbs[i], props[i])); // Grains.cpp:226-231
+        radii.push_back(bound_radius(c, rbs[i], props[i]));
     }
+    // (a superquadric's radius can come out 0 or NaN: a power of 1 / (n2 - 2))
+    radii.erase(std::remove_if(radii.begin(), radii.end(), [](double r) { return !(r > 0.0); }),
+                radii.end());
+    if(!radii.empty())
+        std::nth_element(radii.begin(), radii.begin() + (radii.size() - 1) / 2, radii.end());
     // linked cell: cell = factor * 2 * max circumscribed radius (Grains.cpp:233-246)
     double coeff = c->cfg.cell_size_factor;
     if(coeff < 1.0)
@@ -2049,6 +2080,7 @@ int gb_set_rigid_bodies(gb_ctx* c, const gb_rigid_body_desc* rbs, const double* 
     c->cobs_valid   = false; // the cell size may change
     c->cell         = cell;
     c->rmax         = rmax;
+    c->rmid         = radii.empty() ? 0.0 : radii[(radii.size() - 1) / 2];
     for(int k = 0; k < 3; ++k)
     {
         c->lc_max[k] = lc_max[k];

@@ -2135,7 +2135,9 @@ __global__ void __launch_bounds__(128)
 // registers with a few spilled (measured 3% faster than three blocks at 79
 // registers without, and than five at 48); the FP64 ones need about 125
 // registers and get two blocks.
-template <typename S>
+// LOADED (mixed mode): the plain loop over a grain's records, for packings
+// whose grains have many contacts (many_contacts).
+template <typename S, bool LOADED>
 __global__ void __launch_bounds__(kBlock, sizeof(store_t<S>) == 4 ? 4 : 2)
     k_particles(int n, State<store_t<S>> st, Tables<S> tb, const uint32_t* __restrict__ off,
                 PairOut<store_t<S>> po, StepParams<S> sp, int* __restrict__ contacts_out,
@@ -2229,53 +2231,54 @@ __global__ void __launch_bounds__(kBlock, sizeof(store_t<S>) == 4 ? 4 : 2)
         {
             po.pcount[i] = 0u;
             const uint32_t pe = off[i + 1];
-            auto           add = [&](uint32_t p, uint8_t hit, const V3<S>& f, const V3<S>& t) {
-                nc += hit == kContactParticle;
-                F = F + f;
-                T = T + t;
-                if(sp.has_kr)
-                    T = T + mk<S>(S(po.m[0][p]), S(po.m[1][p]), S(po.m[2][p]));
-            };
-            auto force = [&](uint32_t p) {
-                return mk<S>(S(po.f[0][p]), S(po.f[1][p]), S(po.f[2][p]));
-            };
-            auto torque = [&](uint32_t p) {
-                return mk<S>(S(po.t[0][p]), S(po.t[1][p]), S(po.t[2][p]));
-            };
-            // The FP64 modes take two records at a time, their loads in flight
-            // together (a record out of contact is loaded and dropped): two
-            // resident blocks per SM do not hide a chain of dependent loads
-            // per partner (400k spheres 2790 -> 2746 us per ten steps).  The
-            // mixed mode's four do, and its plain loop, which the compiler
-            // unrolls with several records' flags in flight, must stay one:
-            // written as batches of one record it took a grain with 1,350
-            // partners 109 -> 254 us.
-            if constexpr(is_mixed<S>())
+            if constexpr(LOADED)
                 for(uint32_t p = off[i]; p < pe; ++p)
                 {
                     const uint8_t hit = po.contact[p];
                     if(!hit)
                         continue;
-                    add(p, hit, force(p), torque(p));
+                    nc += hit == kContactParticle;
+                    F = F + mk<S>(S(po.f[0][p]), S(po.f[1][p]), S(po.f[2][p]));
+                    T = T + mk<S>(S(po.t[0][p]), S(po.t[1][p]), S(po.t[2][p]));
+                    if(sp.has_kr)
+                        T = T + mk<S>(S(po.m[0][p]), S(po.m[1][p]), S(po.m[2][p]));
                 }
             else
-                for(uint32_t p = off[i]; p < pe; p += 2)
+            {
+                // The FP64 modes take two records at a time, their loads in
+                // flight together (a record out of contact is loaded and
+                // dropped): two resident blocks per SM do not hide a chain of
+                // dependent loads per partner (400k spheres 2790 -> 2746 us
+                // per ten steps).
+                constexpr uint32_t kBatch = is_mixed<S>() ? 1 : 2;
+                for(uint32_t p = off[i]; p < pe; p += kBatch)
                 {
-                    uint8_t hit[2];
-                    V3<S>   f[2], t[2];
+                    uint8_t hit[kBatch];
+                    V3<S>   f[kBatch], t[kBatch];
 #pragma unroll
-                    for(uint32_t k = 0; k < 2; ++k)
+                    for(uint32_t k = 0; k < kBatch; ++k)
                     {
                         const uint32_t q = p + k < pe ? p + k : pe - 1;
                         hit[k]           = p + k < pe ? po.contact[q] : uint8_t(0);
-                        f[k]             = force(q);
-                        t[k]             = torque(q);
+                        if(kBatch == 1 && !hit[k])
+                            break;
+                        f[k] = mk<S>(S(po.f[0][q]), S(po.f[1][q]), S(po.f[2][q]));
+                        t[k] = mk<S>(S(po.t[0][q]), S(po.t[1][q]), S(po.t[2][q]));
                     }
 #pragma unroll
-                    for(uint32_t k = 0; k < 2; ++k)
+                    for(uint32_t k = 0; k < kBatch; ++k)
                         if(hit[k])
-                            add(p + k, hit[k], f[k], t[k]);
+                        {
+                            nc += hit[k] == kContactParticle;
+                            F = F + f[k];
+                            T = T + t[k];
+                            if(sp.has_kr)
+                                T = T
+                                    + mk<S>(S(po.m[0][p + k]), S(po.m[1][p + k]),
+                                            S(po.m[2][p + k]));
+                        }
                 }
+            }
         }
     }
     else

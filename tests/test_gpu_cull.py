@@ -222,3 +222,26 @@ def test_long_queue_of_signed_volume_solves(gb, oracle, variant):
     assert ok.mean() > 0.97
     err = np.linalg.norm(a[ok] - b[ok], axis=1) / np.linalg.norm(b[ok], axis=1)
     assert np.quantile(err, 0.99) <= 1e-5
+
+
+@pytest.mark.parametrize("large", [True, False])
+def test_mixed_sums_of_long_and_short_lists(gb, large):
+    """The mixed mode's per-particle sums in both forms of that pass: a grain
+    twenty times as large as the median body, with a thousand contacts (the
+    plain loop), and a mixture of like sizes (single records).  Forces against
+    the FP64 mode's: sums of n FP32 values of at most the largest contact
+    force each, within n 2^-24 of their sum and the contacts' own 1e-6."""
+    s = big_grain("sphere", False) if large else packing(400, MIXTURE)
+    m, f = (scenes.System(gb, s, precision=p) for p in (abi.GB_MIXED, abi.GB_FP64))
+    m.detect()
+    f.detect()
+    pairs = f.dump(abi.GB_DUMP_CONTACT_PAIRS)
+    assert np.array_equal(m.dump(abi.GB_DUMP_CONTACT_PAIRS), pairs)
+    force = np.linalg.norm(f.dump(abi.GB_DUMP_CONTACT_FORCES)[:, :3], axis=1)
+    count = np.bincount(pairs[:, 0], minlength=s.n)
+    total = np.bincount(pairs[:, 0], force, minlength=s.n)
+    assert count.max() > 900 if large else 3 < count.max() < 64
+    inside = np.all((s.transforms[:, 9:] > 3e-3)
+                    & (s.transforms[:, 9:] < np.array(s.config["max_coordinate"]) - 3e-3), axis=1)
+    err = np.linalg.norm(m.torces()[:, :3] - f.torces()[:, :3], axis=1)
+    assert np.all(err[inside] <= (count * 2.0 ** -24 + 1e-6)[inside] * total[inside])
