@@ -164,7 +164,7 @@ struct gb_ctx
     double*  d_obs_vel   = nullptr;
     double*  d_rcirc64 = nullptr;
     double   rmax      = 0.0;     // the largest circumscribed radius (the candidate test's radius)
-    double   rmid      = 0.0;     // the (lower) median of the bodies' radii
+    double   rmid      = 0.0;     // the (lower) median of the bodies' radii (a sample)
     // FP64 shape tables: aliases of the above in the FP64 modes, separate
     // copies in the mixed mode (read by its FP64 GJK)
     void* d_shape64 = nullptr;
@@ -965,10 +965,10 @@ int fine_plan(gb_ctx* c)
         r[i] = bound_radius(c, c->h_rb_id[i]);
     std::vector<double> q(r);
     const size_t k97 = (size_t)(0.97 * (n - 1)), k95 = (size_t)(0.95 * (n - 1));
-    std::nth_element(q.begin(), q.begin() + k97, q.end());
-    const double r97 = q[k97];
-    std::nth_element(q.begin(), q.begin() + k95, q.begin() + k97 + 1);
+    std::nth_element(q.begin(), q.begin() + k95, q.end());
     const double r95 = q[k95];
+    std::nth_element(q.begin() + k95, q.begin() + k97, q.end()); // among the largest 5%
+    const double r97 = q[k97];
     FineGrid     g{}, g95{};
     uint64_t     nf = 0, nf95 = 0;
     const bool   has97 = fine_grid(c, r97, &g, &nf);
@@ -2021,7 +2021,8 @@ int gb_set_rigid_bodies(gb_ctx* c, const gb_rigid_body_desc* rbs, const double* 
     // a refused table leaves the context with the bodies that it had.
     std::vector<gb_rigid_body_props> props(c->nrb);
     double rmax         = 0.0;
-    std::vector<double> radii;
+    std::vector<double> radii; // of at most some 4,096 bodies, for their median
+    const int           every = std::max(1, c->nrb / 4096);
     bool   poly_bodies  = false;
     bool   all_spheres  = true;
     bool   some_spheres = false;
@@ -2040,7 +2041,8 @@ int gb_set_rigid_bodies(gb_ctx* c, const gb_rigid_body_desc* rbs, const double* 
             return GB_E_INVALID_ARG;
         GB_TRY(gb_rigid_body_properties(&rbs[i], vertices, &props[i]));
         rmax = std::max(rmax, bound_radius(c, rbs[i], props[i])); // Grains.cpp:226-231
-        radii.push_back(bound_radius(c, rbs[i], props[i]));
+        if(i % every == 0)
+            radii.push_back(bound_radius(c, rbs[i], props[i]));
     }
     // (a superquadric's radius can come out 0 or NaN: a power of 1 / (n2 - 2))
     radii.erase(std::remove_if(radii.begin(), radii.end(), [](double r) { return !(r > 0.0); }),
