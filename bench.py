@@ -811,19 +811,20 @@ TRAFFIC_PER_PARTICLE = {"integration": (95.4e6 + 12.2e6) / 600_000,
                         "broad_phase": (14.48e6 + 2.56e6 + 26.54e6 + 0.06e6) / 600_000}
 
 
-# what bounds each stage or phase, from the same captures and those of the bed
-# at 200,000 grains
-LIMITER = {"integration": "issue and memory latency: 40% warps active (64 registers, four "
+# what bounds each stage or phase, from captures of the bed at 400,000 grains
+# (the broad phase's from those at 600,000)
+LIMITER = {"integration": "issue and memory latency: 37% warps active (64 registers, four "
                           "256-thread blocks per SM), 42% issue slots; 159 B per particle "
                           "read from DRAM",
            "broad_phase": "launch and tail latency of short dependent passes (hash 10 us, "
                           "scan, scatter 9 us, rank 20 us at 600k grains); 73 B per particle "
                           "read from DRAM",
-           "pair_count": "memory latency of the neighbour walk on the finer grid: 16 "
-                         "long-scoreboard stalls per issue at 59% warps active",
-           "narrow": "FP32 issue in the cull (42% issue slots, 30 of 32 lanes, 96 registers) "
-                     "and FP64 GJK chains at 10-15% warps active (220 registers, 168 in "
-                     "its three-block form for long queues)"}
+           "pair_count": "FP32 issue of the neighbour walk on the finer grid (67% issue slots at "
+                         "85% warps active), memory latency in the large grains' pass (54% "
+                         "warps active)",
+           "narrow": "FP32 issue in the cull (44% issue slots, 30 of 32 lanes, 96 registers) "
+                     "and FP64 GJK chains at 14% warps active (168 registers in the "
+                     "three-block form for long queues, 253 otherwise)"}
 
 
 def traffic_bytes(phase, n):

@@ -1905,7 +1905,7 @@ GB_D bool warp_pop(const WarpQueue& q, unsigned& n, uint32_t& p, uint32_t& a, ui
 // gjk_first_iteration_separates), so every mode, the bit-exact one included,
 // keeps the contacts of its own FP64 tests, which the last pass repeats for
 // each record it solves.  Bound by FP32 issue and the latency of the records
-// (42% of issue slots at five blocks per SM; six gave the 1M bed 1% and cost
+// (44% of issue slots at five blocks per SM; six gave the 1M bed 1% and cost
 // the 100k polyhedra 2%).  A launch, against a thread per ordered record in
 // the mode's own precision: 1M bed mixed 398 -> 176 us, 130k bed FP64 242 ->
 // 30 us, 400k drum 334 -> 107 us, 100k polyhedra 149 -> 94 us (and less since
