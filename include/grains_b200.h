@@ -213,7 +213,9 @@ int gb_destroy(gb_ctx* ctx);
 const char* gb_status_string(int status);
 int gb_abi_version(void);
 
-/* ---- set-up (Grains::Construction, Grains/Base/src/Grains.cpp:90-300) ----------- */
+/* ---- set-up (Grains::Construction, Grains/Base/src/Grains.cpp:90-300) -----------
+ * A table of bodies, laws or obstacles that is refused (GB_E_INVALID_ARG,
+ * GB_E_UNSUPPORTED) leaves the context as it was. */
 /* Rigid-body table; `vertices` holds 3 doubles per polyhedron vertex. */
 int gb_set_rigid_bodies(gb_ctx* ctx, const gb_rigid_body_desc* rbs,
                         const double* vertices, int64_t n_vertices);
