@@ -697,8 +697,8 @@ int resize_list(gb_ctx* c, int64_t ncap)
 }
 
 // The other arrays of pair capacity, as many records as the list's, in place
-// of the old ones (freed first: they are the larger part, and hold nothing
-// between detects).  Without memory the context has none (cap 0).
+// of the old ones (freed first: they are the larger part, and hold only the
+// last detect's outputs).  Without memory the context has none (cap 0).
 int resize_work(gb_ctx* c)
 {
     dfree(c->mem_pairs);
